@@ -82,11 +82,12 @@ struct lyd_ctx {
     double *nu = nullptr, *nuC = nullptr, *dnu = nullptr, *inv_dnu = nullptr, *inv_nuC = nullptr;
     bool freq_set = false;
     // work lists
-    lyd_tuning tune{kDefaultRows, 0, SOLVER_PCR, 0, LYD_STAGING_AUTO};
+    lyd_tuning tune{0, 0, SOLVER_PCR, 0, LYD_STAGING_AUTO};
     unsigned char *tmaps = nullptr;    // tensor maps of J, H_r, H_Z: [set][cloud][3] (TMA staging)
     bool tma_ok = false;               // every map encoded (the layout allows bulk tensor copies)
     int4 *tiles = nullptr, *items = nullptr;
-    int ntiles = 0, nitems = 0;
+    int4 *tma_tiles = nullptr;         // the bulk-copy form's own tiles (only when it is used)
+    int ntiles = 0, ntma = 0, nitems = 0;
     double *partials = nullptr;
     int *kwin = nullptr;
     bool active_valid = false;
@@ -215,7 +216,18 @@ static void drop_graph(lyd_ctx *c) {
     }
 }
 
-// Work lists. Advection: tiles of 8 columns x rows x 32 bins, column tile fastest, per cloud.
+static int staging_used(const lyd_ctx *c);
+// rows of the fixed tiles, and the grain of the host step's chunks, when the tuning leaves them open
+static int fixed_rows(const lyd_ctx *c) { return c->tune.rows_per_tile > 0 ? c->tune.rows_per_tile : kDefaultRows; }
+
+// Packed advection tiles of rows [j0, j1) of cloud q: as many places as the widest window needs.
+static void push_tiles(const lyd_ctx *c, int q, int j0, int j1, std::vector<int4> &t) {
+    if (j1 <= j0) return;
+    const int n = adv_tiles(c->nnu, c->nr[q], j1 - j0, c->tune.rows_per_tile, c->desc[q].adv_share);
+    for (int e = 0; e < n; e++) t.push_back(make_int4(q, j0, e, j1));
+}
+
+// Work lists. Advection: packed tiles, per cloud; for bulk copies tiles of 8 columns x rows x 32 bins.
 // Frequency kernel: runs of `cpb` consecutive cells of one cloud per block.
 static int cells_per_block(const lyd_ctx *c) {
     if (c->tune.cells_per_block > 0) return c->tune.cells_per_block;
@@ -225,13 +237,19 @@ static int cells_per_block(const lyd_ctx *c) {
 }
 
 static int build_work(lyd_ctx *c) {
-    const int rows = c->tune.rows_per_tile;
-    std::vector<int4> t, it;
-    const int nkb = (c->nnu + 31) / 32;
-    for (int q = 0; q < c->ncl; q++)
-        for (int kb = 0; kb < nkb; kb++)
-            for (int j0 = c->desc[q].j_own0; j0 < c->desc[q].j_own1; j0 += rows)
-                for (int i0 = 0; i0 < c->nr[q]; i0 += kTileCols) t.push_back(make_int4(q, i0, j0, 32 * kb));
+    const int rows = fixed_rows(c);
+    std::vector<int4> t, tt, it;
+    const int nkb = (c->nnu + 31) / 32, slots = c->sms * adv_ctas_per_sm(c->prec, c->tune.adv_ctas_per_sm);
+    for (int q = 0; q < c->ncl; q++) {
+        const long long cells = (long long)c->nr[q] * c->nz[q];
+        c->desc[q].adv_share = (int)std::max<long long>(1, slots * cells / std::max<long long>(1, (long long)c->ncell));
+        push_tiles(c, q, c->desc[q].j_own0, c->desc[q].j_own1, t);
+    }
+    if (staging_used(c) == LYD_STAGING_TMA)
+        for (int q = 0; q < c->ncl; q++)
+            for (int kb = 0; kb < nkb; kb++)
+                for (int j0 = c->desc[q].j_own0; j0 < c->desc[q].j_own1; j0 += rows)
+                    for (int i0 = 0; i0 < c->nr[q]; i0 += kTileCols) tt.push_back(make_int4(q, i0, j0, 32 * kb));
     const int cpb = cells_per_block(c);
     for (int q = 0; q < c->ncl; q++) {
         const int b0 = c->nr[q] * c->desc[q].j_own0, nc = c->nr[q] * c->desc[q].j_own1;   // owned cells
@@ -240,17 +258,23 @@ static int build_work(lyd_ctx *c) {
         c->desc[q].npb = (int)it.size() - c->desc[q].pb0;
     }
     cudaFree(c->tiles);
+    cudaFree(c->tma_tiles);
     cudaFree(c->items);
     cudaFree(c->partials);
-    c->tiles = c->items = nullptr;
+    c->tiles = c->tma_tiles = c->items = nullptr;
     c->partials = nullptr;
     LYD_TRY(dalloc(c, (void **)&c->tiles, t.size() * sizeof(int4)));
+    if (!tt.empty()) {
+        LYD_TRY(dalloc(c, (void **)&c->tma_tiles, tt.size() * sizeof(int4)));
+        LYD_CU(c, cudaMemcpyAsync(c->tma_tiles, tt.data(), tt.size() * sizeof(int4), cudaMemcpyHostToDevice, c->st));
+    }
     LYD_TRY(dalloc(c, (void **)&c->items, it.size() * sizeof(int4)));
     LYD_TRY(dalloc(c, (void **)&c->partials, it.size() * (size_t)(c->nnu + kExtraCols) * 8));
     LYD_CU(c, cudaMemcpyAsync(c->tiles, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice, c->st));
     LYD_CU(c, cudaMemcpyAsync(c->items, it.data(), it.size() * sizeof(int4), cudaMemcpyHostToDevice, c->st));
     LYD_CU(c, cudaStreamSynchronize(c->st));
     c->ntiles = (int)t.size();
+    c->ntma = (int)tt.size();
     c->nitems = (int)it.size();
     drop_graph(c);
     return sync_desc(c);
@@ -326,16 +350,13 @@ static int encode_tmaps(lyd_ctx *c) {
     return LYD_OK;
 }
 
-// The staging the advection uses: bulk copies when asked for, or by default with FP32 storage,
-// and the maps exist. Measured at 256^2 x 64 (per launch): FP32 storage 0.171 ms with per-lane
-// loads, 0.167 ms with bulk copies; FP64 arithmetic at 3 CTAs per SM 0.333 / 0.341 ms (the row
-// loads are not what stalls it); FP32 arithmetic over FP64 storage 0.183 / 0.215 ms (the raw
-// tile leaves room for 3 CTAs per SM instead of 4).
+// The staging the advection uses: bulk copies when asked for and the maps exist, else the packed
+// tiles' own copies.
+// The packed tiles are the default in every form: a bulk copy's box is fixed when its map is encoded,
+// so its tiles cannot follow the active window (256^2 x 64, 53 active bins, FP32 storage: 140 us packed,
+// 167 us with bulk copies).
 static int staging_used(const lyd_ctx *c) {
-    const int want = c->tune.adv_staging != LYD_STAGING_AUTO
-                         ? c->tune.adv_staging
-                         : (c->prec == LYD_PREC_FP32 ? LYD_STAGING_TMA : LYD_STAGING_LANES);
-    return (want == LYD_STAGING_TMA && c->tma_ok) ? LYD_STAGING_TMA : LYD_STAGING_LANES;
+    return (c->tune.adv_staging == LYD_STAGING_TMA && c->tma_ok) ? LYD_STAGING_TMA : LYD_STAGING_LANES;
 }
 
 const char *lyd_last_error(const lyd_ctx *c) { return c ? c->msg.c_str() : "null context"; }
@@ -482,7 +503,7 @@ int lyd_destroy(lyd_ctx *c) {
     void *ps[] = {c->Hv, c->phi, c->phi_inv, c->aF, c->Ff[0], c->Ff[1], c->Ff[2], c->u_r_star, c->u_Z_star, c->dV,
                   c->inv_dV, c->A_r, c->A_Z, c->inv_r_cell, c->rCoM, c->ZCoM, c->rint, c->zint, c->r_if, c->Z_if,
                   c->nu, c->nuC, c->dnu, c->inv_dnu, c->inv_nuC, c->partials, c->kwin, c->hist, c->step_ctr,
-                  c->last, c->err, c->lut, c->stage, c->small, c->cl, c->tiles, c->items, c->adj_ws,
+                  c->last, c->err, c->lut, c->stage, c->small, c->cl, c->tiles, c->tma_tiles, c->items, c->adj_ws,
                   c->red_cols, c->red_cnt, c->bar, c->hin, c->part_chk, c->kwin_chk, c->ctiles};
     for (void *p : ps) cudaFree(p);
     for (int q = 0; q < CF_N; q++) cudaFree(c->cellf[q]);
@@ -541,6 +562,7 @@ int lyd_set_tuning(lyd_ctx *c, const lyd_tuning *t) {
 int lyd_get_tuning(lyd_ctx *c, lyd_tuning *t) {
     if (!c || !t) return LYD_ERR_ARG;
     *t = c->tune;
+    t->rows_per_tile = fixed_rows(c);
     if (t->cells_per_block == 0) t->cells_per_block = -cells_per_block(c);   // negative: chosen automatically
     t->adv_ctas_per_sm = adv_ctas_per_sm(c->prec, t->adv_ctas_per_sm);
     t->adv_staging = staging_used(c);
@@ -774,12 +796,23 @@ static void fill_adv(lyd_ctx *c, AdvArgs<S> &a, int in_set, int out_set) {
     a.duZ_dZ = c->cellf[CF_DUZ_DZ]; a.ur_over_r = c->cellf[CF_UR_OVER_R];
     a.kwin = c->kwin;
     a.cl = c->cl;
-    a.tiles = c->tiles;
-    a.rows = c->tune.rows_per_tile;
+    const bool tma = c->tma_tiles && staging_used(c) == LYD_STAGING_TMA;
+    a.tiles = tma ? c->tma_tiles : c->tiles;
+    a.ntiles = tma ? c->ntma : c->ntiles;
+    a.rows = tma ? fixed_rows(c) : c->tune.rows_per_tile;
     a.nnu = c->nnu;
     a.jeps = c->jeps_s; a.heps2 = c->heps2_s;
     a.err = c->err;
-    a.tmaps = staging_used(c) == LYD_STAGING_TMA ? c->tmaps + (size_t)in_set * c->ncl * 3 * kTensorMapBytes : nullptr;
+    a.tmaps = tma ? c->tmaps + (size_t)in_set * c->ncl * 3 * kTensorMapBytes : nullptr;
+}
+// Inputs outside the context's buffer sets (which the tensor maps cover), and the persistent step,
+// take the packed tiles.
+template <typename S>
+static void packed_tiles(lyd_ctx *c, AdvArgs<S> &a) {
+    a.tmaps = nullptr;
+    a.tiles = c->tiles;
+    a.ntiles = c->ntiles;
+    a.rows = c->tune.rows_per_tile;
 }
 
 template <typename S>
@@ -885,11 +918,11 @@ static int do_advect(lyd_ctx *c) {
     if (c->sprec == 0) {
         AdvArgs<double> a;
         fill_adv<double>(c, a, in, out);
-        launch_advect(c->prec, c->cfg.flux_method, &a, c->ntiles, c->tune.adv_ctas_per_sm, c->st);
+        launch_advect(c->prec, c->cfg.flux_method, &a, c->tune.adv_ctas_per_sm, c->st);
     } else {
         AdvArgs<float> a;
         fill_adv<float>(c, a, in, out);
-        launch_advect(c->prec, c->cfg.flux_method, &a, c->ntiles, c->tune.adv_ctas_per_sm, c->st);
+        launch_advect(c->prec, c->cfg.flux_method, &a, c->tune.adv_ctas_per_sm, c->st);
     }
     LYD_CU(c, cudaGetLastError());
     c->cur = out;
@@ -940,11 +973,11 @@ int lyd_advect_jh(lyd_ctx *c, double ctdt, int32_t kmin, int32_t kmax, int32_t u
     if (c->sprec == 0) {
         AdvArgs<double> a;
         fill_adv<double>(c, a, in, out);
-        launch_advect(c->prec, c->cfg.flux_method, &a, c->ntiles, c->tune.adv_ctas_per_sm, c->st);
+        launch_advect(c->prec, c->cfg.flux_method, &a, c->tune.adv_ctas_per_sm, c->st);
     } else {
         AdvArgs<float> a;
         fill_adv<float>(c, a, in, out);
-        launch_advect(c->prec, c->cfg.flux_method, &a, c->ntiles, c->tune.adv_ctas_per_sm, c->st);
+        launch_advect(c->prec, c->cfg.flux_method, &a, c->tune.adv_ctas_per_sm, c->st);
     }
     cudaError_t e = cudaGetLastError();
     c->cur = out;
@@ -1120,7 +1153,8 @@ static int enqueue_step(lyd_ctx *c, bool timed, double *tape = nullptr, const S 
     fill_adv<S>(c, aa, A, B);
     aa.tape = tape;
     aa.tape_stride = (long long)c->n3;
-    if (in) { aa.J = in; aa.Hr = in + c->n3; aa.HZ = in + 2 * c->n3; aa.tmaps = nullptr; }
+    if (in) { aa.J = in; aa.Hr = in + c->n3; aa.HZ = in + 2 * c->n3; }
+    if (in || polls > 0) packed_tiles(c, aa);
     FreqArgs<S> fa;
     if (out)
         fill_freq<S>(c, fa, c->set[B][0], c->set[B][1], c->set[B][2], c->set[B][0], out, out + c->n3,
@@ -1138,7 +1172,7 @@ static int enqueue_step(lyd_ctx *c, bool timed, double *tape = nullptr, const S 
     const int prec = c->prec;
     if (polls > 0) {
         if (timed) cudaEventRecord(c->ev[0], c->st);
-        cudaError_t e = launch_persistent(prec, c->cfg.flux_method, &aa, &fa, ra, c->nnu, c->ntiles, c->nitems, c->bar,
+        cudaError_t e = launch_persistent(prec, c->cfg.flux_method, &aa, &fa, ra, c->nnu, c->nitems, c->bar,
                                           polls, c->err, c->st);
         if (timed)
             for (int q = 1; q < 4; q++) cudaEventRecord(c->ev[q], c->st);
@@ -1147,7 +1181,7 @@ static int enqueue_step(lyd_ctx *c, bool timed, double *tape = nullptr, const S 
         return LYD_OK;
     }
     if (timed) cudaEventRecord(c->ev[0], c->st);
-    launch_advect(prec, c->cfg.flux_method, &aa, c->ntiles, c->tune.adv_ctas_per_sm, c->st);
+    launch_advect(prec, c->cfg.flux_method, &aa, c->tune.adv_ctas_per_sm, c->st);
     if (timed) cudaEventRecord(c->ev[1], c->st);
     launch_freq(prec, &fa, c->nnu, c->nitems, c->st);
     if (timed) cudaEventRecord(c->ev[2], c->st);
@@ -1273,13 +1307,13 @@ int lyd_static_steps(lyd_ctx *c, const lyd_step_params *p, lyd_diag *hist_out) {
 constexpr int kMaxHostChunks = 16;
 
 // The work lists grouped by row chunk: chunk q covers a run of the T tile rows, its advection
-// tiles (every bin chunk of those rows), and the frequency items whose cells all lie below the
+// tiles, and the frequency items whose cells all lie below the
 // chunk's last row (the last chunk takes the rest). The first and the last chunk get half the
 // rows of the others: the first chunk's upload runs before anything else can start, and the
 // last chunk's download after everything else has ended.
 static int build_host_chunks(lyd_ctx *c, int chunks) {
-    const int rows = c->tune.rows_per_tile, nr = c->nr[0], nz = c->nz[0];
-    const int ntr = (nz + rows - 1) / rows, nkb = (c->nnu + 31) / 32, cpb = cells_per_block(c);
+    const int rows = fixed_rows(c), nr = c->nr[0], nz = c->nz[0];
+    const int ntr = (nz + rows - 1) / rows, cpb = cells_per_block(c);
     if (c->hs_req == chunks && c->hs_rows == rows && c->hs_cpb == cpb && c->ctiles) return LYD_OK;
     c->hs_req = chunks;
     if (chunks > ntr) chunks = ntr;
@@ -1297,9 +1331,7 @@ static int build_host_chunks(lyd_ctx *c, int chunks) {
     for (int q = 0; q < chunks; q++) {
         const int tr0 = bound(q), tr1 = bound(q + 1);
         c->ct_off[q] = (int)t.size();
-        for (int kb = 0; kb < nkb; kb++)
-            for (int tr = tr0; tr < tr1; tr++)
-                for (int i0 = 0; i0 < nr; i0 += kTileCols) t.push_back(make_int4(0, i0, tr * rows, 32 * kb));
+        push_tiles(c, 0, std::min(nz, tr0 * rows), std::min(nz, tr1 * rows), t);
         c->row_off[q] = std::min(nz, tr0 * rows);
         c->it_off[q] = (int)std::min<long long>(c->nitems, (long long)c->row_off[q] * nr / cpb);
     }
@@ -1413,7 +1445,7 @@ int lyd_static_step_host(lyd_ctx *c, const lyd_step_params *p, const double *J, 
     AdvArgs<double> aa;
     fill_adv<double>(c, aa, A, B);
     aa.J = c->hin; aa.Hr = c->hin + n3; aa.HZ = c->hin + 2 * n3;
-    aa.tmaps = nullptr;
+    packed_tiles(c, aa);
     FreqArgs<double> fa;
     fill_freq<double>(c, fa, c->set[B][0], c->set[B][1], c->set[B][2], c->set[B][0], c->set[A][0], c->set[A][1],
                       c->set[A][2]);
@@ -1424,9 +1456,8 @@ int lyd_static_step_host(lyd_ctx *c, const lyd_step_params *p, const double *J, 
     for (int q = 0; q < nch; q++) {
         LYD_CU(c, cudaStreamWaitEvent(c->st, ev_up[q], 0));
         aa.tiles = c->ctiles + c->ct_off[q];
-        if (c->ct_off[q + 1] > c->ct_off[q])
-            launch_advect(c->prec, c->cfg.flux_method, &aa, c->ct_off[q + 1] - c->ct_off[q], c->tune.adv_ctas_per_sm,
-                          c->st);
+        aa.ntiles = c->ct_off[q + 1] - c->ct_off[q];
+        launch_advect(c->prec, c->cfg.flux_method, &aa, c->tune.adv_ctas_per_sm, c->st);
         LYD_CU(c, cudaEventRecord(ev_adv[q], c->st));
         LYD_CU(c, cudaStreamWaitEvent(c->st_fq, ev_adv[q], 0));
         fa.item0 = c->it_off[q];
@@ -2076,13 +2107,13 @@ int lyd_adjoint_run(lyd_ctx *c, const lyd_adjoint_cfg *cfg, lyd_adjoint_out *out
         if (sn) {
             LYD_TRY(copy_state(sn, c->cur, s));
             aa.J = sn; aa.Hr = sn + n3; aa.HZ = sn + 2 * n3;
-            aa.tmaps = nullptr;     // the maps cover the context's buffer sets, not the workspace
+            packed_tiles(c, aa);    // the maps cover the context's buffer sets, not the workspace
         }
         aa.Jo = xA; aa.Hro = xA + n3; aa.HZo = xA + 2 * n3;
         aa.kwin = win + 2 * n;
         aa.tape = tape;
         aa.tape_stride = (long long)n3;
-        launch_advect(LYD_PREC_FP64, c->cfg.flux_method, &aa, c->ntiles, 2, s);
+        launch_advect(LYD_PREC_FP64, c->cfg.flux_method, &aa, 2, s);
         if (freq) {
             FreqArgs<double> fq;
             fill_freq<double>(c, fq, xA, xA + n3, xA + 2 * n3, xA, c->set[c->cur][0], c->set[c->cur][1],

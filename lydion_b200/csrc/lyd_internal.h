@@ -25,6 +25,7 @@ struct CloudDesc {
     int bc_r_left, bc_r_right, bc_z_bot, bc_z_top;
     int j_own0, j_own1;  // rows this context updates; outside them, halo rows of a Z-slab
                          // decomposition (domain neighbours' rows, read by the stencil only)
+    int adv_share;       // this cloud's share of the GPU's resident advection CTAs, by its cells
     int pb0, npb;        // this cloud's blocks in the frequency-kernel work list / partials
     double ctdt, dt, c_tilde, z_center;
 };
@@ -59,15 +60,18 @@ struct AdvArgs {
     const double *dur_dr, *dur_dZ, *duZ_dr, *duZ_dZ, *ur_over_r;
     const int *kwin;             // device {kmin, kmax} per cloud
     const CloudDesc *cl;
-    const int4 *tiles;           // (cloud, i0, j0, k0)
-    int rows;                    // rows per tile
+    // packed tiles: (cloud, first row, place in the list of those rows, end of the rows); the
+    // bulk-copy form: (cloud, i0, j0, k0)
+    const int4 *tiles;
+    int ntiles;
+    int rows;                    // rows per tile; packed tiles: 0 leaves them to pack_rows
     int nnu;
     double jeps, heps2;          // closure floors in storage units
     double *tape;                // adjoint recomputation: the cell update's values before its
                                  // floors and limiter, 4 fields of tape_stride (or nullptr)
     long long tape_stride;
     const unsigned char *tmaps;  // tensor maps of the input J, H_r, H_Z, [cloud][3] of
-                                 // kTensorMapBytes each in device memory, or nullptr: per-lane loads
+                                 // kTensorMapBytes each in device memory, or nullptr: packed tiles
     int *err;                    // device error bits (ERRB_TIMEOUT)
 };
 
@@ -140,7 +144,9 @@ int bins_per_lane(int nnu);
 // type of the state arrays (0: double, 1: float).
 void launch_find_active(int sprec, const void *J, int nnu, const double *dnu, const double *dV, const CloudDesc *cl,
                         const int4 *items, int nitems, double jeps, double *partials, cudaStream_t st);
-void launch_advect(int prec, int flux, const void *args, int ntiles, int ctas_per_sm, cudaStream_t st);
+void launch_advect(int prec, int flux, const void *args, int ctas_per_sm, cudaStream_t st);
+// the most packed tiles any window of 1..nnu bins makes of `nz` rows of a cloud of nr columns
+int adv_tiles(int nnu, int nr, int nz, int rows, int share);
 int adv_ctas_per_sm(int prec, int want);   // the occupancy variant launch_advect uses
 void launch_freq(int prec, const void *args, int nnu, int nitems, cudaStream_t st);
 // fn 0: rsqrt_nr, 1: rcp<double>, 2: x * rsqrt_nr(x), 3: chi_L84<double>, 4: exp_tab
@@ -148,7 +154,7 @@ void launch_math(int fn, const double *x, double *y, size_t n, cudaStream_t st);
 // one fused step in one cooperative launch (advection, frequency step, reduction, with bounded
 // grid barriers between them); bar: two unsigned of device memory
 cudaError_t launch_persistent(int prec, int flux, const void *adv, const void *freq, const RedArgs &red, int nnu,
-                              int ntiles, int nitems, unsigned *bar, long long polls, int *err, cudaStream_t st);
+                              int nitems, unsigned *bar, long long polls, int *err, cudaStream_t st);
 void launch_reduce(const RedArgs &a, cudaStream_t st);
 int freq_blocks(int ncell, int dev);
 

@@ -199,28 +199,17 @@ constexpr int MWARPS = MT + 1;
 constexpr int MTHREADS = 32 * MWARPS;
 constexpr int MCOL = MT + 4;           // staged columns i0-2 .. i0+MT+1
 constexpr int RING = 4;
-// staged fields per cell: J, f_r, f_Z and alpha_F (formed once per staged cell; four face sides
-// read each cell's)
-template <typename R> __host__ __device__ constexpr int nf() { return 4; }
 // The own columns' state (J, H_r, H_Z in the storage type) is kept for the rows j .. j+2 only
 // (staged at j+2, updated at j): a ring of three slots.
 constexpr int HRING = 3;
 __host__ __device__ constexpr int hslot(int r) { return ((r % HRING) + HRING) % HRING; }
 
-// The staged-cell ring A: [RING][MCOL][nf][32] (staged column lc, ring slot of the row), or with
-// H1 the own columns' ring [RING][MT][nf][32] followed by one row of the four halo columns
-// (lc 0, 1, MT+2, MT+3) [4][nf][32]: with per-lane staging the halo of row j is staged for and
-// read by row j's r faces alone, so one row of it suffices (12 KB less in FP64).
-template <typename R, bool H1>
+// The staged-cell ring A of the bulk-copy tile: [RING][MCOL][4][32] (ring slot of the row, staged
+// column lc).
+template <typename R>
 __device__ __forceinline__ R *a_cell(R *A, int slot, int lc) {
-    if constexpr (H1) {
-        if (lc >= 2 && lc < MT + 2) return A + ((slot * MT + (lc - 2)) * nf<R>()) * 32;
-        return A + ((RING * MT + (lc < 2 ? lc : lc - MT)) * nf<R>()) * 32;
-    } else {
-        return A + ((slot * MCOL + lc) * nf<R>()) * 32;
-    }
+    return A + (slot * MCOL + lc) * 4 * 32;
 }
-template <typename R, bool H1> __host__ __device__ constexpr int a_cells() { return H1 ? RING * MT + 4 : RING * MCOL; }
 
 template <typename S, typename R>
 __device__ __forceinline__ Cell<R> raw_cell(const AdvArgs<S> &a, const View &v, int col, int row, int k) {
@@ -229,108 +218,28 @@ __device__ __forceinline__ Cell<R> raw_cell(const AdvArgs<S> &a, const View &v, 
     return ld_cell<S, R>(a, v, col, row, k);
 }
 
+// alpha_F at a staged cell: a ghost cell takes that of the in-grid cell it clamps to.
+template <typename S, typename R>
+__device__ __forceinline__ R alpha_F_clamped(const AdvArgs<S> &a, const View &v, int col, int row, int k) {
+    const int cc = col < 0 ? 0 : (col >= v.nr ? v.nr - 1 : col);
+    const int rr = row < 0 ? 0 : (row >= v.nz ? v.nz - 1 : row);
+    return alpha_F<S, R>(a, v, cc, rr, k);
+}
+
 // Stage cell (col, row) into ring slot `slot`, staged column lc (= col - i0 + 2): the flux
 // inputs in the arithmetic type R, and for the tile's own columns the state (J, H_r, H_Z) in
 // the storage type S, which the cell update accumulates into.
-template <typename S, typename R, bool H1>
+template <typename S, typename R>
 __device__ __forceinline__ void stage_cell(const AdvArgs<S> &a, const View &v, R *A, S *Hh, int slot, int lc,
                                            int col, int row, int k, int lane, R jeps) {
     Cell<S> c = raw_cell<S, S>(a, v, col, row, k);
     // the alpha_F loads are issued together with the state's (one load latency per cell)
-    R aF = R(0);
-    if (nf<R>() == 4) {
-        int cc = col < 0 ? 0 : (col >= v.nr ? v.nr - 1 : col);
-        int rr = row < 0 ? 0 : (row >= v.nz ? v.nz - 1 : row);
-        aF = alpha_F<S, R>(a, v, cc, rr, k);
-    }
+    const R aF = alpha_F_clamped<S, R>(a, v, col, row, k);
     CellF<R> f = cell_f<R>(R(c.J), R(c.Hr), R(c.HZ), jeps);
-    R *p = a_cell<R, H1>(A, slot, lc) + lane;
-    p[0] = f.J; p[32] = f.fr; p[64] = f.fZ;
-    if (nf<R>() == 4) p[96] = aF;
-    if (lc >= 2 && lc < 2 + MT) {
-        // the state in S; with S == R the ring's J is the state's J
-        constexpr int HF = sizeof(S) == sizeof(R) ? 2 : 3;
-        S *q = Hh + ((hslot(row) * MT + (lc - 2)) * HF) * 32 + lane;
-        q[0] = c.Hr; q[32] = c.HZ;
-        if (HF == 3) q[64] = c.J;
-    }
-}
-
-// ---- a row ahead by cp.async (FP64 arithmetic with per-lane staging) ----
-// The cell a staged stencil cell (col, row) copies, and the boundary rules that r_cell / z_cell
-// apply to the copy: rr for H_r, rz for H_Z (1: negate; 2: keep the part <= 0; 3: keep the
-// part >= 0). A corner cell (ghost in both directions) is never staged.
-struct CellSrc { int i, j, rr, rz; };
-__device__ __forceinline__ CellSrc cell_src(const View &v, int col, int row) {
-    CellSrc s{col, row, 0, 0};
-    if (col < 0) {
-        if (v.bcl == 0) { s.i = -1 - col; s.rr = 1; } else { s.i = 0; s.rr = 2; }
-    } else if (col >= v.nr) {
-        if (v.bcr == 0) { s.i = 2 * v.nr - 1 - col; s.rr = 1; } else { s.i = v.nr - 1; s.rr = 3; }
-    } else if (row < 0) {
-        if (v.bzb == 0) { s.j = -1 - row; s.rz = 1; } else { s.j = 0; s.rz = 2; }
-    } else if (row >= v.nz) {
-        if (v.bzt == 0) { s.j = 2 * v.nz - 1 - row; s.rz = 1; } else { s.j = v.nz - 1; s.rz = 3; }
-    }
-    return s;
-}
-template <typename S>
-__device__ __forceinline__ S bc_rule(S h, int rule) {
-    if (rule == 1) return -h;
-    if (rule == 2) return h < S(0) ? h : S(0);
-    if (rule == 3) return h > S(0) ? h : S(0);
-    return h;
-}
-// A raw slot holds one staged cell's inputs as copied: [4][32] values of the storage type
-// (J, H_r, H_Z of the cell it mirrors, and alpha_F, or H_voigt when alpha_F is derived, of the
-// in-grid cell it clamps to) and two doubles (alpha and alpha_cF of that cell).
-constexpr int RAW_SLOT = 4 * 32 + 2;   // doubles (storage FP64)
-
-// Copies of staged cell (col, row)'s inputs into the raw slot `dst` (cp.async, one 8-byte copy
-// per value; lanes outside the active bins copy no bin values; lane 0 copies the per-cell ones).
-template <typename S>
-__device__ __forceinline__ void raw_issue(const AdvArgs<S> &a, const View &v, S *dst, int col, int row, int k,
-                                          int lane, bool kact) {
-    const CellSrc s = cell_src(v, col, row);
-    const int cc = col < 0 ? 0 : (col >= v.nr ? v.nr - 1 : col);
-    const int rr = row < 0 ? 0 : (row >= v.nz ? v.nz - 1 : row);
-    const long long cla = (long long)cc + (long long)v.nr * rr;
-    if (kact) {
-        const long long x = v.o3 + (long long)k + (long long)a.nnu * ((long long)s.i + (long long)v.nr * s.j);
-        const long long xa = v.o3 + (long long)k + (long long)a.nnu * cla;
-        cp_async_el(dst + lane, a.J + x);
-        cp_async_el(dst + 32 + lane, a.Hr + x);
-        cp_async_el(dst + 64 + lane, a.HZ + x);
-        cp_async_el(dst + 96 + lane, a.aF ? a.aF + xa : a.Hv + xa);
-    }
-    if (lane == 0 && !a.aF) {
-        double *dsc = reinterpret_cast<double *>(dst + 128);
-        cp_async_el(dsc, a.alpha + v.oc + cla);
-        if (a.alpha_cF) cp_async_el(dsc + 1, a.alpha_cF + v.oc + cla);
-    }
-}
-// stage_cell from a raw slot that raw_issue filled (its copies complete and visible to the
-// warp): the same values through the same arithmetic.
-template <typename S, typename R, bool H1>
-__device__ __forceinline__ void stage_raw(const AdvArgs<S> &a, const View &v, const S *src, R *A, S *Hh, int slot,
-                                          int lc, int col, int row, int lane, R jeps) {
-    const CellSrc s = cell_src(v, col, row);
-    Cell<S> c;
-    c.J = src[lane];
-    c.Hr = bc_rule(src[32 + lane], s.rr);
-    c.HZ = bc_rule(src[64 + lane], s.rz);
-    R aF;
-    if (a.aF) {
-        aF = R(src[96 + lane]);
-    } else {
-        const double *dsc = reinterpret_cast<const double *>(src + 128);
-        aF = R(dsc[0]) * R(src[96 + lane]);
-        if (a.alpha_cF) aF = aF + R(dsc[1]);
-    }
-    CellF<R> f = cell_f<R>(R(c.J), R(c.Hr), R(c.HZ), jeps);
-    R *p = a_cell<R, H1>(A, slot, lc) + lane;
+    R *p = a_cell<R>(A, slot, lc) + lane;
     p[0] = f.J; p[32] = f.fr; p[64] = f.fZ; p[96] = aF;
     if (lc >= 2 && lc < 2 + MT) {
+        // the state in S; with S == R the ring's J is the state's J
         constexpr int HF = sizeof(S) == sizeof(R) ? 2 : 3;
         S *q = Hh + ((hslot(row) * MT + (lc - 2)) * HF) * 32 + lane;
         q[0] = c.Hr; q[32] = c.HZ;
@@ -348,7 +257,7 @@ __host__ __device__ constexpr int raw_tile_bytes() { return 3 * MCOL * 32 * (int
 // Stage cell (col, row) into ring slot `slot` from the raw tile, applying the ghost-cell rules
 // of r_cell / z_cell: a ghost column takes the column it mirrors from the same tile (every such
 // column lies in the tile: i0 < n_r), a ghost row's H_Z gets the rule of its boundary.
-template <typename S, typename R, bool H1>
+template <typename S, typename R>
 __device__ __forceinline__ void stage_from_raw(const AdvArgs<S> &a, const View &v, const S *raw, R *A, S *Hh,
                                                int slot, int lc, int col, int row, int k, int lane, R jeps, int i0) {
     int sc = lc;
@@ -371,16 +280,10 @@ __device__ __forceinline__ void stage_from_raw(const AdvArgs<S> &a, const View &
         if (v.bzt == 0) c.HZ = -c.HZ;
         else c.HZ = c.HZ > S(0) ? c.HZ : S(0);
     }
-    R aF = R(0);
-    if (nf<R>() == 4) {
-        int cc = col < 0 ? 0 : (col >= v.nr ? v.nr - 1 : col);
-        int rr = row >= v.nz ? v.nz - 1 : row;
-        aF = alpha_F<S, R>(a, v, cc, rr, k);
-    }
+    const R aF = alpha_F_clamped<S, R>(a, v, col, row, k);
     CellF<R> f = cell_f<R>(R(c.J), R(c.Hr), R(c.HZ), jeps);
-    R *p = a_cell<R, H1>(A, slot, lc) + lane;
-    p[0] = f.J; p[32] = f.fr; p[64] = f.fZ;
-    if (nf<R>() == 4) p[96] = aF;
+    R *p = a_cell<R>(A, slot, lc) + lane;
+    p[0] = f.J; p[32] = f.fr; p[64] = f.fZ; p[96] = aF;
     if (lc >= 2 && lc < 2 + MT) {
         constexpr int HF = sizeof(S) == sizeof(R) ? 2 : 3;
         S *q = Hh + ((hslot(row) * MT + (lc - 2)) * HF) * 32 + lane;
@@ -389,73 +292,113 @@ __device__ __forceinline__ void stage_from_raw(const AdvArgs<S> &a, const View &
     }
 }
 
-// A staged cell; with FP32 arithmetic also its alpha_F from the ring.
-template <typename R, bool H1>
-__device__ __forceinline__ CellF<R> staged(const R *A, int slot, int lc, int lane, R &aF) {
-    const R *p = a_cell<R, H1>(const_cast<R *>(A), slot, lc) + lane;
+// A staged cell and its alpha_F: four planes `ps` elements apart (J, f_r, f_Z, alpha_F).
+template <typename R>
+__device__ __forceinline__ CellF<R> staged(const R *p, int ps, R &aF) {
     CellF<R> c;
-    c.J = p[0]; c.fr = p[32]; c.fZ = p[64];
-    if (nf<R>() == 4) aF = p[96];
+    c.J = p[0]; c.fr = p[ps]; c.fZ = p[2 * ps];
+    aF = p[3 * ps];
     return c;
 }
 
-// With FP32 arithmetic the faces read u* (`up`) and the Z face's PLM intervals (`ivz`) where the
-// caller points, the warp's row slot in shared memory (see GEO_N below); with FP64 arithmetic
-// they load them from global memory where they are used and ignore the two pointers.
-// r face f (between cells f-1 and f) of row j held in ring slot `slot`; wl = f - i0 is the
-// staged column of the stencil's first cell (src/AdvectJandH.jl:641-968).
-template <typename S, typename R, int FLUX, bool H1>
-__device__ __forceinline__ void face_r_staged(const AdvArgs<S> &a, const View &v, const R *A, int slot, int wl,
-                                              int f, int j, int k, int lane, R jeps, const double *up,
-                                              const double *riv, R *F, R &kL, R &kR) {
-    const double us = *up;
+// The face between staged cells pi and pp (pm, p2: the stencil's outer cells) with the PLM intervals
+// ivp and u* (src/AdvectJandH.jl:641-968, 978-1289).
+template <typename R, int FLUX, bool ZDIR>
+__device__ __forceinline__ void face_cells(const R *pm, const R *pi, const R *pp, const R *p2, int ps, R jeps,
+                                           double us, const double *ivp, R *F, R &kL, R &kR, R &JR, R &HZR) {
     R d0, aFi, aFp, d3;
-    CellF<R> cm1 = staged<R, H1>(A, slot, wl, lane, d0);
-    CellF<R> ci = staged<R, H1>(A, slot, wl + 1, lane, aFi);
-    CellF<R> cp1 = staged<R, H1>(A, slot, wl + 2, lane, aFp);
-    CellF<R> cp2 = staged<R, H1>(A, slot, wl + 3, lane, d3);
+    const CellF<R> cm1 = staged<R>(pm, ps, d0);
+    const CellF<R> ci = staged<R>(pi, ps, aFi);
+    const CellF<R> cp1 = staged<R>(pp, ps, aFp);
+    const CellF<R> cp2 = staged<R>(p2, ps, d3);
     R iv[5];
 #pragma unroll
-    for (int t = 0; t < 5; t++) iv[t] = R(riv[t]);
-    Recon<R> q = reconstruct_f<R>(cm1, ci, cp1, cp2, iv, aFi, aFp, jeps);
-    R DrrL, DZZL, DrZL, DrrR, DZZR, DrZR;
-    D_from_f_n<R>(q.f_L, q.nr_L, q.nZ_L, DrrL, DZZL, DrZL);
-    D_from_f_n<R>(q.f_R, q.nr_R, q.nZ_R, DrrR, DZZR, DrZR);
-    R FJ, FHr, FHZ;
-    m1_flux<R, FLUX, false>(q.Hr_L, q.Hr_R, DrrL * q.J_L, DrrR * q.J_R, DrZL * q.J_L, DrZR * q.J_R, q, ci.J, cp1.J,
-                            FJ, FHr, FHZ);
-    R uc = R(us * kInvC);
-    F[0] = FJ + adv_flux(uc, q.J_L, q.J_R);
-    F[1] = FHr + adv_flux(uc, q.Hr_L, q.Hr_R);
-    F[2] = FHZ + adv_flux(uc, q.HZ_L, q.HZ_R);
-    kL = clamp01(R(1) - DrrL - DZZL) * q.J_L;
-    kR = (f == 0) ? k_phiphi_axis<R>(q.J_R, q.HZ_R, jeps) : clamp01(R(1) - DrrR - DZZR) * q.J_R;
+    for (int t = 0; t < 5; t++) iv[t] = R(ivp[t]);
+    face_flux<R, FLUX, ZDIR>(cm1, ci, cp1, cp2, iv, aFi, aFp, R(us * kInvC), jeps, F, kL, kR, JR, HZR);
+}
+template <typename R, int FLUX>
+__device__ __forceinline__ void face_z_cells(const R *pm, const R *pi, const R *pp, const R *p2, int ps, R jeps,
+                                             double us, const double *ivp, R *F) {
+    R kL, kR, JR, HZR;
+    face_cells<R, FLUX, true>(pm, pi, pp, p2, ps, jeps, us, ivp, F, kL, kR, JR, HZR);
+}
+// r face: K_phiphi of both sides too; on the axis (f = 0) the right side's is that of the axis.
+template <typename R, int FLUX>
+__device__ __forceinline__ void face_r_cells(const R *pm, const R *pi, const R *pp, const R *p2, int ps, bool axis,
+                                             R jeps, double us, const double *ivp, R *F, R &kL, R &kR) {
+    R JR, HZR;
+    face_cells<R, FLUX, false>(pm, pi, pp, p2, ps, jeps, us, ivp, F, kL, kR, JR, HZR);
+    if (axis) kR = k_phiphi_axis<R>(JR, HZR, jeps);
 }
 
-// Z face f (between rows f-1 and f) of column i, staged column lc (src/AdvectJandH.jl:978-1289).
-template <typename S, typename R, int FLUX, bool H1>
-__device__ __forceinline__ void face_z_staged(const AdvArgs<S> &a, const View &v, const R *A, int lc, int i, int f,
-                                              int k, int lane, R jeps, const double *ivz, const double *up, R *F) {
-    const double us = *up;
-    R d0, aFi, aFp, d3;
-    CellF<R> cm1 = staged<R, H1>(A, (f + 2) & (RING - 1), lc, lane, d0);     // row f-2
-    CellF<R> ci = staged<R, H1>(A, (f + 3) & (RING - 1), lc, lane, aFi);     // row f-1
-    CellF<R> cp1 = staged<R, H1>(A, f & (RING - 1), lc, lane, aFp);          // row f
-    CellF<R> cp2 = staged<R, H1>(A, (f + 1) & (RING - 1), lc, lane, d3);     // row f+1
-    R iv[5];
-#pragma unroll
-    for (int t = 0; t < 5; t++) iv[t] = R(ivz[t]);
-    Recon<R> q = reconstruct_f<R>(cm1, ci, cp1, cp2, iv, aFi, aFp, jeps);
-    R DrrL, DZZL, DrZL, DrrR, DZZR, DrZR;
-    D_from_f_n<R>(q.f_L, q.nr_L, q.nZ_L, DrrL, DZZL, DrZL);
-    D_from_f_n<R>(q.f_R, q.nr_R, q.nZ_R, DrrR, DZZR, DrZR);
-    R FJ, FHr, FHZ;
-    m1_flux<R, FLUX, true>(q.HZ_L, q.HZ_R, DrZL * q.J_L, DrZR * q.J_R, DZZL * q.J_L, DZZR * q.J_R, q, ci.J, cp1.J,
-                           FJ, FHr, FHZ);
-    R uc = R(us * kInvC);
-    F[0] = FJ + adv_flux(uc, q.J_L, q.J_R);
-    F[1] = FHr + adv_flux(uc, q.Hr_L, q.Hr_R);
-    F[2] = FHZ + adv_flux(uc, q.HZ_L, q.HZ_R);
+// The scalars of one cell's update: face areas, c~dt/dV's factors, the velocity gradients.
+struct UpdGeo {
+    double ArL, ArR, AZL, AZR, idv, ga, gb, gc, gd, ge, irc;
+};
+
+// The cell update (src/AdvectJandH.jl:1302-1382) of the state (uJ, uHr, uHZ) from the fluxes of
+// its faces (zL, zR; FL, FR: planes `ps` apart of flux J, H_r, H_Z, K left, K right), written at x.
+template <typename S, typename R>
+__device__ __forceinline__ void cell_update(const AdvArgs<S> &a, long long x, S uJ, S uHr, S uHZ, const R *zL,
+                                            const R *zR, const R *FL, const R *FR, int ps, const UpdGeo &g,
+                                            double ctdt, R jeps) {
+    const double ctdt_c = ctdt * kInvC;
+    const R sJ = R(uJ), sHr = R(uHr), sHZ = R(uHZ);
+    const double fac = ctdt * g.idv;
+    // increments in R, accumulated into the state in S
+    S Jn, Hrn, HZn;
+    const S ujeps = S(a.jeps);
+    if (sizeof(R) == 8) {
+        R fr_ = R(fac);
+        Jn = uJ - S(fr_ * ((R(g.ArR) * FR[0] - R(g.ArL) * FL[0]) + (R(g.AZR) * zR[0] - R(g.AZL) * zL[0])));
+        HZn = uHZ - S(fr_ * ((R(g.ArR) * FR[2 * ps] - R(g.ArL) * FL[2 * ps]) + (R(g.AZR) * zR[2] - R(g.AZL) * zL[2])));
+        Hrn = uHr - S(fr_ * ((R(g.ArR) * FR[ps] - R(g.ArL) * FL[ps]) + (R(g.AZR) * zR[1] - R(g.AZL) * zL[1])));
+    } else {
+        R wrL = R(fac * g.ArL), wrR = R(fac * g.ArR), wzL = R(fac * g.AZL), wzR = R(fac * g.AZR);
+        Jn = uJ - S((wrR * FR[0] - wrL * FL[0]) + (wzR * zR[0] - wzL * zL[0]));
+        HZn = uHZ - S((wrR * FR[2 * ps] - wrL * FL[2 * ps]) + (wzR * zR[2] - wzL * zL[2]));
+        Hrn = uHr - S((wrR * FR[ps] - wrL * FL[ps]) + (wzR * zR[1] - wzL * zL[1]));
+    }
+    const S Jn0 = Jn;
+    Jn = Jn > ujeps ? Jn : ujeps;
+    const R ga = R(g.ga), gb = R(g.gb), gc = R(g.gc), gd = R(g.gd), ge = R(g.ge);
+    R DdU = work_rate<R>(sJ, sHr, sHZ, jeps, R(a.heps2), ga, gb + gc, gd, ga + gd + ge);
+    R Kav = R(0.5) * (FL[4 * ps] + FR[3 * ps]);
+    if (sizeof(R) == 8)
+        Hrn += S(R(ctdt) * Kav * R(g.irc));
+    else
+        Hrn += S(R(ctdt * g.irc) * Kav);
+    R cc = R(ctdt_c);
+    R dHr = -cc * (sHr * ga + sHZ * gb);
+    R dHZ = -cc * (sHr * gc + sHZ * gd);
+    Hrn = Hrn + S(dHr);
+    HZn = HZn + S(dHZ);
+    Jn = Jn - S(cc * DdU * sJ);
+    if (a.tape) {
+        // the values before the floors and the causality limiter, for the adjoint
+        a.tape[x] = double(Jn0);
+        a.tape[x + a.tape_stride] = double(Jn);
+        a.tape[x + 2 * a.tape_stride] = double(Hrn);
+        a.tape[x + 3 * a.tape_stride] = double(HZn);
+    }
+    Jn = Jn > ujeps ? Jn : ujeps;
+    S H2 = Hrn * Hrn + HZn * HZn;
+    if (H2 > Jn * Jn) {
+        S fsc;
+        if constexpr (sizeof(S) == 4) {
+            // a flushed (zero) root of a subnormal |H|^2 scales H to zero
+            const S Hm = rsq(H2);
+            fsc = Hm > S(0) ? Jn / Hm : S(0);
+        } else {
+            // |H|^2 > J^2 >= jeps^2, far inside the normal range
+            fsc = Jn * rsqrt_nr(H2);
+        }
+        Hrn *= fsc;
+        HZn *= fsc;
+    }
+    a.Jo[x] = S(Jn);
+    a.Hro[x] = S(Hrn);
+    a.HZo[x] = S(HZn);
 }
 
 // The per-row scalars a warp needs: the cell's geometry and velocity gradients (0..10), u*_r of
@@ -505,44 +448,30 @@ __device__ __forceinline__ double geo_fetch(const double *src, int stride, int j
     return (src != nullptr && j < j1) ? __ldg(src + (long long)stride * j) : 0.0;
 }
 
-// Shared memory of the advection tile before the bulk-copy staging area, in bytes.
-// PFR: every staged input copied a row ahead by per-lane cp.async into raw slots (the own
-// column's row j+3 and warp 8's halo cells of row j+1, while row j's faces and update run),
-// with the one-row halo ring of a_cell paying for the slots: FP64 arithmetic with per-lane
-// staging, 76 KB per CTA, three CTAs per SM. FP64 advection 0.288 -> 0.282 ms at 256^2 x 64,
-// 1.219 -> 1.169 ms at 512^2 x 128, 4.82 -> 4.64 ms at 1024^2 x 128; bit for bit unchanged.
-template <typename R, bool TMA> __host__ __device__ constexpr bool adv_pfr() { return !TMA && sizeof(R) == 8; }
-
-// Shared memory of the advection tile before the bulk-copy staging area, in bytes (with PFR
-// the one-row halo ring and the raw slots).
-template <typename S, typename R, bool PFR>
+// Shared memory of the bulk-copy tile before its raw staging area, in bytes.
+template <typename S, typename R>
 __host__ __device__ constexpr size_t adv_smem_base() {
-    return sizeof(R) * 32 * (a_cells<R, PFR>() * nf<R>() + (MT + 1) * 5) +
+    return sizeof(R) * 32 * (RING * MCOL * 4 + (MT + 1) * 5) +
            sizeof(S) * 32 * HRING * MT * (sizeof(S) == sizeof(R) ? 2 : 3) +
-           sizeof(double) * (MWARPS * 2 * GEO_N + (MT + 1) * 5) +
-           (PFR ? sizeof(double) * (MT + 4) * RAW_SLOT : 0);
+           sizeof(double) * (MWARPS * 2 * GEO_N + (MT + 1) * 5);
 }
 __host__ __device__ constexpr size_t adv_tma_off(size_t base) { return (base + 127) / 128 * 128; }
 
-// TMA: rows j0+2 .. of the tile arrive as bulk tensor copies (one 32-bin x MCOL-column box per
-// field, issued by one thread a row ahead of their use into one raw tile, completed on an
-// mbarrier) instead of per-lane loads; the converting warps apply the ghost-cell rules. The
-// first rows (j0-2 .. j0+1) are staged by per-lane loads while the first copy is in flight.
-// One tile of the advection (tile `tile` of the work list) by the calling CTA of MTHREADS
-// threads, in dynamic shared memory `adv_smem`: the body of k_advect, also run by the persistent
-// batch kernel.
-template <typename S, typename R, int FLUX, bool TMA>
-__device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsigned char *adv_smem) {
+// The advection with bulk tensor copies: rows j0+2 .. of the tile arrive as copies of one 32-bin x
+// MCOL-column box per field, issued by one thread a row ahead of their use into one raw tile,
+// completed on an mbarrier; the converting warps apply the ghost-cell rules. The first rows
+// (j0-2 .. j0+1) are staged by per-lane loads while the first copy is in flight. The box is fixed
+// when the tensor map is encoded, so this form keeps the fixed tile of 8 columns x 32 bins; the
+// packed tile below is the default (see there).
+template <typename S, typename R, int FLUX>
+__device__ __forceinline__ void advect_tile_tma(const AdvArgs<S> &a, int tile, unsigned char *adv_smem) {
     constexpr int HF = sizeof(S) == sizeof(R) ? 2 : 3;
-    constexpr int NF = nf<R>();
-    constexpr bool PFR = adv_pfr<R, TMA>();
-    R *A = reinterpret_cast<R *>(adv_smem);                            // a_cells cells of [NF][32] (a_cell)
-    S *Hh = reinterpret_cast<S *>(A + a_cells<R, PFR>() * NF * 32);    // [HRING][MT][HF][32]
-    R *Fr = reinterpret_cast<R *>(Hh + HRING * MT * HF * 32);           // [MT+1][5][32]
+    R *A = reinterpret_cast<R *>(adv_smem);                            // [RING][MCOL][4][32]
+    S *Hh = reinterpret_cast<S *>(A + RING * MCOL * 4 * 32);           // [HRING][MT][HF][32]
+    R *Fr = reinterpret_cast<R *>(Hh + HRING * MT * HF * 32);          // [MT+1][5][32]
     double *geo = reinterpret_cast<double *>(Fr + (MT + 1) * 5 * 32);  // [MWARPS][2][GEO_N]: the row slots
-    double *riv = geo + MWARPS * 2 * GEO_N;                             // [MT+1][5]: the r faces' intervals
-    double *rawp = riv + (MT + 1) * 5;                                  // PFR: [MT + 4][RAW_SLOT] raw slots
-    constexpr size_t toff = adv_tma_off(adv_smem_base<S, R, false>());
+    double *riv = geo + MWARPS * 2 * GEO_N;                            // [MT+1][5]: the r faces' intervals
+    constexpr size_t toff = adv_tma_off(adv_smem_base<S, R>());
     S *raw = reinterpret_cast<S *>(adv_smem + toff);                                   // [3][MCOL][32]
     unsigned long long *bar = reinterpret_cast<unsigned long long *>(adv_smem + toff + raw_tile_bytes<S>());
     int *abort_flag = reinterpret_cast<int *>(bar + 1);
@@ -581,50 +510,29 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
         return;
     }
 
-    if constexpr (TMA) {
-        if (threadIdx.x == 0) {
-            mbar_init(bar, 1);
-            *abort_flag = 0;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0 && j0 + 2 <= rlast) issue_row(j0 + 2);
+    if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        *abort_flag = 0;
     }
-    // PFR: the first row-ahead copies (the own column's row j0+2, warp 8's halo cells of row j0)
-    // go out before the prologue's own loads and are waited for at its end
-    S *rawo = reinterpret_cast<S *>(rawp + w * RAW_SLOT);   // own warps; halo cell q: slot MT + q
+    __syncthreads();
+    if (threadIdx.x == 0 && j0 + 2 <= rlast) issue_row(j0 + 2);
     const int hl[4] = {0, 1, MT + 2, MT + 3};
-    if constexpr (PFR) {
-        if (own) {
-            const int r = j0 + 2;
-            if (r <= j1 + 1 && col <= v.nr + 1 && r <= v.nz + 1 && !(col >= v.nr && r >= v.nz))
-                raw_issue<S>(a, v, rawo, col, r, k, lane, kact);
-        } else if (j0 < j1) {
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int c2 = i0 - 2 + hl[q];
-                if (c2 <= v.nr + 1) raw_issue<S>(a, v, reinterpret_cast<S *>(rawp + (MT + q) * RAW_SLOT), c2, j0, k, lane, kact);
-            }
-        }
-        cp_async_commit();
-    }
     // prologue: own columns, rows j0-2 .. j0+1
     if (own && kact && col <= v.nr + 1) {
         for (int r = j0 - 2; r <= j0 + 1; r++) {
             bool gcol = col >= v.nr, grow = (r < 0 || r >= v.nz);
             if (r < -2 || r > v.nz + 1 || (gcol && grow)) continue;
-            stage_cell<S, R, PFR>(a, v, A, Hh, r & (RING - 1), w + 2, col, r, k, lane, jeps);
+            stage_cell<S, R>(a, v, A, Hh, r & (RING - 1), w + 2, col, r, k, lane, jeps);
         }
     }
-    if constexpr (TMA) {
-        // with bulk copies the halo columns of a row come with its copy, two rows before the
-        // r faces read them: the prologue stages those of rows j0 and j0+1
-        if (!own && kact) {
-            for (int r = j0; r <= j0 + 1 && r < j1 && r < v.nz; r++) {
+    // the halo columns of a row come with its copy, two rows before the r faces read them: the
+    // prologue stages those of rows j0 and j0+1
+    if (!own && kact) {
+        for (int r = j0; r <= j0 + 1 && r < j1 && r < v.nz; r++) {
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    int c2 = i0 - 2 + hl[q];
-                    if (c2 <= v.nr + 1) stage_cell<S, R, PFR>(a, v, A, Hh, r & (RING - 1), hl[q], c2, r, k, lane, jeps);
-                }
+            for (int q = 0; q < 4; q++) {
+                int c2 = i0 - 2 + hl[q];
+                if (c2 <= v.nr + 1) stage_cell<S, R>(a, v, A, Hh, r & (RING - 1), hl[q], c2, r, k, lane, jeps);
             }
         }
     }
@@ -639,19 +547,19 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
         const int f = i0 + t / 5;
         riv[t] = f <= v.nr ? __ldg(a.rint + v.orint + 5 * f + t % 5) : 0.0;
     }
-    if constexpr (PFR) cp_async_wait<0>();
     __syncthreads();
+    // the Z face f of the own column: rows f-2 .. f+1 of the ring
+    auto zface = [&](int f, const double *ivz, const double *up, R *F) {
+        auto row = [&](int r) { return a_cell<R>(A, r & (RING - 1), w + 2) + lane; };
+        face_z_cells<R, FLUX>(row(f + 2), row(f + 3), row(f), row(f + 1), 32, jeps, *up, ivz, F);
+    };
     R zL[3] = {R(0), R(0), R(0)};
     if (own && kact && col < v.nr)
-        face_z_staged<S, R, FLUX, PFR>(a, v, A, w + 2, col, j0, k, lane, jeps, a.zint + v.ozint + 5 * j0,
-                                  a.u_Z_star + v.ozf + col + (long long)v.nr * j0, zL);   // face j0
+        zface(j0, a.zint + v.ozint + 5 * j0, a.u_Z_star + v.ozf + col + (long long)v.nr * j0, zL);   // face j0
 
     const double ctdt = v.ctdt;
-    const double ctdt_c = ctdt * kInvC;
-    // FP32 arithmetic (56 registers at 4 CTAs per SM) holds the next row's scalar in a register
-    // and keeps one buffer; FP64 arithmetic, at its register limit, copies it with cp.async into
-    // the other buffer (mixed advection 0.183 ms with the register, 0.189 ms with the copy;
-    // FP64 advection 0.333 -> 0.320 ms with the copy, at 256^2 x 64)
+    // FP32 arithmetic holds the next row's scalar in a register and keeps one buffer; FP64
+    // arithmetic, at its register limit, copies it with cp.async into the other buffer
     constexpr bool GREG = sizeof(R) == 4;
     for (int j = j0; j < j1; j++) {
         double *g = GREG ? g0 : g0 + ((j - j0) & 1) * GEO_N;
@@ -666,175 +574,59 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
             }
             cp_async_commit();
         }
-        if constexpr (TMA) {
-            // (A) row j+2 from its bulk copy: the own column, and (warp 8) the halo columns
-            const int r = j + 2;
-            if (r <= rlast) {
-                if (!mbar_wait_bounded(bar, (unsigned)((r - (j0 + 2)) & 1))) {
-                    *abort_flag = 1;
-                    atomicOr(a.err, ERRB_TIMEOUT);
-                } else if (kact) {
-                    const bool grow = r >= v.nz;
-                    if (own) {
-                        if (col <= v.nr + 1 && !(col >= v.nr && grow))
-                            stage_from_raw<S, R, PFR>(a, v, raw, A, Hh, r & (RING - 1), w + 2, col, r, k, lane, jeps, i0);
-                    } else if (!grow && r < j1) {
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            int c2 = i0 - 2 + hl[q];
-                            if (c2 <= v.nr + 1)
-                                stage_from_raw<S, R, PFR>(a, v, raw, A, Hh, r & (RING - 1), hl[q], c2, r, k, lane, jeps, i0);
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-            if (*reinterpret_cast<volatile int *>(abort_flag)) {
-                // a copy never arrived: wait once more (bounded) for it, then leave the tile
-                if (threadIdx.x == 0) mbar_wait_bounded(bar, (unsigned)((r - (j0 + 2)) & 1));
-                return;
-            }
-            // the raw tile is free again: fetch row j+3 while this row's faces and update run
-            if (threadIdx.x == 0 && j + 3 <= rlast) issue_row(j + 3);
-        } else if constexpr (PFR) {
-            // (A) from the raw slots: the own column's row j+2 and warp 8's halo cells of row j,
-            // copied a row ago; then the copies of the next ones go out and land while this
-            // row's faces and update run (the wait at the end of the row)
-            if (own) {
-                const int r = j + 2;
-                if (kact && col <= v.nr + 1 && r <= v.nz + 1 && !(col >= v.nr && r >= v.nz))
-                    stage_raw<S, R, PFR>(a, v, rawo, A, Hh, r & (RING - 1), w + 2, col, r, lane, jeps);
-                __syncwarp();
-                const int rn = r + 1;
-                if (rn <= j1 + 1 && col <= v.nr + 1 && rn <= v.nz + 1 && !(col >= v.nr && rn >= v.nz))
-                    raw_issue<S>(a, v, rawo, col, rn, k, lane, kact);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int c2 = i0 - 2 + hl[q];
-                    if (kact && c2 <= v.nr + 1)
-                        stage_raw<S, R, PFR>(a, v, reinterpret_cast<const S *>(rawp + (MT + q) * RAW_SLOT), A, Hh,
-                                             j & (RING - 1), hl[q], c2, j, lane, jeps);
-                }
-                __syncwarp();
-                if (j + 1 < j1) {
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int c2 = i0 - 2 + hl[q];
-                        if (c2 <= v.nr + 1)
-                            raw_issue<S>(a, v, reinterpret_cast<S *>(rawp + (MT + q) * RAW_SLOT), c2, j + 1, k, lane, kact);
-                    }
-                }
-            }
-            cp_async_commit();
-            __syncthreads();
-        } else {
-            // (A) stage row j+2 of the own column; warp 8 stages the halo columns of row j (spread
-            // over four warps instead, one halo cell each, the FP64 advection took 0.336 ms
-            // against 0.322 ms at 256^2 x 64, before the row-ahead copies)
-            if (kact) {
+        // (A) row j+2 from its bulk copy: the own column, and (warp 8) the halo columns
+        const int r = j + 2;
+        if (r <= rlast) {
+            if (!mbar_wait_bounded(bar, (unsigned)((r - (j0 + 2)) & 1))) {
+                *abort_flag = 1;
+                atomicOr(a.err, ERRB_TIMEOUT);
+            } else if (kact) {
+                const bool grow = r >= v.nz;
                 if (own) {
-                    int r = j + 2;
-                    bool gcol = col >= v.nr, grow = r >= v.nz;
-                    if (col <= v.nr + 1 && r <= v.nz + 1 && !(gcol && grow))
-                        stage_cell<S, R, PFR>(a, v, A, Hh, r & (RING - 1), w + 2, col, r, k, lane, jeps);
-                } else {
+                    if (col <= v.nr + 1 && !(col >= v.nr && grow))
+                        stage_from_raw<S, R>(a, v, raw, A, Hh, r & (RING - 1), w + 2, col, r, k, lane, jeps, i0);
+                } else if (!grow && r < j1) {
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         int c2 = i0 - 2 + hl[q];
                         if (c2 <= v.nr + 1)
-                            stage_cell<S, R, PFR>(a, v, A, Hh, j & (RING - 1), hl[q], c2, j, k, lane, jeps);
+                            stage_from_raw<S, R>(a, v, raw, A, Hh, r & (RING - 1), hl[q], c2, r, k, lane, jeps, i0);
                     }
                 }
             }
-            __syncthreads();
         }
+        __syncthreads();
+        if (*reinterpret_cast<volatile int *>(abort_flag)) {
+            // a copy never arrived: wait once more (bounded) for it, then leave the tile
+            if (threadIdx.x == 0) mbar_wait_bounded(bar, (unsigned)((r - (j0 + 2)) & 1));
+            return;
+        }
+        // the raw tile is free again: fetch row j+3 while this row's faces and update run
+        if (threadIdx.x == 0 && j + 3 <= rlast) issue_row(j + 3);
         // (B) the r face left of the own column (warp 8: the tile's right face), the Z face j+1/2
         const int f = i0 + w;
         R zR[3] = {R(0), R(0), R(0)};
         if (kact && f <= v.nr) {
             R F[3], kL, kR;
-            face_r_staged<S, R, FLUX, PFR>(a, v, A, j & (RING - 1), w, f, j, k, lane, jeps, g + G_UR, riv + 5 * w, F,
-                                      kL, kR);
+            const R *p0 = a_cell<R>(A, j & (RING - 1), w) + lane;
+            face_r_cells<R, FLUX>(p0, p0 + 128, p0 + 256, p0 + 384, 32, f == 0, jeps, g[G_UR], riv + 5 * w, F, kL, kR);
             R *p = Fr + (w * 5) * 32 + lane;
             p[0] = F[0]; p[32] = F[1]; p[64] = F[2]; p[96] = kL; p[128] = kR;
         }
-        if (own && kact && col < v.nr)
-            face_z_staged<S, R, FLUX, PFR>(a, v, A, w + 2, col, j + 1, k, lane, jeps, g + G_ZIV, g + G_UZ, zR);
+        if (own && kact && col < v.nr) zface(j + 1, g + G_ZIV, g + G_UZ, zR);
         __syncthreads();
-        // (C) cell update, src/AdvectJandH.jl:1302-1382
+        // (C) cell update
         if (own && col < v.nr && k < a.nnu) {
-            const int i = col;
-            long long cl = (long long)i + (long long)v.nr * j;
-            long long x = v.o3 + (long long)k + (long long)a.nnu * cl;
+            long long x = v.o3 + (long long)k + (long long)a.nnu * ((long long)col + (long long)v.nr * j);
             if (!kact) {
                 a.Jo[x] = a.J[x]; a.Hro[x] = a.Hr[x]; a.HZo[x] = a.HZ[x];
             } else {
                 const S *pH = Hh + ((hslot(j) * MT + w) * HF) * 32 + lane;
-                const S uHr = pH[0], uHZ = pH[32];
-                const S uJ = HF == 3 ? pH[64] : S(a_cell<R, PFR>(A, j & (RING - 1), w + 2)[lane]);
-                const R sJ = R(uJ), sHr = R(uHr), sHZ = R(uHZ);
-                R Drr, DZZ, DrZ;
-                D_edd<R>(sHr, sHZ, sJ, jeps, R(a.heps2), Drr, DZZ, DrZ);
+                const S uJ = HF == 3 ? pH[64] : S(a_cell<R>(A, j & (RING - 1), w + 2)[lane]);
                 const R *FL = Fr + (w * 5) * 32 + lane;
-                const R *FR = FL + 5 * 32;
-                const double ArL = g[G_ARL], ArR = g[G_ARR], AZL = g[G_AZL], AZR = g[G_AZR];
-                const double fac = ctdt * g[G_IDV];
-                // increments in R, accumulated into the state in S
-                S Jn, Hrn, HZn;
-                const S ujeps = S(a.jeps);
-                if (sizeof(R) == 8) {
-                    R fr_ = R(fac);
-                    Jn = uJ - S(fr_ * ((R(ArR) * FR[0] - R(ArL) * FL[0]) + (R(AZR) * zR[0] - R(AZL) * zL[0])));
-                    HZn = uHZ - S(fr_ * ((R(ArR) * FR[64] - R(ArL) * FL[64]) + (R(AZR) * zR[2] - R(AZL) * zL[2])));
-                    Hrn = uHr - S(fr_ * ((R(ArR) * FR[32] - R(ArL) * FL[32]) + (R(AZR) * zR[1] - R(AZL) * zL[1])));
-                } else {
-                    R wrL = R(fac * ArL), wrR = R(fac * ArR), wzL = R(fac * AZL), wzR = R(fac * AZR);
-                    Jn = uJ - S((wrR * FR[0] - wrL * FL[0]) + (wzR * zR[0] - wzL * zL[0]));
-                    HZn = uHZ - S((wrR * FR[64] - wrL * FL[64]) + (wzR * zR[2] - wzL * zL[2]));
-                    Hrn = uHr - S((wrR * FR[32] - wrL * FL[32]) + (wzR * zR[1] - wzL * zL[1]));
-                }
-                const S Jn0 = Jn;
-                Jn = Jn > ujeps ? Jn : ujeps;
-                const R ga = R(g[G_DURDR]), gb = R(g[G_DURDZ]), gc = R(g[G_DUZDR]), gd = R(g[G_DUZDZ]);
-                const R ge = R(g[G_UROR]);
-                R DdU = d_colon_grad_u<R>(Drr, DrZ, DZZ, ga, gb, gc, gd, ge);
-                R Kav = R(0.5) * (FL[128] + FR[96]);
-                if (sizeof(R) == 8)
-                    Hrn += S(R(ctdt) * Kav * R(g[G_IRC]));
-                else
-                    Hrn += S(R(ctdt * g[G_IRC]) * Kav);
-                R cc = R(ctdt_c);
-                R dHr = -cc * (sHr * ga + sHZ * gb);
-                R dHZ = -cc * (sHr * gc + sHZ * gd);
-                Hrn = Hrn + S(dHr);
-                HZn = HZn + S(dHZ);
-                Jn = Jn - S(cc * DdU * sJ);
-                if (a.tape) {
-                    // the values before the floors and the causality limiter, for the adjoint
-                    a.tape[x] = double(Jn0);
-                    a.tape[x + a.tape_stride] = double(Jn);
-                    a.tape[x + 2 * a.tape_stride] = double(Hrn);
-                    a.tape[x + 3 * a.tape_stride] = double(HZn);
-                }
-                Jn = Jn > ujeps ? Jn : ujeps;
-                S H2 = Hrn * Hrn + HZn * HZn;
-                if (H2 > Jn * Jn) {
-                    S fsc;
-                    if constexpr (sizeof(S) == 4) {
-                        // a flushed (zero) root of a subnormal |H|^2 scales H to zero
-                        const S Hm = rsq(H2);
-                        fsc = Hm > S(0) ? Jn / Hm : S(0);
-                    } else {
-                        // |H|^2 > J^2 >= jeps^2, far inside the normal range
-                        fsc = Jn * rsqrt_nr(H2);
-                    }
-                    Hrn *= fsc;
-                    HZn *= fsc;
-                }
-                a.Jo[x] = S(Jn);
-                a.Hro[x] = S(Hrn);
-                a.HZo[x] = S(HZn);
+                const UpdGeo ug = {g[G_ARL], g[G_ARR], g[G_AZL], g[G_AZR], g[G_IDV], g[G_DURDR], g[G_DURDZ],
+                                   g[G_DUZDR], g[G_DUZDZ], g[G_UROR], g[G_IRC]};
+                cell_update<S, R>(a, x, uJ, pH[0], pH[32], zL, zR, FL, FL + 5 * 32, 32, ug, ctdt, jeps);
             }
         }
         zL[0] = zR[0]; zL[1] = zR[1]; zL[2] = zR[2];
@@ -852,10 +644,439 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
     }
 }
 
-template <typename S, typename R, int FLUX, int MINB, bool TMA>
-__global__ void __launch_bounds__(MTHREADS, MINB) k_advect(AdvArgs<S> a) {
+template <typename S, typename R, int FLUX, int MINB>
+__global__ void __launch_bounds__(MTHREADS, MINB) k_advect_tma(AdvArgs<S> a) {
     extern __shared__ __align__(128) unsigned char adv_smem[];
-    advect_tile<S, R, FLUX, TMA>(a, blockIdx.x, adv_smem);
+    advect_tile_tma<S, R, FLUX>(a, blockIdx.x, adv_smem);
+}
+
+// ---- k_advect: the packed tile ---------------------------------------------------------------
+//
+// A CTA of 256 threads owns `ncol` columns (r) x `rows` rows (Z) x `nbk` bins of one cloud and
+// marches up its rows. The active window holds nact = kmax - kmin + 1 of the n_nu bins (24 of 48
+// in the ragged batches, 50 of 64 in the benchmark's cloud), so lanes fixed to bins stand idle for
+// a quarter to two thirds of the work: here the window is cut into nb chunks of nbk = ceil(nact /
+// nb) bins and the threads are dealt out over (column, bin) pairs, thread t to column t / nbk and
+// bin t % nbk of the chunk; a row's cells are runs of nbk consecutive bins, so a warp's loads stay
+// a few contiguous runs. The window is known on the device only, so the CTA works out its own
+// nb, nbk and ncol (pack_bins) from its place in the cloud's work list, which is as long as the
+// widest need; CTAs beyond the window's share leave at once. Bins outside the window are copied
+// through, the rows of a tile shared out over its chunks.
+// A ring of four rows in shared memory holds, for the ncol + 1 columns that have an r face, what
+// every face needs: J, the reduced fluxes H / max(J, Jeps) (so the reciprocal of J is taken once per
+// cell) and alpha_F; the three columns beyond (two left, one right) keep the current row alone. Per
+// row: stage row j+2 -> barrier -> each thread computes the r face on its left into shared memory
+// and its Z face j+1/2 into registers -> barrier -> the cell update of row j from the two r faces in
+// shared memory and the Z faces j-1/2 (carried) and j+1/2. Faces never touch HBM. Every staged
+// input comes a row ahead by cp.async when S and R agree (FP64, FP32 storage); the mixed form has no
+// room for the landing rows at four CTAs per SM and loads its rows where it stages them.
+// Bound by dependent FP64 latency and instruction issue (24 warps per SM, 80 registers: FP64 pipe 36 %,
+// issue 60 %). Per launch, against tiles of 8 columns x 32 fixed bins with one warp per column and
+// branches in the faces: 256^2 x 64 with 53 active bins 262 -> 202 us (FP64), 187 -> 176 us (mixed),
+// 171 -> 140 us (FP32 storage); 512^2 x 128 with 85 active 1877 -> 1105 us; 24 clouds of 17..96
+// cells a side x 48 bins 254 -> 134 us; 131 x 203 x 50 with the HLL flux 155 -> 95 us. Executed warp
+// instructions at 256^2 x 64: 153 -> 125 million from the branch-free faces. A ninth warp for the
+// halo columns and the right face (288 threads, 72 registers) was slower (210 us): it stages four
+// cells to the others' one and holds up the row's barrier.
+constexpr int PT = 256;                // threads
+constexpr int PNC = 18;                // most columns with an r face (own columns + 1)
+constexpr int PHALO = 96;              // 3 halo columns x 32 bins
+// Per-row scalars of each column: areas of its left r face and of its two Z faces, 1/dV, the
+// velocity gradients, u*_r of the left r face, u*_Z of the Z face above, and, for the row staged
+// three rows later, alpha and alpha_cF; then the PLM intervals of the Z face above the row.
+enum { P_AR, P_UR, P_AZL, P_AZR, P_IDV, P_DURDR, P_DURDZ, P_DUZDR, P_DUZDZ, P_UROR, P_UZ, P_AL, P_ACF, P_N };
+constexpr int PGEO = P_N * PNC + 5;
+static_assert(PGEO <= PT, "one copy per thread");
+
+// How a window of nact bins of a cloud of nr columns is cut: nb chunks of nbk <= 32 bins, tiles of
+// ncol columns (ncol + 1 columns of nbk bins fit the CTA's threads), the fewest tiles of four
+// candidates; then the columns are shared out evenly over the tiles.
+struct Pack { int nb, nbk, ncol, nct; };
+__host__ __device__ __forceinline__ int pack_cost(int nact, int nr, int nb) {
+    const int nbk = (nact + nb - 1) / nb;
+    int nc = PT / nbk - 1;
+    nc = nc < PNC - 1 ? nc : PNC - 1;
+    return nb * ((nr + nc - 1) / nc);
+}
+__host__ __device__ __forceinline__ Pack pack_of(int nact, int nr, int nb) {
+    Pack p;
+    p.nb = nb;
+    p.nbk = (nact + nb - 1) / nb;
+    p.nct = pack_cost(nact, nr, nb) / nb;
+    p.ncol = (nr + p.nct - 1) / p.nct;
+    return p;
+}
+// device: lane q of every warp weighs candidate nb0 + q
+__device__ __forceinline__ Pack pack_bins(int nact, int nr) {
+    const int q = threadIdx.x & 3, nb0 = (nact + 31) / 32;
+    const unsigned key = (unsigned)pack_cost(nact, nr, nb0 + q) * 4u + (unsigned)q;
+    return pack_of(nact, nr, nb0 + (int)(__reduce_min_sync(0xffffffffu, key) & 3u));
+}
+// Rows per tile when the caller leaves them open: nz rows, tpb tiles to a band of rows, for a
+// cloud whose share of the GPU's resident CTAs is `share`. A field that one wave of tiles of up to 12
+// rows covers is cut until its tiles just fill the wave, down to two rows: its time is a tile's
+// latency (64^2 x 64: 25 us with 2 rows, 28 / 36 / 58 us with 4 / 8 / 16; 131 x 203 x 50: 95 us with 10,
+// 105 / 112 with 8 / 16). Beyond, a tile's prologue (about 1.3 rows of work) pulls towards tall tiles
+// and the last wave, which runs partly empty, towards short ones: rows^2 = 2 x the rows of a single
+// wave balances the two (256^2 x 64: 200 us with 8 or 9 rows, 205 / 225 with 16 / 4; the 24 clouds
+// 134 us with 8, 156 / 145 with 16 / 4; 512^2 x 128: 1099 us with 16, 1164 with 8).
+constexpr int kPackRows = 16;
+__host__ __device__ __forceinline__ int pack_rows(int tpb, int nz, int share) {
+    const int wave = (tpb * nz + share - 1) / share;          // rows per tile of a single wave
+    int rows = wave;
+    if (wave > 12) {
+        rows = 4;
+        while (rows < kPackRows && rows * rows < 2 * wave) rows++;
+    }
+    rows = rows < 2 ? 2 : rows;
+    const int bands = (nz + rows - 1) / rows;
+    return (nz + bands - 1) / bands;
+}
+// host: the most tiles any window of 1..nnu bins makes of `nz` rows
+int adv_tiles(int nnu, int nr, int nz, int rows, int share) {
+    int most = 1;
+    for (int n = 1; n <= nnu; n++) {
+        int tpb = 1 << 30;
+        for (int q = 0; q < 4; q++) {
+            const int c = pack_cost(n, nr, (n + 31) / 32 + q);
+            tpb = c < tpb ? c : tpb;
+        }
+        const int r = rows > 0 ? rows : pack_rows(tpb, nz, share);
+        const int m = tpb * ((nz + r - 1) / r);
+        most = m > most ? m : most;
+    }
+    return most;
+}
+
+// The cell a staged stencil cell (col, row) copies, and the boundary rules that r_cell / z_cell
+// apply to the copy: rr for H_r, rz for H_Z (1: negate; 2: keep the part <= 0; 3: keep the
+// part >= 0). A corner cell (ghost in both directions) is never staged.
+struct CellSrc { int i, j, rr, rz; };
+__device__ __forceinline__ CellSrc cell_src(const View &v, int col, int row) {
+    CellSrc s{col, row, 0, 0};
+    if (col < 0) {
+        if (v.bcl == 0) { s.i = -1 - col; s.rr = 1; } else { s.i = 0; s.rr = 2; }
+    } else if (col >= v.nr) {
+        if (v.bcr == 0) { s.i = 2 * v.nr - 1 - col; s.rr = 1; } else { s.i = v.nr - 1; s.rr = 3; }
+    } else if (row < 0) {
+        if (v.bzb == 0) { s.j = -1 - row; s.rz = 1; } else { s.j = 0; s.rz = 2; }
+    } else if (row >= v.nz) {
+        if (v.bzt == 0) { s.j = 2 * v.nz - 1 - row; s.rz = 1; } else { s.j = v.nz - 1; s.rz = 3; }
+    }
+    return s;
+}
+template <typename S>
+__device__ __forceinline__ S bc_rule(S h, int rule) {
+    if (rule == 1) return -h;
+    if (rule == 2) return h < S(0) ? h : S(0);
+    if (rule == 3) return h > S(0) ? h : S(0);
+    return h;
+}
+
+// Every staged input a row ahead: when the landing rows fit, i.e. when S and R agree.
+template <typename S, typename R> __host__ __device__ constexpr bool adv_ahead() { return sizeof(S) == sizeof(R); }
+// The halo's landing row fills the gaps of its staged row's planes (96 of 256 values) in FP64;
+// with FP32 it has its own space.
+template <typename S, typename R> __host__ __device__ constexpr bool adv_overlay() { return sizeof(S) == 8 && sizeof(R) == 8; }
+template <typename S, typename R>
+__host__ __device__ constexpr size_t adv_pack_smem() {
+    size_t b = sizeof(R) * ((RING + 1) * 4 * PT + 5 * PT);           // ring, halo row, r faces
+    b += sizeof(S) * RING * (adv_ahead<S, R>() ? 2 : 3) * PT;        // the state's rows
+    if (adv_ahead<S, R>()) b += sizeof(S) * 2 * PT;                  // landing row: J, H_voigt
+    if (adv_ahead<S, R>() && !adv_overlay<S, R>()) b += sizeof(S) * 4 * PHALO + sizeof(double) * 2 * PHALO;
+    return b + sizeof(double) * (2 * PGEO + PNC * 5 + PNC);
+}
+
+// One tile of the work list by the calling CTA of PT threads, in dynamic shared memory `sm`: the
+// body of k_advect, also run by the persistent batch kernel.
+template <typename S, typename R, int FLUX>
+__device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsigned char *sm) {
+    constexpr bool AHEAD = adv_ahead<S, R>(), OVER = adv_overlay<S, R>();
+    constexpr int HF = AHEAD ? 2 : 3;
+    R *A = reinterpret_cast<R *>(sm);                       // [RING][4][PT]
+    R *HB = A + RING * 4 * PT;                              // [4][PT]: the halo columns' current row
+    R *Fr = HB + 4 * PT;                                    // [5][PT]
+    S *Hs = reinterpret_cast<S *>(Fr + 5 * PT);             // [RING][HF][PT]: H_r, H_Z (, J) as stored
+    S *raw = Hs + RING * HF * PT;                           // AHEAD: [2][PT]: J, H_voigt (or alpha_F) landing
+    double *geo = reinterpret_cast<double *>(raw + (AHEAD ? 2 * PT : 0));   // [2][PGEO]
+    double *riv = geo + 2 * PGEO;                           // [PNC][5]: the r faces' intervals
+    double *irc = riv + PNC * 5;                            // [PNC]: <1/r>
+    double *hal = irc + PNC;                                // AHEAD, not OVER: [2][PHALO], then [4][PHALO] of S
+    const int t = threadIdx.x;
+    const int4 it = a.tiles[tile];                          // cloud, rows [y, w), place z in their list
+    View v;
+    load_view(a.cl[it.x], v);
+    int kmin = a.kwin[2 * it.x], kmax = a.kwin[2 * it.x + 1];
+    kmin = kmin > 0 ? kmin : 0;
+    kmax = kmax < a.nnu - 1 ? kmax : a.nnu - 1;
+    const int nact = kmax >= kmin ? kmax - kmin + 1 : 0;
+    const Pack pk = pack_bins(nact > 0 ? nact : 1, v.nr);
+    const int tpb = pk.nb * pk.nct, band = it.z / tpb, e0 = it.z - band * tpb;
+    const int kb = e0 / pk.nct, ct = e0 - kb * pk.nct;
+    const int rows = a.rows > 0 ? a.rows : pack_rows(tpb, it.w - it.y, a.cl[it.x].adv_share);
+    const int j0 = it.y + band * rows;
+    if (j0 >= it.w) return;
+    const int j1 = j0 + rows < it.w ? j0 + rows : it.w;
+    const int nbk = pk.nbk, i0 = ct * pk.ncol;
+    int ncol = pk.ncol;
+    if (i0 >= v.nr) return;                                 // (shares rounded up can leave a last one empty)
+    ncol = i0 + ncol <= v.nr ? ncol : v.nr - i0;
+    const int kbeg = kmin + kb * nbk;
+    const R jeps = R(a.jeps);
+
+    // bins outside the window pass through: the rows of the tile in turn over its chunks
+    if (nact < a.nnu) {
+        const int nin = a.nnu - nact, n = ncol * nin;
+        for (int j = j0 + kb; j < j1; j += pk.nb) {
+            const long long row = v.o3 + (long long)a.nnu * (i0 + (long long)v.nr * j);
+            for (int e = t; e < n; e += PT) {
+                const int c = e / nin, m = e - c * nin;
+                const long long x = row + (long long)a.nnu * c + (m < kmin ? m : m + nact);
+                a.Jo[x] = a.J[x]; a.Hro[x] = a.Hr[x]; a.HZo[x] = a.HZ[x];
+            }
+        }
+    }
+    if (nact == 0 || kbeg > kmax) return;
+
+    // this thread's item: column i0 + c (c = ncol: the column right of the tile, for its r face)
+    const int c = t / nbk, k = kbeg + (t - c * nbk), col = i0 + c;
+    const bool item = c <= ncol && k <= kmax && col <= v.nr + 1;
+    const bool own = item && c < ncol;
+    const bool busy = __any_sync(0xffffffffu, item);
+    const int cg = c < ncol ? c : ncol;
+    // and its halo cell, counted from the top so that the threads without an own cell come first:
+    // columns i0-2, i0-1 and i0+ncol+1
+    const int hq = PT - 1 - t, hc = hq / nbk, hk = kbeg + (hq - hc * nbk);
+    const int hcol = hc < 2 ? i0 - 2 + hc : i0 + ncol + 1;
+    const bool halo = hc < 3 && hk <= kmax && hcol <= v.nr + 1;
+    R *hp = HB + hq;
+    S *hraw = nullptr;
+    int hps = 0;                                            // plane stride of the halo's landing row
+    double *hal0 = nullptr, *hal1 = nullptr;                // its alpha, alpha_cF
+    if constexpr (OVER) {
+        hraw = reinterpret_cast<S *>(HB) + PHALO + hq;
+        hps = PT;
+        hal0 = reinterpret_cast<double *>(HB) + (hq >> 6) * PT + 2 * PHALO + (hq & 63);
+        hal1 = hal0 + 2 * PT;
+    } else if constexpr (AHEAD) {
+        hraw = reinterpret_cast<S *>(hal + 2 * PHALO) + hq;
+        hps = PHALO;
+        hal0 = hal + hq;
+        hal1 = hal0 + PHALO;
+    }
+
+    // ---- copies a row ahead ----
+    // a cell's column and bin are the thread's own: what changes from row to row is the source row
+    const unsigned rstr = (unsigned)a.nnu * (unsigned)v.nr;
+    auto copy_cell = [&](long long xc, long long xac, int row, S *dJ, S *dHr, S *dHZ, S *dHv) {
+        int sj = row, rj = row;
+        if (row >= v.nz) {
+            sj = v.bzt == 0 ? 2 * v.nz - 1 - row : v.nz - 1;
+            rj = v.nz - 1;
+        }
+        const long long x = xc + (long long)((unsigned long long)rstr * (unsigned)sj);
+        const long long xa = xac + (long long)((unsigned long long)rstr * (unsigned)rj);
+        cp_async_el(dJ, a.J + x);
+        cp_async_el(dHr, a.Hr + x);
+        cp_async_el(dHZ, a.HZ + x);
+        cp_async_el(dHv, (a.aF ? a.aF : a.Hv) + xa);
+    };
+    // where a (possibly ghost) column's cells and opacities come from, and the rule of its H_r
+    auto col_base = [&](int cc, int kk, long long &xc, long long &xac, int &rule) {
+        const CellSrc s = cell_src(v, cc, 0);
+        const int ci = cc < 0 ? 0 : (cc >= v.nr ? v.nr - 1 : cc);
+        xc = v.o3 + kk + (long long)a.nnu * s.i;
+        xac = v.o3 + kk + (long long)a.nnu * ci;
+        rule = s.rr;
+    };
+    long long xo = 0, xoa = 0, xh = 0, xha = 0;
+    int orule = 0, hrule = 0;
+    if (AHEAD && item) col_base(col, k, xo, xoa, orule);
+    if (AHEAD && halo) col_base(hcol, hk, xh, xha, hrule);
+    // rows the own columns stage: up to j1 + 1 and the second ghost row; no corner ghosts
+    auto stages = [&](int r) { return item && r <= j1 + 1 && r <= v.nz + 1 && !(col >= v.nr && r >= v.nz); };
+    auto issue_own = [&](int r) {
+        if (stages(r)) {
+            S *h = Hs + (r & (RING - 1)) * HF * PT + t;
+            copy_cell(xo, xoa, r, raw + t, h, h + PT, raw + PT + t);
+        }
+    };
+    auto issue_halo = [&](int r) {
+        if (halo && r < j1) {
+            copy_cell(xh, xha, r, hraw, hraw + hps, hraw + 2 * hps, hraw + 3 * hps);
+            if (!a.aF) {
+                const int ci = hcol < 0 ? 0 : (hcol >= v.nr ? v.nr - 1 : hcol);
+                const long long cl = v.oc + ci + (long long)v.nr * r;
+                cp_async_el(hal0, a.alpha + cl);
+                if (a.alpha_cF) cp_async_el(hal1, a.alpha_cF + cl);
+            }
+        }
+    };
+    auto put = [&](R *p, S J, S Hr, S HZ, R aF) {
+        const CellF<R> f = cell_f<R>(R(J), R(Hr), R(HZ), jeps);
+        p[0] = f.J; p[PT] = f.fr; p[2 * PT] = f.fZ; p[3 * PT] = aF;
+    };
+    auto aF_of = [&](S hv, double al, double acF) {
+        if (a.aF) return R(hv);
+        R x = R(al) * R(hv);
+        if (a.alpha_cF) x = x + R(acF);
+        return x;
+    };
+    // cell (cc, row) by loads, with its state into Hs for the own columns
+    auto keep = [&](S *h, const Cell<S> &x) {
+        h[0] = x.Hr; h[PT] = x.HZ;
+        if (HF == 3) h[2 * PT] = x.J;
+    };
+    auto stage_direct = [&](R *p, S *h, int cc, int row, int kk) {
+        const Cell<S> x = raw_cell<S, S>(a, v, cc, row, kk);
+        const R aF = alpha_F_clamped<S, R>(a, v, cc, row, kk);
+        put(p, x.J, x.Hr, x.HZ, aF);
+        if (h) keep(h, x);
+    };
+
+    // ---- per-row scalars: entry t of a row's slot comes from gsrc + row * gstr ----
+    const double *gsrc = nullptr;
+    int gstr = 0;
+    const int gi = t / PNC, gc = t - gi * PNC, gcol = i0 + gc;
+    if (gi < P_N) {
+        const bool face = gi == P_AR || gi == P_UR, al = gi >= P_AL;
+        if (gc <= ncol && (face ? gcol <= v.nr : al ? gcol <= v.nr + 1 : (gc < ncol && gcol < v.nr))) {
+            const int cc = gcol < v.nr ? gcol : v.nr - 1;
+            gstr = face ? v.nr + 1 : v.nr;
+            switch (gi) {
+                case P_AR: gsrc = a.A_r + v.orf + gcol; break;
+                case P_UR: gsrc = a.u_r_star + v.orf + gcol; break;
+                case P_AZL: gsrc = a.A_Z + v.ozf + gcol; break;
+                case P_AZR: gsrc = a.A_Z + v.ozf + gcol + v.nr; break;
+                case P_IDV: gsrc = a.inv_dV + v.oc + gcol; break;
+                case P_DURDR: gsrc = a.dur_dr + v.oc + gcol; break;
+                case P_DURDZ: gsrc = a.dur_dZ + v.oc + gcol; break;
+                case P_DUZDR: gsrc = a.duZ_dr + v.oc + gcol; break;
+                case P_DUZDZ: gsrc = a.duZ_dZ + v.oc + gcol; break;
+                case P_UROR: gsrc = a.ur_over_r + v.oc + gcol; break;
+                case P_UZ: gsrc = a.u_Z_star + v.ozf + gcol + v.nr; break;       // face j + 1
+                case P_AL: gsrc = AHEAD && !a.aF ? a.alpha + v.oc + cc : nullptr; break;
+                default: gsrc = AHEAD && !a.aF && a.alpha_cF ? a.alpha_cF + v.oc + cc : nullptr; break;
+            }
+        }
+    } else if (t < PGEO) {
+        gsrc = a.zint + v.ozint + 5 + (t - P_N * PNC);                           // face j + 1
+        gstr = 5;
+    }
+    const bool g_al = gi == P_AL || gi == P_ACF;
+    auto geo_copy = [&](int jb) {
+        int row = jb;
+        if (g_al) row = jb + 3 < v.nz ? jb + 3 : v.nz - 1;
+        if (gsrc != nullptr && (g_al || jb < j1)) cp_async_el(geo + (jb & 1) * PGEO + t, gsrc + (long long)gstr * row);
+    };
+
+    // ---- prologue: the first copies, then rows j0-2 .. j0+1 by loads ----
+    if constexpr (AHEAD) {
+        issue_own(j0 + 2);
+        issue_halo(j0);
+    }
+    geo_copy(j0);
+    if (g_al) geo_copy(j0 - 1);
+    cp_async_commit();
+    if (item) {
+        // (the loads of all four rows first, then their conversions)
+        Cell<S> x[4];
+        R aF[4];
+        auto skip = [&](int r) { return r < -2 || r > v.nz + 1 || (col >= v.nr && (r < 0 || r >= v.nz)); };
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int r = j0 - 2 + q;
+            if (skip(r)) continue;
+            x[q] = raw_cell<S, S>(a, v, col, r, k);
+            aF[q] = alpha_F_clamped<S, R>(a, v, col, r, k);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int r = j0 - 2 + q, sl = r & (RING - 1);
+            if (skip(r)) continue;
+            put(A + sl * 4 * PT + t, x[q].J, x[q].Hr, x[q].HZ, aF[q]);
+            // (the state of rows below j0 is not needed, and row j0-2's slot is row j0+2's)
+            if (q >= 2) keep(Hs + sl * HF * PT + t, x[q]);
+        }
+    }
+    for (int e = t; e < PNC * 5; e += PT) {
+        const int f = i0 + e / 5;
+        if (f <= v.nr) riv[e] = __ldg(a.rint + v.orint + 5 * f + e % 5);
+    }
+    if (t < PNC && i0 + t < v.nr) irc[t] = __ldg(a.inv_r_cell + v.ocol + i0 + t);
+    cp_async_wait<0>();
+    __syncthreads();
+    auto zface = [&](int f, const double *ivz, double us, R *F) {
+        auto row = [&](int r) { return A + (r & (RING - 1)) * 4 * PT + t; };
+        face_z_cells<R, FLUX>(row(f + 2), row(f + 3), row(f), row(f + 1), PT, jeps, us, ivz, F);
+    };
+    R zL[3] = {R(0), R(0), R(0)};
+    if (own) zface(j0, a.zint + v.ozint + 5 * j0, __ldg(a.u_Z_star + v.ozf + col + (long long)v.nr * j0), zL);
+    long long x = v.o3 + (long long)k + (long long)a.nnu * ((long long)col + (long long)v.nr * j0);
+
+    for (int j = j0; j < j1; j++) {
+        const double *g = geo + (j & 1) * PGEO;
+        // (A) row j+2 of the own columns and row j of the halo columns
+        if constexpr (AHEAD) {
+            const int r = j + 2;
+            if (stages(r)) {
+                const int zrule = r < v.nz ? 0 : (v.bzt == 0 ? 1 : 3);
+                const S *h = Hs + (r & (RING - 1)) * HF * PT + t;
+                const double *gp = geo + ((j - 1) & 1) * PGEO + c;
+                put(A + (r & (RING - 1)) * 4 * PT + t, raw[t], bc_rule(h[0], orule), bc_rule(h[PT], zrule),
+                    aF_of(raw[PT + t], gp[P_AL * PNC], gp[P_ACF * PNC]));
+            }
+            issue_own(r + 1);
+            if (halo) {
+                put(hp, hraw[0], bc_rule(hraw[hps], hrule), hraw[2 * hps],
+                    aF_of(hraw[3 * hps], *hal0, *hal1));
+                issue_halo(j + 1);
+            }
+        } else {
+            const int r = j + 2;
+            if (stages(r))
+                stage_direct(A + (r & (RING - 1)) * 4 * PT + t, Hs + (r & (RING - 1)) * HF * PT + t, col, r, k);
+            if (halo) stage_direct(hp, nullptr, hcol, j, hk);
+        }
+        __syncthreads();
+        geo_copy(j + 1);
+        cp_async_commit();
+        // (B) the r face left of the column, the Z face j+1/2: computed by every thread of a warp that
+        // has an item (a thread without one reads what lies in its places and keeps nothing), so that
+        // the two faces are one straight run of code
+        R zR[3] = {R(0), R(0), R(0)};
+        if (busy) {
+            const R *p = A + (j & (RING - 1)) * 4 * PT + t;
+            const R *hb = HB + (k - kbeg);
+            R F[3], kL, kR;
+            face_r_cells<R, FLUX>(c >= 2 ? p - 2 * nbk : hb + c * nbk, c >= 1 ? p - nbk : hb + nbk, p,
+                                  c < ncol ? p + nbk : hb + 2 * nbk, PT, col == 0, jeps, g[P_UR * PNC + cg],
+                                  riv + 5 * cg, F, kL, kR);
+            zface(j + 1, g + P_N * PNC, g[P_UZ * PNC + cg], zR);
+            R *o = Fr + t;
+            o[0] = F[0]; o[PT] = F[1]; o[2 * PT] = F[2]; o[3 * PT] = kL; o[4 * PT] = kR;
+        }
+        __syncthreads();
+        // (C) cell update
+        if (own) {
+            const S *h = Hs + (j & (RING - 1)) * HF * PT + t;
+            const S uJ = HF == 3 ? h[2 * PT] : S(A[(j & (RING - 1)) * 4 * PT + t]);
+            const double *q = g + c;
+            const UpdGeo ug = {q[P_AR * PNC],    q[P_AR * PNC + 1], q[P_AZL * PNC],   q[P_AZR * PNC],
+                               q[P_IDV * PNC],   q[P_DURDR * PNC],  q[P_DURDZ * PNC], q[P_DUZDR * PNC],
+                               q[P_DUZDZ * PNC], q[P_UROR * PNC],   irc[c]};
+            cell_update<S, R>(a, x, uJ, h[0], h[PT], zL, zR, Fr + t, Fr + t + nbk, PT, ug, v.ctdt, jeps);
+        }
+        x += (long long)a.nnu * v.nr;
+        zL[0] = zR[0]; zL[1] = zR[1]; zL[2] = zR[2];
+        cp_async_wait<0>();
+    }
+}
+
+template <typename S, typename R, int FLUX, int MINB>
+__global__ void __launch_bounds__(PT, MINB) k_advect(AdvArgs<S> a) {
+    extern __shared__ __align__(128) unsigned char adv_smem[];
+    advect_tile<S, R, FLUX>(a, blockIdx.x, adv_smem);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1844,10 +2065,10 @@ struct PersistArgs {
 
 // RA: arithmetic of the advection; RF, RC: of the frequency step and its closure (as k_freq).
 template <typename S, typename RA, typename RF, typename RC, int FLUX, int M>
-__global__ void __launch_bounds__(MTHREADS, 2) k_step_persistent(PersistArgs<S> p) {
+__global__ void __launch_bounds__(PT, 2) k_step_persistent(PersistArgs<S> p) {
     extern __shared__ __align__(128) unsigned char psm[];
     for (int t = blockIdx.x; t < p.ntiles; t += gridDim.x) {
-        advect_tile<S, RA, FLUX, false>(p.adv, t, psm);
+        advect_tile<S, RA, FLUX>(p.adv, t, psm);
         __syncthreads();
     }
     if (!grid_barrier(p.bar, gridDim.x, p.polls, p.err)) return;
@@ -1863,59 +2084,60 @@ __global__ void __launch_bounds__(MTHREADS, 2) k_step_persistent(PersistArgs<S> 
 }
 
 // ---- launch wrappers ----------------------------------------------------------------------
-template <typename S, typename R, bool TMA>
-static size_t adv_smem_bytes() {
-    if (!TMA) return adv_smem_base<S, R, adv_pfr<R, TMA>()>();
-    return adv_tma_off(adv_smem_base<S, R, false>()) + raw_tile_bytes<S>() + 16;   // raw tile, mbarrier, abort flag
-}
-
-template <typename S, typename R, int FLUX, int MINB, bool TMA>
-static void adv_launch_t(const void *args, int ntiles, cudaStream_t st) {
+template <typename S, typename R, int FLUX, int MINB>
+static void adv_launch(const void *args, cudaStream_t st) {
     static bool attr = false;
-    size_t sm = adv_smem_bytes<S, R, TMA>();
+    const AdvArgs<S> &a = *static_cast<const AdvArgs<S> *>(args);
+    // the bulk-copy form runs when the caller encoded tensor maps for this launch's input state
+    if (a.tmaps) {
+        constexpr size_t sm = adv_tma_off(adv_smem_base<S, R>()) + raw_tile_bytes<S>() + 16;   // + mbarrier, abort flag
+        static bool attr_t = false;
+        if (!attr_t) {
+            cudaFuncSetAttribute(k_advect_tma<S, R, FLUX, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            attr_t = true;
+        }
+        k_advect_tma<S, R, FLUX, MINB><<<a.ntiles, MTHREADS, sm, st>>>(a);
+        return;
+    }
+    constexpr size_t sm = adv_pack_smem<S, R>();
     if (!attr) {
-        cudaFuncSetAttribute(k_advect<S, R, FLUX, MINB, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaFuncSetAttribute(k_advect<S, R, FLUX, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         attr = true;
     }
-    k_advect<S, R, FLUX, MINB, TMA><<<ntiles, MTHREADS, sm, st>>>(*static_cast<const AdvArgs<S> *>(args));
-}
-
-// the bulk-copy staging runs when the caller encoded tensor maps for this launch's input state
-template <typename S, typename R, int FLUX, int MINB>
-static void adv_launch(const void *args, int ntiles, cudaStream_t st) {
-    if (static_cast<const AdvArgs<S> *>(args)->tmaps) adv_launch_t<S, R, FLUX, MINB, true>(args, ntiles, st);
-    else adv_launch_t<S, R, FLUX, MINB, false>(args, ntiles, st);
+    k_advect<S, R, FLUX, MINB><<<a.ntiles, PT, sm, st>>>(a);
 }
 
 template <typename S, typename R, int FLUX>
-static void adv_occ(const void *args, int ntiles, cudaStream_t st, int ctas) {
-    if (ctas >= 4) adv_launch<S, R, FLUX, 4>(args, ntiles, st);
-    else if (ctas == 2) adv_launch<S, R, FLUX, 2>(args, ntiles, st);
-    else adv_launch<S, R, FLUX, 3>(args, ntiles, st);
+static void adv_occ(const void *args, cudaStream_t st, int ctas) {
+    if (ctas >= 4) adv_launch<S, R, FLUX, 4>(args, st);
+    else if (ctas == 2) adv_launch<S, R, FLUX, 2>(args, st);
+    else adv_launch<S, R, FLUX, 3>(args, st);
 }
 
 int adv_ctas_per_sm(int prec, int want) {
-    if (prec == PREC_K_FP64) return (want == 2) ? 2 : 3;   // FP64: 76 KB of shared memory, 72 registers
+    if (prec == PREC_K_FP64) return (want == 2) ? 2 : 3;   // FP64: 75 KB of shared memory, 80 registers
     return (want >= 2 && want <= 4) ? want : 4;
 }
 
-void launch_advect(int prec, int flux, const void *args, int ntiles, int ctas, cudaStream_t st) {
-    if (ntiles <= 0) return;
+void launch_advect(int prec, int flux, const void *args, int ctas, cudaStream_t st) {
     ctas = adv_ctas_per_sm(prec, ctas);
     if (prec == PREC_K_FP64) {
+        if (static_cast<const AdvArgs<double> *>(args)->ntiles <= 0) return;
         if (ctas == 3) {
-            if (flux == 0) adv_launch<double, double, 0, 3>(args, ntiles, st);
-            else adv_launch<double, double, 1, 3>(args, ntiles, st);
+            if (flux == 0) adv_launch<double, double, 0, 3>(args, st);
+            else adv_launch<double, double, 1, 3>(args, st);
         } else {
-            if (flux == 0) adv_launch<double, double, 0, 2>(args, ntiles, st);
-            else adv_launch<double, double, 1, 2>(args, ntiles, st);
+            if (flux == 0) adv_launch<double, double, 0, 2>(args, st);
+            else adv_launch<double, double, 1, 2>(args, st);
         }
     } else if (prec == PREC_K_MIXED) {
-        if (flux == 0) adv_occ<double, float, 0>(args, ntiles, st, ctas);
-        else adv_occ<double, float, 1>(args, ntiles, st, ctas);
+        if (static_cast<const AdvArgs<double> *>(args)->ntiles <= 0) return;
+        if (flux == 0) adv_occ<double, float, 0>(args, st, ctas);
+        else adv_occ<double, float, 1>(args, st, ctas);
     } else {
-        if (flux == 0) adv_occ<float, float, 0>(args, ntiles, st, ctas);
-        else adv_occ<float, float, 1>(args, ntiles, st, ctas);
+        if (static_cast<const AdvArgs<float> *>(args)->ntiles <= 0) return;
+        if (flux == 0) adv_occ<float, float, 0>(args, st, ctas);
+        else adv_occ<float, float, 1>(args, st, ctas);
     }
 }
 
@@ -1996,26 +2218,25 @@ void launch_find_active(int sprec, const void *J, int nnu, const double *dnu, co
 }
 
 template <typename S, typename RA, typename RF, typename RC, int FLUX, int M>
-static cudaError_t persist_launch(const void *adv, const void *freq, const RedArgs &red, int ntiles, int nitems,
+static cudaError_t persist_launch(const void *adv, const void *freq, const RedArgs &red, int nitems,
                                   unsigned *bar, long long polls, int *err, cudaStream_t st) {
     PersistArgs<S> p;
     p.adv = *static_cast<const AdvArgs<S> *>(adv);
-    p.adv.tmaps = nullptr;
     p.freq = *static_cast<const FreqArgs<S> *>(freq);
     p.freq.vec16 = LaneRow<S, M>::ok && p.freq.nnu % M == 0 && (p.freq.nnu * sizeof(S)) % 16 == 0 && al16(p.freq.Jin) &&
                    al16(p.freq.Hrin) && al16(p.freq.HZin) && al16(p.freq.Jold) && al16(p.freq.Hv) &&
                    al16(p.freq.Jout) && al16(p.freq.Hrout) && al16(p.freq.HZout);
     p.red = red;
     if (!red.colsum) p.red.cnt = nullptr;
-    const int ncols = red.nnu + kExtraCols, rw = MTHREADS / 32;
-    p.ntiles = ntiles;
+    const int ncols = red.nnu + kExtraCols, rw = PT / 32;
+    p.ntiles = p.adv.ntiles;
     p.nitems = nitems;
     p.nred = p.red.cnt ? red.nclouds * ((ncols + rw - 1) / rw) : red.nclouds;
     p.bar = bar;
     p.polls = polls;
     p.err = err;
     auto kern = k_step_persistent<S, RA, RF, RC, FLUX, M>;
-    const size_t sa = adv_smem_bytes<S, RA, false>();
+    const size_t sa = adv_pack_smem<S, RA>();
     const size_t sf = sizeof(double) * freq_smem_doubles<M>(FREQ_THREADS / 32, p.freq.solver == SOLVER_THOMAS,
                                                             p.freq.Jold == p.freq.Jin ? 4 : 5);
     const size_t sm = sa > sf ? sa : sf;
@@ -2024,12 +2245,12 @@ static cudaError_t persist_launch(const void *adv, const void *freq, const RedAr
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, MTHREADS, sm);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, PT, sm);
     if (e != cudaSuccess) return e;
     if (per < 1) return cudaErrorInvalidConfiguration;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(per * sms));
-    cfg.blockDim = dim3(MTHREADS);
+    cfg.blockDim = dim3(PT);
     cfg.dynamicSmemBytes = sm;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -2043,11 +2264,11 @@ static cudaError_t persist_launch(const void *adv, const void *freq, const RedAr
 }
 
 cudaError_t launch_persistent(int prec, int flux, const void *adv, const void *freq, const RedArgs &red, int nnu,
-                              int ntiles, int nitems, unsigned *bar, long long polls, int *err, cudaStream_t st) {
+                              int nitems, unsigned *bar, long long polls, int *err, cudaStream_t st) {
     const int M = bins_per_lane(nnu);
 #define LYD_PS1(S_, RA_, RF_, RC_, M_)                                                                     \
-    return flux == 0 ? persist_launch<S_, RA_, RF_, RC_, 0, M_>(adv, freq, red, ntiles, nitems, bar, polls, err, st) \
-                     : persist_launch<S_, RA_, RF_, RC_, 1, M_>(adv, freq, red, ntiles, nitems, bar, polls, err, st);
+    return flux == 0 ? persist_launch<S_, RA_, RF_, RC_, 0, M_>(adv, freq, red, nitems, bar, polls, err, st) \
+                     : persist_launch<S_, RA_, RF_, RC_, 1, M_>(adv, freq, red, nitems, bar, polls, err, st);
 #define LYD_PS(S_, RA_, RF_, RC_)                                                                         \
     switch (M) {                                                                                          \
     case 1: LYD_PS1(S_, RA_, RF_, RC_, 1)                                                                 \

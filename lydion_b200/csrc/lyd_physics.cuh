@@ -117,10 +117,17 @@ __device__ __forceinline__ float rsqf(float x) {
 }
 constexpr float kFltMinNormal = 1.17549435e-38f;
 
-// MinMod, src/ConstantsAndFunctions.jl:1571-1582
+// MinMod, src/ConstantsAndFunctions.jl:1571-1582. FP64: the smaller in magnitude, or zero where the
+// sign bits differ, which is the reference's a b <= 0 without its product (a b underflows to zero
+// only for slopes below 1e-154, whose sum with anything is that thing).
 template <typename R>
 __device__ __forceinline__ R minmod(R a, R b) {
-    return (a * b <= R(0)) ? R(0) : (fabs(a) < fabs(b) ? a : b);
+    if constexpr (sizeof(R) == 8) {
+        const R m = fabs(a) < fabs(b) ? a : b;
+        return (__double2hiint(a) ^ __double2hiint(b)) < 0 ? R(0) : m;
+    } else {
+        return (a * b <= R(0)) ? R(0) : (fabs(a) < fabs(b) ? a : b);
+    }
 }
 
 // Levermore closure chi(f), src/M1Closure.jl:28-33, evaluated as (5 - 2 sqrt(4 - 3 f^2)) / 3,
@@ -136,6 +143,49 @@ __device__ __forceinline__ R chi_L84(R f) {
         return (R(5) - R(2) * rsq(t)) * R(1.0f / 3.0f);
     else
         return fma(-2.0 * t, rsqrt_nr(t), 5.0) * (1.0 / 3.0);
+}
+
+// 1 / |v| from |v|^2 for a vector whose length may vanish: the reciprocal root of s + tiny, so
+// that a zero vector gets a zero direction with no test (s is far above tiny wherever a direction
+// matters: |f| >= 1e-10 in the closure, and tiny is 1e-300 in FP64 and FLT_MIN in FP32).
+__device__ __forceinline__ double inv_len(double s) { return rsqrt_nr(s + 1e-300); }
+__device__ __forceinline__ float inv_len(float s) { return rsqf(s + kFltMinNormal); }
+
+// The two coefficients of the Eddington tensor D = a I + b n n (src/M1Closure.jl:46-119) at reduced
+// flux f <= fmax: with s = sqrt(4 - 3 f^2), chi = (5 - 2 s) / 3 and the reference's (1 - chi) / 2 and
+// (3 chi - 1) / 2 are (s - 1) / 3 and 2 - s. At f below fmin (1e-10) s rounds to 2: a = 1/3, b = 0, the
+// isotropic tensor the reference switches to there, so no branch is needed; and since n is a unit
+// vector wherever b is not 0, D_phiphi = 1 - D_rr - D_ZZ is a.
+template <typename R>
+__device__ __forceinline__ void eddington_ab(R f, R &a, R &b) {
+    const R t = R(4) - R(3) * (f * f);
+    R s;
+    if constexpr (sizeof(R) == 4) s = rsq(t);
+    else s = t * rsqrt_nr(t);
+    a = (s - R(1)) * Num<R>::third();
+    b = R(2) - s;
+}
+
+// D : grad u (D_colon_grad_u_Cylindrical, src/ConstantsAndFunctions.jl:883-895) with the closure of
+// a cell's (J, H_r, H_Z) (Compute_D_Edd, src/M1Closure.jl:46-83): a (g0 + g3 + g4) + b (n_r (n_r g0 +
+// n_Z g12) + n_Z^2 g3), g0 = du_r/dr, g12 = du_r/dZ + du_Z/dr, g3 = du_Z/dZ, tr = g0 + g3 + u_r/r.
+// jeps / heps2 are the floors in storage units: at or below them the tensor is isotropic.
+template <typename R>
+__device__ __forceinline__ R work_rate(R J, R Hr, R HZ, R jeps, R heps2, R g0, R g12, R g3, R tr) {
+    const R H2 = Hr * Hr + HZ * HZ;
+    bool on = J > jeps && H2 > heps2;
+    // |H|^2 below the type's normal range counts as no direction
+    if constexpr (sizeof(R) == 4) on = on && H2 >= kFltMinNormal;
+    else on = on && H2 >= kDblMinNormal;
+    R iH;
+    if constexpr (sizeof(R) == 4) iH = rsqf(on ? H2 : R(1));
+    else iH = rsqrt_nr(on ? H2 : R(1));
+    R f = (H2 * iH) * rcp<R>(on ? J : R(1));
+    f = on ? (f < Num<R>::fmax() ? f : Num<R>::fmax()) : R(0);
+    R a, b;
+    eddington_ab(f, a, b);
+    const R nr = Hr * iH, nZ = HZ * iH;
+    return a * tr + b * (nr * (nr * g0 + nZ * g12) + (nZ * nZ) * g3);
 }
 
 // Compute_D_Edd_from_f_n, src/M1Closure.jl:91-119
@@ -215,7 +265,7 @@ __device__ __forceinline__ void hll_eigen(R f, R mu, R &l1, R &l3) {
 // One cell of the reconstruction stencil.
 template <typename R> struct Cell { R J, Hr, HZ; };
 
-// ReconstructInterface output, src/AdvectJandH.jl:359-473
+// ReconstructInterface output, src/AdvectJandH.jl:359-473 (the adjoint's replay keeps it whole)
 template <typename R> struct Recon {
     R J_L, J_R, Hr_L, Hr_R, HZ_L, HZ_R, tau_L, tau_R, f_L, f_R, nr_L, nr_R, nZ_L, nZ_R;
 };
@@ -233,104 +283,88 @@ __device__ __forceinline__ CellF<R> cell_f(R J, R Hr, R HZ, R jeps) {
     return c;
 }
 
-// ReconstructInterface, src/AdvectJandH.jl:359-473, on prepared cells im1, i, ip1, ip2
-// around the interface between i and ip1; iv = {dL, dR, inv_i_im1, inv_ip1_i, inv_ip2_ip1}.
-template <typename R>
-__device__ __forceinline__ Recon<R> reconstruct_f(const CellF<R> &cm1, const CellF<R> &ci, const CellF<R> &cp1,
-                                                  const CellF<R> &cp2, const R iv[5], R aF_i, R aF_ip1, R jeps) {
-    Recon<R> o;
-    const R dL = iv[0], dR = iv[1];
-    o.tau_L = aF_i * dL;
-    o.tau_R = aF_ip1 * dR;
-    R dJc = (cp1.J - ci.J) * iv[3];
-    R dJL = minmod((ci.J - cm1.J) * iv[2], dJc);
-    R dJR = minmod((cp2.J - cp1.J) * iv[4], dJc);
-    R dfrc = (cp1.fr - ci.fr) * iv[3];
-    R dfrL = minmod((ci.fr - cm1.fr) * iv[2], dfrc);
-    R dfrR = minmod((cp2.fr - cp1.fr) * iv[4], dfrc);
-    R dfZc = (cp1.fZ - ci.fZ) * iv[3];
-    R dfZL = minmod((ci.fZ - cm1.fZ) * iv[2], dfZc);
-    R dfZR = minmod((cp2.fZ - cp1.fZ) * iv[4], dfZc);
-
-    R JL = ci.J + dJL * dL;
-    R JR = cp1.J - dJR * dR;
-    o.J_L = JL > jeps ? JL : jeps;
-    o.J_R = JR > jeps ? JR : jeps;
-    R frL = ci.fr + dfrL * dL, frR = cp1.fr - dfrR * dR;
-    R fZL = ci.fZ + dfZL * dL, fZR = cp1.fZ - dfZR * dR;
-
-    // one reciprocal square root gives |f| and 1/|f|; |f|^2 below the type's normal range
-    // counts as no flux (no direction)
-    const R sL = frL * frL + fZL * fZL, sR = frR * frR + fZR * fZR;
-    R iL, iR;
-    if constexpr (sizeof(R) == 4) {
-        iL = sL >= kFltMinNormal ? rsqf(sL) : R(0);
-        iR = sR >= kFltMinNormal ? rsqf(sR) : R(0);
-    } else {
-        iL = sL >= kDblMinNormal ? rsqrt_nr(sL) : R(0);
-        iR = sR >= kDblMinNormal ? rsqrt_nr(sR) : R(0);
-    }
-    R fL = sL * iL, fR = sR * iR;
-    if (fL > R(1)) { frL *= iL; fZL *= iL; fL = R(1); iL = R(1); }
-    if (fR > R(1)) { frR *= iR; fZR *= iR; fR = R(1); iR = R(1); }
-    o.Hr_L = frL * o.J_L; o.Hr_R = frR * o.J_R;
-    o.HZ_L = fZL * o.J_L; o.HZ_R = fZR * o.J_R;
-    o.nr_L = frL * iL; o.nZ_L = fZL * iL;
-    o.nr_R = frR * iR; o.nZ_R = fZR * iR;
-    o.f_L = fL; o.f_R = fR;
+// One side of an interface: the reconstructed J (floored) and reduced flux, its flux vector after the
+// causality limit |f| <= 1, and the second moments J D along the face's normal (Kn), across it (Kt)
+// and along phi (kp). ZDIR: the normal is Z, else r.
+template <typename R> struct Side { R J, Hr, HZ, Kn, Kt, kp, f, mu; };
+template <typename R, bool ZDIR>
+__device__ __forceinline__ Side<R> side_of(R J, R fr, R fZ) {
+    Side<R> o;
+    o.J = J;
+    const R s = fr * fr + fZ * fZ;
+    const R i = inv_len(s);                    // one reciprocal root gives |f| and the direction
+    const R f = s * i, nr = fr * i, nZ = fZ * i;
+    R a, b;
+    eddington_ab(f < Num<R>::fmax() ? f : Num<R>::fmax(), a, b);
+    o.f = f < R(1) ? f : R(1);
+    const R fJ = o.f * J;
+    o.Hr = nr * fJ;
+    o.HZ = nZ * fJ;
+    o.mu = ZDIR ? nZ : nr;
+    o.kp = a * J;
+    const R bn = (b * J) * o.mu;
+    o.Kn = o.kp + bn * o.mu;
+    o.Kt = bn * (ZDIR ? nr : nZ);
     return o;
 }
 
-// ReconstructInterface from raw cells (J, H_r, H_Z).
-template <typename R>
-__device__ __forceinline__ Recon<R> reconstruct(const Cell<R> &cm1, const Cell<R> &ci, const Cell<R> &cp1,
-                                                const Cell<R> &cp2, const R iv[5], R aF_i, R aF_ip1, R jeps) {
-    return reconstruct_f<R>(cell_f<R>(cm1.J, cm1.Hr, cm1.HZ, jeps), cell_f<R>(ci.J, ci.Hr, ci.HZ, jeps),
-                            cell_f<R>(cp1.J, cp1.Hr, cp1.HZ, jeps), cell_f<R>(cp2.J, cp2.Hr, cp2.HZ, jeps), iv,
-                            aF_i, aF_ip1, jeps);
-}
-
-// GetFluxGLF / GetFluxHLL, src/AdvectJandH.jl:81-118, 155-204, with the wave speeds of
-// M1WaveSpeeds_r/Z (src/M1Closure.jl:301-326). F{J,Hr,HZ}_{L,R} are the physical fluxes of
-// the three conserved quantities on either side; Ji/Jip1 the cell values for the
-// diffusion-limit term. ZDIR selects n_Z (true) or n_r (false) for the HLL eigenvalues.
+// One interface between cells ci and cp1 (outer stencil cells cm1 and cp2): ReconstructInterface
+// (src/AdvectJandH.jl:359-473), the closures of both sides, GetFluxGLF / GetFluxHLL (:81-118, 155-204)
+// with the wave speeds of M1WaveSpeeds_r/Z (src/M1Closure.jl:301-326), and the advection flux of
+// u*/c = uc (:276-282). iv = {dL, dR, inv_i_im1, inv_ip1_i, inv_ip2_ip1}. kL / kR: K_phiphi of the two
+// sides. The diffusion-limit weight 1 - eps = tau^2 / (0.2 + tau + tau^2) is formed as that product and
+// cancelled against the 1 / tau of the diffusive flux: one reciprocal, and none of the rounding of
+// 1 - eps divided by a small tau. No branches (the reference's floors and limits are selects), so
+// the two faces a thread computes can be scheduled together (FP64 advection at 256^2 x 64, packed
+// tiles: 258 -> 205 us).
 template <typename R, int FLUX, bool ZDIR>
-__device__ __forceinline__ void m1_flux(R FJ_L, R FJ_R, R FHr_L, R FHr_R, R FHZ_L, R FHZ_R,
-                                        const Recon<R> &q, R Ji, R Jip1, R &FJ, R &FHr, R &FHZ) {
-    R tau = q.tau_L + q.tau_R;
-    R num = R(0.2) + tau;
-    R eps = num * rcp<R>(num + tau * tau);
-    R ome = R(1) - eps;
-    R tau_eff = tau > Num<R>::tiny() ? tau : Num<R>::tiny();
-    R FJ_diff = -Num<R>::third() * (Jip1 - Ji) * rcp<R>(tau_eff);
+__device__ __forceinline__ void face_flux(const CellF<R> &cm1, const CellF<R> &ci, const CellF<R> &cp1,
+                                          const CellF<R> &cp2, const R iv[5], R aF_i, R aF_ip1, R uc, R jeps, R *F,
+                                          R &kL, R &kR, R &JR, R &HZR) {
+    const R dL = iv[0], dR = iv[1];
+    const R dJc = (cp1.J - ci.J) * iv[3], dfrc = (cp1.fr - ci.fr) * iv[3], dfZc = (cp1.fZ - ci.fZ) * iv[3];
+    const R J_L = ci.J + minmod((ci.J - cm1.J) * iv[2], dJc) * dL;
+    const R J_R = cp1.J - minmod((cp2.J - cp1.J) * iv[4], dJc) * dR;
+    const R fr_L = ci.fr + minmod((ci.fr - cm1.fr) * iv[2], dfrc) * dL;
+    const R fr_R = cp1.fr - minmod((cp2.fr - cp1.fr) * iv[4], dfrc) * dR;
+    const R fZ_L = ci.fZ + minmod((ci.fZ - cm1.fZ) * iv[2], dfZc) * dL;
+    const R fZ_R = cp1.fZ - minmod((cp2.fZ - cp1.fZ) * iv[4], dfZc) * dR;
+    const Side<R> L = side_of<R, ZDIR>(J_L > jeps ? J_L : jeps, fr_L, fZ_L);
+    const Side<R> Q = side_of<R, ZDIR>(J_R > jeps ? J_R : jeps, fr_R, fZ_R);
+    const R tau = aF_i * dL + aF_ip1 * dR;
+    const R num = R(0.2) + tau;
+    const R r = rcp<R>(num + tau * tau);
+    const R eps = num * r, te = tau * r;
+    const R diff = -Num<R>::third() * (cp1.J - ci.J) * te;
+    const R Kr_L = ZDIR ? L.Kt : L.Kn, Kr_R = ZDIR ? Q.Kt : Q.Kn, KZ_L = ZDIR ? L.Kn : L.Kt, KZ_R = ZDIR ? Q.Kn : Q.Kt;
+    const R Hn_L = ZDIR ? L.HZ : L.Hr, Hn_R = ZDIR ? Q.HZ : Q.Hr;
+    const bool up = uc < R(0);
+    const R aJ = uc * (up ? Q.J : L.J), aHr = uc * (up ? Q.Hr : L.Hr), aHZ = uc * (up ? Q.HZ : L.HZ);
     if (FLUX == 0) {
-        R FJ_glf = R(0.5) * (FJ_L + FJ_R) - R(0.5) * (q.J_R - q.J_L);
-        FJ = eps * FJ_glf + ome * FJ_diff;
-        R he = R(0.5) * eps;
-        FHr = R(0.5) * (FHr_L + FHr_R) - he * (q.Hr_R - q.Hr_L);
-        FHZ = R(0.5) * (FHZ_L + FHZ_R) - he * (q.HZ_R - q.HZ_L);
+        const R he = R(0.5) * eps;
+        F[0] = he * ((Hn_L + Hn_R) - (Q.J - L.J)) + (diff + aJ);
+        F[1] = R(0.5) * (Kr_L + Kr_R) - he * (Q.Hr - L.Hr) + aHr;
+        F[2] = R(0.5) * (KZ_L + KZ_R) - he * (Q.HZ - L.HZ) + aHZ;
     } else {
         R l1L, l3L, l1R, l3R;
-        hll_eigen<R>(q.f_L, ZDIR ? q.nZ_L : q.nr_L, l1L, l3L);
-        hll_eigen<R>(q.f_R, ZDIR ? q.nZ_R : q.nr_R, l1R, l3R);
-        R SR = fmax(fmax(l3L, l3R), R(0));
-        R SL = fmin(fmin(l1L, l1R), R(0));
-        R dS = SR - SL;
-        R inv_dS = rcp<R>(dS > Num<R>::tiny() ? dS : Num<R>::tiny());
-        R SRSL = SR * SL;
-        R FJh = (SR * FJ_L - SL * FJ_R + SRSL * (q.J_R - q.J_L)) * inv_dS;
-        R FHrh = (SR * FHr_L - SL * FHr_R + SRSL * (q.Hr_R - q.Hr_L)) * inv_dS;
-        R FHZh = (SR * FHZ_L - SL * FHZ_R + SRSL * (q.HZ_R - q.HZ_L)) * inv_dS;
-        R hom = R(0.5) * ome;
-        FJ = eps * FJh + ome * FJ_diff;
-        FHr = eps * FHrh + hom * (FHr_L + FHr_R);
-        FHZ = eps * FHZh + hom * (FHZ_L + FHZ_R);
+        hll_eigen<R>(L.f, L.mu, l1L, l3L);
+        hll_eigen<R>(Q.f, Q.mu, l1R, l3R);
+        R SR = l3L > l3R ? l3L : l3R, SL = l1L < l1R ? l1L : l1R;
+        SR = SR > R(0) ? SR : R(0);
+        SL = SL < R(0) ? SL : R(0);
+        const R dS = SR - SL;
+        const R w = eps * rcp<R>(dS > Num<R>::tiny() ? dS : Num<R>::tiny());
+        const R SRSL = SR * SL;
+        const R hom = R(0.5) * (tau * te);
+        F[0] = w * (SR * Hn_L - SL * Hn_R + SRSL * (Q.J - L.J)) + (diff + aJ);
+        F[1] = w * (SR * Kr_L - SL * Kr_R + SRSL * (Q.Hr - L.Hr)) + hom * (Kr_L + Kr_R) + aHr;
+        F[2] = w * (SR * KZ_L - SL * KZ_R + SRSL * (Q.HZ - L.HZ)) + hom * (KZ_L + KZ_R) + aHZ;
     }
+    kL = L.kp;
+    kR = Q.kp;
+    JR = Q.J;
+    HZR = Q.HZ;
 }
-
-// GetAdvectionFlux, src/AdvectJandH.jl:276-282
-template <typename R>
-__device__ __forceinline__ R adv_flux(R uc, R L, R Rv) { return uc * (uc < R(0) ? Rv : L); }
 
 // Compute_K_phiphi_InnerAxis, src/AdvectJandH.jl:499-522
 template <typename R>
@@ -346,9 +380,6 @@ __device__ __forceinline__ R k_phiphi_axis(R J, R HZ, R jeps) {
     k = k < R(0) ? R(0) : (k > R(1) ? R(1) : k);
     return k * J;
 }
-
-template <typename R>
-__device__ __forceinline__ R clamp01(R x) { return x < R(0) ? R(0) : (x > R(1) ? R(1) : x); }
 
 // D_colon_grad_u_Cylindrical, src/ConstantsAndFunctions.jl:883-895
 template <typename R>
