@@ -1304,15 +1304,38 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Per-k constants of UpdateFreqFactors! staged in shared memory once per CTA.
-// KC_EXP2: the 32 entries of exp_tab's table.
-enum { KC_NCK, KC_NCKP, KC_NCKM, KC_DNKP, KC_DNK, KC_DNKM, KC_IDNU, KC_ICK, KC_ICKP, KC_ICKM, KC_DNU, KC_EXP2, KC_N };
+// Per-bin constants of UpdateFreqFactors! staged in shared memory once per CTA. With the half-widths
+// dl = nuC - nu (left) and dr = nu_{k+1} - nuC (right) of a bin, the Peclet number at one of the three
+// places a row needs is P = C r, r = d / K, C = vel nuC + K (h/kT - 2 / nuC) (src/FreqFactors.jl:205-250),
+// i.e. P = vel (nuC d) / K + (h/kT) d - 2 d / nuC: KC_A* = nuC d, KC_D* = d, KC_B* = -2 d / nuC (zero without
+// recoil). *P: the left half of bin k+1, stored at k; *R: the right half of bin k (and, read at k-1,
+// of bin k-1). KC_EXP2: the 32 entries of exp_tab's table.
+enum { KC_AP, KC_DP, KC_BP, KC_AR, KC_DR, KC_BR, KC_IDNU, KC_DNU, KC_EXP2, KC_N };
 
-// Per-cell inputs staged in shared memory, 32 cells at a time per warp.
-// CS_SUM_R / CS_SUM_Z receive each cell's sum over bins of dnu (H_old - H), which the warp's
-// lanes turn into the cell's momentum, force and diagnostics once per 32 cells, one cell per lane.
-enum { CS_ALPHA, CS_ALPHA_C, CS_PD, CS_JS, CS_PHI_INV, CS_ALPHA_CF, CS_T, CS_DUR_DR, CS_DUR_DZ, CS_DUZ_DR,
-       CS_DUZ_DZ, CS_UR_OVER_R, CS_DV, CS_DRU_R, CS_DRU_Z, CS_SUM_R, CS_SUM_Z, CS_N };
+// Per-cell inputs staged in shared memory, 32 cells at a time per warp, one cell per lane, already in
+// the combinations the cell loop uses: opacities times c~ dt, the source, the prefactor of K, h/kT, the
+// velocity gradients over c (g0 = du_r/dr, g12 = du_r/dZ + du_Z/dr, g3 = du_Z/dZ, tr = the trace with
+// u_r/r), dV, the emitted power. CS_SUM_R / CS_SUM_Z receive each cell's sum over bins of
+// dnu (H_old - H), which the warp's lanes turn into the cell's momentum, force and diagnostics once per
+// 32 cells, one cell per lane.
+enum { CS_AL, CS_AC, CS_APD, CS_ACF, CS_SRC, CS_PREF, CS_REC0, CS_G0, CS_G12, CS_G3, CS_TR, CS_DV, CS_POW,
+       CS_DRU_R, CS_DRU_Z, CS_SUM_R, CS_SUM_Z, CS_N };
+
+// A lane's M contiguous doubles of a shared-memory row, as 16-byte loads where M allows.
+template <int M>
+__device__ __forceinline__ void lds_row(const double *p, double (&v)[M]) {
+    if constexpr (M % 2 == 0) {
+#pragma unroll
+        for (int m = 0; m < M; m += 2) {
+            const double2 t = *reinterpret_cast<const double2 *>(p + m);
+            v[m] = t.x;
+            v[m + 1] = t.y;
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < M; m++) v[m] = p[m];
+    }
+}
 
 // The next cell's bin rows (J, H_r, H_Z, H_voigt, J_old) are prefetched into a per-warp double
 // buffer while the current cell computes, up to two bins per lane (four or more would leave
@@ -1323,8 +1346,8 @@ template <int M> __host__ __device__ constexpr bool freq_prefetch() { return M <
 // reduction rows (without prefetch; with it, each warp's row lies in its own prefetch area,
 // free once the warp's cells are done), per-warp staged cell inputs, the per-warp prefetch
 // buffers (two slots of `ns` rows: 4, or 5 when J_old is not J's own buffer), and the
-// lane-serial solver rows when that solver runs: 72 KB per CTA at two bins per lane with J_old
-// aliased (86.5 KB before the overlay and the fourth row), which leaves L1 the difference. A
+// lane-serial solver rows when that solver runs: 71 KB per CTA at two bins per lane with J_old
+// aliased, which leaves L1 the difference. A
 // third CTA per SM would fit, but its 80-register bound spills in the cell loop (FP64 at
 // 256^2 x 64: 0.258 ms against 0.184 ms at two CTAs).
 template <int M>
@@ -1395,6 +1418,14 @@ __device__ __forceinline__ void warp_cell_run(int4 it, int warp, int nw, int &wb
 // (mixed frequency kernel at 256^2 x 64: 0.259 -> 0.246 ms; the mixed form's M_F after 2000
 // steps 5.93e-7 -> 5.95e-7 from FP64).
 //
+// Bound by instruction issue and dependent FP64 latency (16 warps per SM). What a cell's 32 lanes
+// share (opacities times c~ dt, the prefactor of K, h/kT, the gradients' combinations, column and row) is
+// formed once per 32 cells, one cell per lane; the Peclet numbers come from per-bin constants by
+// three multiply-adds; and the factors of a lane's bins are straight-line code (no branch per bin,
+// padding bins computed and dropped). Warp instructions per launch at 256^2 x 64: 122 -> 96 million;
+// per launch 178 -> 141 us (FP64), 174 -> 138 (mixed), 163 -> 129 (FP32 storage); 512^2 x 128 1474 ->
+// 1026 us, 24 clouds x 48 bins 158 -> 123 us, 64^2 x 64 27 -> 24 us.
+//
 // freq_item is one work item (`item` of `nitems`) by the calling CTA, whose first `nw` warps take
 // its cells (the others only meet its barriers), in dynamic shared memory `fsm`: the body of
 // k_freq, also run by the persistent batch kernel.
@@ -1409,18 +1440,16 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nnu = a.nnu;
     for (int t = threadIdx.x; t < NP; t += blockDim.x) {
-        bool in = (t >= 1 && t <= nnu - 2);
-        kc[KC_NCK * NP + t] = in ? a.nuC[t] : 0.0;
-        kc[KC_NCKP * NP + t] = in ? a.nuC[t + 1] : 0.0;
-        kc[KC_NCKM * NP + t] = in ? a.nuC[t - 1] : 0.0;
-        kc[KC_DNKP * NP + t] = in ? a.nuC[t + 1] - a.nu[t + 1] : 0.0;
-        kc[KC_DNK * NP + t] = in ? a.nu[t + 1] - a.nuC[t] : 0.0;
-        kc[KC_DNKM * NP + t] = in ? a.nu[t] - a.nuC[t - 1] : 0.0;
+        const bool up = t + 1 < nnu, in = t < nnu;
+        const double dp = up ? a.nuC[t + 1] - a.nu[t + 1] : 0.0, dr = in ? a.nu[t + 1] - a.nuC[t] : 0.0;
+        kc[KC_AP * NP + t] = up ? a.nuC[t + 1] * dp : 0.0;
+        kc[KC_DP * NP + t] = dp;
+        kc[KC_BP * NP + t] = up && a.recoil ? -2.0 * dp * a.inv_nuC[t + 1] : 0.0;
+        kc[KC_AR * NP + t] = in ? a.nuC[t] * dr : 0.0;
+        kc[KC_DR * NP + t] = dr;
+        kc[KC_BR * NP + t] = in && a.recoil ? -2.0 * dr * a.inv_nuC[t] : 0.0;
         kc[KC_IDNU * NP + t] = in ? a.inv_dnu[t] : 0.0;
-        kc[KC_ICK * NP + t] = in ? a.inv_nuC[t] : 0.0;
-        kc[KC_ICKP * NP + t] = in ? a.inv_nuC[t + 1] : 0.0;
-        kc[KC_ICKM * NP + t] = in ? a.inv_nuC[t - 1] : 0.0;
-        kc[KC_DNU * NP + t] = (t < nnu) ? a.dnu[t] : 0.0;
+        kc[KC_DNU * NP + t] = in ? a.dnu[t] : 0.0;
         kc[KC_EXP2 * NP + t] = (t < 32) ? kExp2Tab[t] : 0.0;
     }
     __syncthreads();
@@ -1485,6 +1514,8 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
     };
     const double k4 = kFourPiOverC * (1.0 / c_tilde) * a.j_scale;
     const double inv_dt = 1.0 / dt;
+    // emission/absorption steps over c~ dt; its source in storage units
+    const double ctdt_e = c_tilde * dt, src_w = c_tilde * dt / a.j_scale;
     // the per-cell part of the epilogue for cells [gb, ge) of the run (ge - gb <= 32), one
     // cell per lane: the momentum Delta rho u, this step's force, and the M_F, L and radial
     // partials (Update_f_Lya_MF_L_Lya!, src/ConstantsAndFunctions.jl:588-674)
@@ -1504,7 +1535,7 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
             double fr = (k4 * drs) * inv_dt, fz = (k4 * dzs) * inv_dt;
             if (a.f_r) { a.f_r[c] = fr; a.f_Z[c] = fz; }
             acc_mf += dV * sqrt(fr * fr + fz * fz);
-            acc_L += kFourPi * dV * cs[CS_JS * 32 + lane];
+            acc_L += cs[CS_POW * 32 + lane];
             double drr = __ldg(a.rCoM + cd.ocol + i), dzz = __ldg(a.ZCoM + cd.orow + j) - z_center;
             double dist = sqrt(drr * drr + dzz * dzz);
             double frad = 0.0;
@@ -1521,8 +1552,10 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
         cp_async_commit();
     }
     int g0 = wbeg;
+    int i = wbeg % nr - 1, j = wbeg / nr;      // the cell's column and row, advanced with it
+    S nonfin = S(0);                           // 0 x everything written: NaN once something is not finite
     for (int cl = wbeg; cl < wend; cl++) {
-        const int i = cl % nr, j = cl / nr;
+        if (++i == nr) { i = 0; j++; }
         const long long c = oc + cl;
         const long long base = o3 + (long long)cl * nnu;
         if (((cl - wbeg) & 31) == 0) {
@@ -1534,19 +1567,26 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
             const bool v = cl + lane < wend;
             const long long cc = c + lane;
             auto ld = [&](const double *p, bool need) { return (v && need && p) ? __ldg(p + cc) : 0.0; };
-            cs[CS_ALPHA * 32 + lane] = ld(a.alpha, a.do_emission || need_ff);
-            cs[CS_ALPHA_C * 32 + lane] = ld(a.alpha_c, a.do_emission);
-            cs[CS_PD * 32 + lane] = ld(a.pd, a.do_emission);
-            cs[CS_JS * 32 + lane] = ld(a.js, need_js);
-            cs[CS_PHI_INV * 32 + lane] = ld(a.phi_inv, a.do_emission && !a.phi);
-            cs[CS_ALPHA_CF * 32 + lane] = ld(a.alpha_cF, a.do_emission);
-            cs[CS_T * 32 + lane] = ld(a.T, need_ff);
-            cs[CS_DUR_DR * 32 + lane] = ld(a.dur_dr, need_ff);
-            cs[CS_DUR_DZ * 32 + lane] = ld(a.dur_dZ, need_ff);
-            cs[CS_DUZ_DR * 32 + lane] = ld(a.duZ_dr, need_ff);
-            cs[CS_DUZ_DZ * 32 + lane] = ld(a.duZ_dZ, need_ff);
-            cs[CS_UR_OVER_R * 32 + lane] = ld(a.ur_over_r, need_ff);
-            cs[CS_DV * 32 + lane] = ld(a.dV, a.parts != 0);
+            const double alv = ld(a.alpha, a.do_emission || need_ff), js = ld(a.js, need_js);
+            const double dV = ld(a.dV, a.parts != 0);
+            cs[CS_AL * 32 + lane] = alv * ctdt_e;
+            cs[CS_AC * 32 + lane] = ld(a.alpha_c, a.do_emission) * ctdt_e;
+            cs[CS_APD * 32 + lane] = alv * ld(a.pd, a.do_emission) * ctdt_e;
+            cs[CS_ACF * 32 + lane] = ld(a.alpha_cF, a.do_emission) * ctdt_e;
+            cs[CS_SRC * 32 + lane] = js * src_w * (a.phi ? 1.0 : ld(a.phi_inv, a.do_emission));
+            if (need_ff) {
+                // (the padding lanes get a temperature and no opacity)
+                const double T = v ? ld(a.T, true) : 1.0, dnuD = compute_dnuD(T);
+                cs[CS_PREF * 32 + lane] = 0.5 * (alv > a.alpha_floor ? alv : a.alpha_floor) * (dnuD * dnuD);
+                cs[CS_REC0 * 32 + lane] = a.recoil ? kHOverKB / T : 0.0;
+                const double g0 = ld(a.dur_dr, true), g3 = ld(a.duZ_dZ, true);
+                cs[CS_G0 * 32 + lane] = g0 * kInvC;
+                cs[CS_G12 * 32 + lane] = (ld(a.dur_dZ, true) + ld(a.duZ_dr, true)) * kInvC;
+                cs[CS_G3 * 32 + lane] = g3 * kInvC;
+                cs[CS_TR * 32 + lane] = (g0 + g3 + ld(a.ur_over_r, true)) * kInvC;
+            }
+            cs[CS_DV * 32 + lane] = dV;
+            cs[CS_POW * 32 + lane] = kFourPi * dV * js;
             cs[CS_DRU_R * 32 + lane] = ld(a.dru_r, a.do_emission);
             cs[CS_DRU_Z * 32 + lane] = ld(a.dru_Z, a.do_emission);
             __syncwarp();
@@ -1608,28 +1648,23 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
         double dr_sum = 0.0, dz_sum = 0.0;
         // ---- LyaEmissionAbsorptionUpdate! (src/ConstantsAndFunctions.jl:526-567) ----
         if (a.do_emission) {
-            const R al = R(cv[CS_ALPHA * 32]), acv = R(cv[CS_ALPHA_C * 32]);
-            const R al_pd = al * R(cv[CS_PD * 32]);
-            const R js_ct = R(cv[CS_JS * 32] * c_tilde / a.j_scale);
-            const R ct = R(c_tilde), dtr = R(dt);
-            const R pinv = a.phi ? R(0) : R(cv[CS_PHI_INV * 32]);
-            const R acF = a.alpha_cF ? R(cv[CS_ALPHA_CF * 32]) : R(0);
+            const R al = R(cv[CS_AL * 32]), ac = R(cv[CS_AC * 32]), apd = R(cv[CS_APD * 32]);
+            const R acF = R(cv[CS_ACF * 32]), src = R(cv[CS_SRC * 32]);
+            double dn[M];
+            lds_row<M>(kc + KC_DNU * NP + lane * M, dn);
 #pragma unroll
             for (int m = 0; m < M; m++) {
-                int k = lane * M + m;
-                if (k >= nnu) continue;
-                R phi = a.phi ? R(__ldg(a.phi + base + k))
-                              : ((k >= a.phi_kmin && k <= a.phi_kmax) ? Hv[m] * pinv : R(0));
-                R aabs = acv + al_pd * Hv[m];
-                R dJdt = js_ct * phi;
-                R aH = a.aF ? R(__ldg(a.aF + base + k)) : (a.alpha_cF ? al * Hv[m] + acF : al * Hv[m]);
-                double dn = kc[KC_DNU * NP + k];
-                R Jn = (R(Jo[m]) + dJdt * dtr) * rcp<R>(R(1) + aabs * ct * dtr);
-                R iden = rcp<R>(R(1) + aH * ct * dtr);
-                R hr = R(Hr[m]) * iden;
-                R hz = R(HZ[m]) * iden;
-                dr_sum += dn * (double(Hr[m]) - double(hr));
-                dz_sum += dn * (double(HZ[m]) - double(hz));
+                const int k = lane * M + m;
+                R phi = (k >= a.phi_kmin && k <= a.phi_kmax) ? Hv[m] : R(0);
+                R aH = al * Hv[m] + acF;
+                if (a.phi) phi = k < nnu ? R(__ldg(a.phi + base + k)) : R(0);
+                if (a.aF) aH = k < nnu ? R(__ldg(a.aF + base + k)) * R(ctdt_e) : R(0);
+                // (bins beyond n_nu hold zeros and have no width)
+                const R Jn = (R(Jo[m]) + src * phi) * rcp<R>(R(1) + (ac + apd * Hv[m]));
+                const R iden = rcp<R>(R(1) + aH);
+                const R hr = R(Hr[m]) * iden, hz = R(HZ[m]) * iden;
+                dr_sum += dn[m] * (double(Hr[m]) - double(hr));
+                dz_sum += dn[m] * (double(HZ[m]) - double(hz));
                 Hr[m] = S(hr);
                 HZ[m] = S(hz);
                 J[m] = S(Jn);
@@ -1647,73 +1682,69 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
             Row<M> sys;
             double Fp[M], F0[M], Fm[M];
             if (a.update_ff) {
-                // UpdateFreqFactors!, src/FreqFactors.jl:181-275
-                const double T = cv[CS_T * 32];
-                const double dnuD = compute_dnuD(T);
-                const double alv = cv[CS_ALPHA * 32];
-                const double pref = 0.5 * (alv > a.alpha_floor ? alv : a.alpha_floor) * (dnuD * dnuD);
-                const double rec0 = kHOverKB / T;
-                const R ga = R(cv[CS_DUR_DR * 32]), gb = R(cv[CS_DUR_DZ * 32]), gc = R(cv[CS_DUZ_DR * 32]);
-                const R gd = R(cv[CS_DUZ_DZ * 32]), ge = R(cv[CS_UR_OVER_R * 32]);
-                // K_k = pref H_voigt[k] and 1/K_k once per bin; the k+-1 neighbours come by
-                // shuffle (the same products the reference forms at k-1 and k+1)
+                // UpdateFreqFactors!, src/FreqFactors.jl:181-275, for every bin the lane holds (rows 0 and
+                // n_nu - 1, and padding bins, form values nobody keeps), so the lane's bins are one
+                // straight run of code.
                 // The frequency factors stay FP64 in every precision variant: with F/dw up to
                 // ~1e9 at tau0 = 1e8, an FP32 rounding of F0 against Fm + Fp acts as a spurious
                 // source or sink tens of times larger than the step's own change.
-                double Kb[M], iK[M];
+                const double pref = cv[CS_PREF * 32], rec0 = cv[CS_REC0 * 32];
+                const RC g0 = RC(cv[CS_G0 * 32]), g12 = RC(cv[CS_G12 * 32]), g3 = RC(cv[CS_G3 * 32]);
+                const RC tr = RC(cv[CS_TR * 32]);
+                // 1/K_k = 1 / (pref H_voigt[k]) once per bin; the k+-1 neighbours come by shuffle
+                double iK[M];
 #pragma unroll
-                for (int m = 0; m < M; m++) {
-                    Kb[m] = pref * double(Hv[m]);
-                    iK[m] = rcp<double>(Kb[m]);
-                }
-                double K_up = __shfl_up_sync(0xffffffffu, Kb[M - 1], 1);
-                double K_dn = __shfl_down_sync(0xffffffffu, Kb[0], 1);
-                double iK_up = __shfl_up_sync(0xffffffffu, iK[M - 1], 1);
-                double iK_dn = __shfl_down_sync(0xffffffffu, iK[0], 1);
+                for (int m = 0; m < M; m++) iK[m] = rcp<double>(pref * double(Hv[m]));
+                const double iK_up = __shfl_up_sync(0xffffffffu, iK[M - 1], 1);
+                const double iK_dn = __shfl_down_sync(0xffffffffu, iK[0], 1);
+                const double *kl = kc + lane * M, *etab = kc + KC_EXP2 * NP;
+                // the right half of the bin below the lane's first
+                const int kb = lane > 0 ? -1 : 0;
+                double ar = kl[KC_AR * NP + kb], drr = kl[KC_DR * NP + kb], br = kl[KC_BR * NP + kb];
+                constexpr int W = M >= 2 ? 2 : 1;       // bins whose constants are held at a time
 #pragma unroll
-                for (int m = 0; m < M; m++) {
-                    int k = lane * M + m;
-                    Fp[m] = 0.0; F0[m] = 0.0; Fm[m] = 0.0;
-                    if (k < 1 || k > nnu - 2) continue;
-                    RC Drr, DZZ, DrZ;
-                    D_edd<RC>(RC(Hr[m]), RC(HZ[m]), RC(J[m]), RC(jeps), RC(a.heps2), Drr, DZZ, DrZ);
-                    double vel =
-                        double(d_colon_grad_u<RC>(Drr, DrZ, DZZ, RC(ga), RC(gb), RC(gc), RC(gd), RC(ge))) * kInvC;
-                    double Kk = Kb[m];
-                    double Kkm = (m > 0) ? Kb[m - 1] : K_up;
-                    double Kkp = (m < M - 1) ? Kb[m + 1] : K_dn;
-                    double iKkm = (m > 0) ? iK[m - 1] : iK_up;
-                    double iKkp = (m < M - 1) ? iK[m + 1] : iK_dn;
-                    double nCk = kc[KC_NCK * NP + k], nCkp = kc[KC_NCKP * NP + k], nCkm = kc[KC_NCKM * NP + k];
-                    double Ckp = vel * nCkp, Ck = vel * nCk, Ckm = vel * nCkm;
-                    if (a.recoil) {
-                        Ckp += Kkp * (rec0 - 2.0 * kc[KC_ICKP * NP + k]);
-                        Ck += Kk * (rec0 - 2.0 * kc[KC_ICK * NP + k]);
-                        Ckm += Kkm * (rec0 - 2.0 * kc[KC_ICKM * NP + k]);
+                for (int mb = 0; mb < M; mb += W) {
+                    double AP[W], DP[W], BP[W], AR[W], DR[W], BR[W], idn[W];
+                    lds_row<W>(kl + KC_AP * NP + mb, AP);
+                    lds_row<W>(kl + KC_DP * NP + mb, DP);
+                    lds_row<W>(kl + KC_BP * NP + mb, BP);
+                    lds_row<W>(kl + KC_AR * NP + mb, AR);
+                    lds_row<W>(kl + KC_DR * NP + mb, DR);
+                    lds_row<W>(kl + KC_BR * NP + mb, BR);
+                    lds_row<W>(kl + KC_IDNU * NP + mb, idn);
+#pragma unroll
+                    for (int w = 0; w < W; w++) {
+                        const int m = mb + w;
+                        const double vel = double(work_rate<RC>(RC(J[m]), RC(Hr[m]), RC(HZ[m]), RC(jeps), RC(a.heps2),
+                                                                g0, g12, g3, tr));
+                        const double iKm = (m > 0) ? iK[m > 0 ? m - 1 : 0] : iK_up;
+                        const double iKp = (m < M - 1) ? iK[m < M - 1 ? m + 1 : 0] : iK_dn;
+                        const double rkp = DP[w] * iKp, rk = DR[w] * iK[m], rkm = drr * iKm;
+                        const double Pkp = clamp_P(fma(vel * AP[w], iKp, fma(rec0, DP[w], BP[w])));
+                        const double Pk = clamp_P(fma(vel * AR[w], iK[m], fma(rec0, DR[w], BR[w])));
+                        const double Pkm = clamp_P(fma(vel * ar, iKm, fma(rec0, drr, br)));
+                        double oRkp, xRkp, oLk, xLk, oRk, xRk, oLkm, xLkm;
+                        omphi_R(Pkp, oRkp, xRkp, etab);
+                        omphi_LR(Pk, oLk, xLk, oRk, xRk, etab);
+                        omphi_L(Pkm, oLkm, xLkm, etab);
+                        const double dkp = idn[w] * rcp<double>(xLk * rk - xRkp * rkp);
+                        const double dkm = idn[w] * rcp<double>(xLkm * rkm - xRk * rk);
+                        Fp[m] = oRkp * dkp;
+                        Fm[m] = oLkm * dkm;
+                        F0[m] = oLk * dkp + oRk * dkm;
+                        ar = AR[w]; drr = DR[w]; br = BR[w];
                     }
-                    double rkp = kc[KC_DNKP * NP + k] * iKkp;
-                    double rk = kc[KC_DNK * NP + k] * iK[m];
-                    double rkm = kc[KC_DNKM * NP + k] * iKkm;
-                    double Pkp = fmin(fmax(Ckp * rkp, -kPmax), kPmax);
-                    double Pk = fmin(fmax(Ck * rk, -kPmax), kPmax);
-                    double Pkm = fmin(fmax(Ckm * rkm, -kPmax), kPmax);
-                    double oRkp, xRkp, oLk, xLk, oRk, xRk, oLkm, xLkm;
-                    const double *etab = kc + KC_EXP2 * NP;
-                    omphi_R(Pkp, oRkp, xRkp, etab);
-                    omphi_LR(Pk, oLk, xLk, oRk, xRk, etab);
-                    omphi_L(Pkm, oLkm, xLkm, etab);
-                    double idn = kc[KC_IDNU * NP + k];
-                    double dkp = idn * rcp<double>(xLk * rk - xRkp * rkp);
-                    double dkm = idn * rcp<double>(xLkm * rkm - xRk * rk);
-                    Fp[m] = oRkp * dkp;
-                    Fm[m] = oLkm * dkm;
-                    F0[m] = oLk * dkp + oRk * dkm;
                 }
                 if (a.Fkp) {
 #pragma unroll
                     for (int m = 0; m < M; m++) {
                         int k = lane * M + m;
-                        if (k < nnu) { a.Fkp[base + k] = Fp[m]; a.Fk[base + k] = F0[m]; a.Fkm[base + k] = Fm[m]; }
+                        const bool in = k >= 1 && k <= nnu - 2;
+                        if (k < nnu) {
+                            a.Fkp[base + k] = in ? Fp[m] : 0.0;
+                            a.Fk[base + k] = in ? F0[m] : 0.0;
+                            a.Fkm[base + k] = in ? Fm[m] : 0.0;
+                        }
                     }
                 }
             } else {
@@ -1747,7 +1778,6 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
 #pragma unroll
             for (int m = 0; m < M; m++) {
                 int k = lane * M + m;
-                if (k >= nnu) continue;
                 bool in = (k >= 1 && k <= nnu - 2);
                 double Jn = in ? sys.d[m] : double(J[m]);
                 if (!(sys.b[m] != 0.0)) bad |= ERRB_SOLVE;
@@ -1769,9 +1799,7 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
         if (LR::ok && vec) {
             if (lane * M < nnu) {
 #pragma unroll
-                for (int m = 0; m < M; m++)
-                    if (!isfinite(double(J[m])) || !isfinite(double(Hr[m])) || !isfinite(double(HZ[m])))
-                        bad |= ERRB_NONFINITE;
+                for (int m = 0; m < M; m++) nonfin += J[m] * S(0) + Hr[m] * S(0) + HZ[m] * S(0);
                 LR::store(a.Jout + base + lane * M, J);
                 LR::store(a.Hrout + base + lane * M, Hr);
                 LR::store(a.HZout + base + lane * M, HZ);
@@ -1781,25 +1809,24 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
             for (int m = 0; m < M; m++) {
                 int k = lane * M + m;
                 if (k >= nnu) continue;
-                S js = S(J[m]), hs = S(Hr[m]), zs = S(HZ[m]);
-                if (!isfinite(double(js)) || !isfinite(double(hs)) || !isfinite(double(zs))) bad |= ERRB_NONFINITE;
-                a.Jout[base + k] = js;
-                a.Hrout[base + k] = hs;
-                a.HZout[base + k] = zs;
+                nonfin += J[m] * S(0) + Hr[m] * S(0) + HZ[m] * S(0);
+                a.Jout[base + k] = J[m];
+                a.Hrout[base + k] = Hr[m];
+                a.HZout[base + k] = HZ[m];
             }
         }
         // ---- epilogue partials ----
         if (a.parts & PART_ACTIVE) {
+            // (bins beyond n_nu have no width)
             const double dV = cv[CS_DV * 32];
+            double dn[M];
+            lds_row<M>(kc + KC_DNU * NP + lane * M, dn);
 #pragma unroll
             for (int m = 0; m < M; m++) {
-                int k = lane * M + m;
-                if (k >= nnu) continue;
-                double dn = kc[KC_DNU * NP + k];
-                double Jv = double(S(J[m]));
-                double e1 = Jv - 10.0 * jeps, e0 = Jv - jeps;
-                acc_e[m] += dn * (e1 > 0.0 ? e1 : 0.0) * dV;
-                acc_tot += dn * (e0 > 0.0 ? e0 : 0.0) * dV;
+                const double Jv = double(J[m]), w = dn[m] * dV;
+                const double e1 = Jv - 10.0 * jeps, e0 = Jv - jeps;
+                acc_e[m] += w * (e1 > 0.0 ? e1 : 0.0);
+                acc_tot += w * (e0 > 0.0 ? e0 : 0.0);
             }
         }
         if (a.parts & PART_DIAG) {
@@ -1825,6 +1852,7 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
         }
     }
     if (wbeg < wend) flush(g0, wend);
+    if (nonfin != S(0)) bad |= ERRB_NONFINITE;
     if constexpr (PF) cp_async_wait<0>();
     if (bad) atomicOr(a.err, bad);
     if (!a.parts) return;
@@ -1893,9 +1921,9 @@ __global__ void __launch_bounds__(FREQ_THREADS) k_find_active(const S *J, int nn
             if (k >= nnu) continue;
             double Jv = double(__ldg(J + o3 + (long long)c * nnu + k));
             double dn = __ldg(dnu + k);
-            double e1 = Jv - 10.0 * jeps, e0 = Jv - jeps;
-            acc_e[m] += dn * (e1 > 0.0 ? e1 : 0.0) * v;
-            acc_tot += dn * (e0 > 0.0 ? e0 : 0.0) * v;
+            const double e1 = Jv - 10.0 * jeps, e0 = Jv - jeps, w = dn * v;
+            acc_e[m] += w * (e1 > 0.0 ? e1 : 0.0);
+            acc_tot += w * (e0 > 0.0 ? e0 : 0.0);
         }
     }
     const int stride = NP + 8;

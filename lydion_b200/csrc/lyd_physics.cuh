@@ -421,8 +421,18 @@ __device__ __forceinline__ double exp_tab(double x, const double *tab) {
     q = fma(q, r, 1.0);
     q *= r;
     const double T = tab[N & 31];
-    const double s = __hiloint2double(((N >> 5) + 1023) << 20, 0);
-    return fma(T, q, T) * s;
+    // times 2^m by adding m to the exponent (|m| <= 58: no range to leave)
+    const double e = fma(T, q, T);
+    return __hiloint2double(__double2hiint(e) + ((N & ~31) << 15), __double2loint(e));
+}
+
+// The Peclet number clamped to [-Pmax, Pmax] (src/FreqFactors.jl:248-250) on its high word: Pmax = 40
+// has a zero low word, so |P| >= 40 shows there (a NaN clamps to +-40, as through fmin/fmax).
+__device__ __forceinline__ double clamp_P(double P) {
+    static_assert(kPmax == 40.0, "the high word of Pmax");
+    const int hi = __double2hiint(P);
+    const bool big = (hi & 0x7fffffff) >= 0x40440000;
+    return __hiloint2double(big ? (hi & 0x80000000) | 0x40440000 : hi, big ? 0 : __double2loint(P));
 }
 
 // OneMinusphi_L_and_chi_L / OneMinusphi_R_and_chi_R, src/FreqFactors.jl:54-133, in FP64.
