@@ -232,8 +232,9 @@ static void push_tiles(const lyd_ctx *c, int q, int j0, int j1, std::vector<int4
 static int cells_per_block(const lyd_ctx *c) {
     if (c->tune.cells_per_block > 0) return c->tune.cells_per_block;
     long long want = (long long)(c->ncell + 4 * c->sms - 1) / (4 * c->sms);
-    want = (want + 7) / 8 * 8;
-    return (int)std::min<long long>(1024, std::max<long long>(8, want));
+    const int warps = 8 * freq_cells_per_warp(c->nnu);       // a CTA's cells at a time
+    want = (want + warps - 1) / warps * warps;
+    return (int)std::min<long long>(1024, std::max<long long>(warps, want));
 }
 
 static int build_work(lyd_ctx *c) {

@@ -140,6 +140,7 @@ enum { ERRB_NONFINITE = 1, ERRB_SOLVE = 2, ERRB_TIMEOUT = 4 };
 constexpr int kTensorMapBytes = 128;
 
 int bins_per_lane(int nnu);
+int freq_cells_per_warp(int nnu);   // cells a warp of the frequency kernel takes at a time
 // `prec` of the step launches is a PREC_K_* variant; `sprec` of the others is the storage
 // type of the state arrays (0: double, 1: float).
 void launch_find_active(int sprec, const void *J, int nnu, const double *dnu, const double *dV, const CloudDesc *cl,

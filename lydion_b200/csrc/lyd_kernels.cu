@@ -1087,6 +1087,8 @@ struct Row {
     double a[M], b[M], c[M], d[M];
 };
 
+// (A cell's bins lie across a group of G lanes, M contiguous bins to a lane; `ln` is the lane's place in
+// its group, and every shuffle stays inside the group.)
 // Fetch, for every owned row r = lane*M + m, the quantity v of row r - s (dir = -1) or r + s
 // (dir = +1). Rows outside [0, 32M) read the identity-row value `idv`.
 template <int M>
@@ -1154,20 +1156,20 @@ __device__ __forceinline__ void pcr_solve(Row<M> &R_, int lane) {
     for (int m = 0; m < M; m++) R_.d[m] = R_.d[m] * rcp<double>(R_.b[m]);
 }
 
-// Lane-serial elimination of the same system: the warp writes its rows to shared memory and
-// lane 0 runs the forward elimination and back substitution of dgtsv's no-interchange branch
-// (the Thomas algorithm), then the rows are read back. `sm` holds 4*32*M doubles per warp.
-template <int M>
-__device__ __forceinline__ void thomas_solve(Row<M> &R_, int lane, double *sm) {
-    constexpr int N = 32 * M;
+// Lane-serial elimination of the same system: the group writes its rows to shared memory and its
+// first lane runs the forward elimination and back substitution of dgtsv's no-interchange branch
+// (the Thomas algorithm), then the rows are read back. `sm` holds 4*G*M doubles of the group.
+template <int M, int G>
+__device__ __forceinline__ void thomas_solve(Row<M> &R_, int ln, double *sm) {
+    constexpr int N = G * M;
     double *a = sm, *b = sm + N, *c = sm + 2 * N, *d = sm + 3 * N;
 #pragma unroll
     for (int m = 0; m < M; m++) {
-        int r = lane * M + m;
+        int r = ln * M + m;
         a[r] = R_.a[m]; b[r] = R_.b[m]; c[r] = R_.c[m]; d[r] = R_.d[m];
     }
     __syncwarp();
-    if (lane == 0) {
+    if (ln == 0) {
         for (int r = 1; r < N; r++) {
             double fact = a[r] / b[r - 1];
             b[r] = b[r] - fact * c[r - 1];
@@ -1179,75 +1181,31 @@ __device__ __forceinline__ void thomas_solve(Row<M> &R_, int lane, double *sm) {
     __syncwarp();
 #pragma unroll
     for (int m = 0; m < M; m++) {
-        int r = lane * M + m;
+        int r = ln * M + m;
         R_.d[m] = d[r];
         R_.b[m] = b[r];
     }
     __syncwarp();
 }
 
-// Two rows per lane (rows 2l and 2l+1): one cyclic-reduction step eliminates the odd rows,
-// leaving one row per lane, which parallel cyclic reduction across the warp solves in five
-// levels; the odd rows then follow by back-substitution. Half the divisions and shuffles of
-// PCR on all 64 rows, the same arithmetic per eliminated row. Returns x in d.
-__device__ __forceinline__ void cr_pcr_solve2(Row<2> &R_, int lane) {
-    // odd row o = 2l+1 of this lane; o- = 2l-1 is the previous lane's odd row
-    const double ibo = rcp<double>(R_.b[1]);
-    double a_om = __shfl_up_sync(0xffffffffu, R_.a[1], 1);
-    double c_om = __shfl_up_sync(0xffffffffu, R_.c[1], 1);
-    double d_om = __shfl_up_sync(0xffffffffu, R_.d[1], 1);
-    double ib_om = __shfl_up_sync(0xffffffffu, ibo, 1);
-    if (lane == 0) { a_om = 0.0; c_om = 0.0; d_om = 0.0; ib_om = 1.0; }
-    // even row e = 2l: eliminate x_{e-1} (row o-) and x_{e+1} (row o)
-    double al = -R_.a[0] * ib_om;
-    double ga = -R_.c[0] * ibo;
-    double ea = al * a_om;
-    double eb = R_.b[0] + al * c_om + ga * R_.a[1];
-    double ec = ga * R_.c[1];
-    double ed = R_.d[0] + al * d_om + ga * R_.d[1];
-    // PCR over the 32 even rows (one per lane), every row scaled to a unit diagonal so that a
-    // level fetches three values from each neighbour instead of four (and no reciprocal pivot)
-    double ib = rcp<double>(eb);
-    double na = ea * ib, nc = ec * ib, nd = ed * ib;
-#pragma unroll
-    for (int s = 1; s < 32; s <<= 1) {
-        double am = __shfl_up_sync(0xffffffffu, na, s), cm = __shfl_up_sync(0xffffffffu, nc, s);
-        double dm = __shfl_up_sync(0xffffffffu, nd, s);
-        double ap = __shfl_down_sync(0xffffffffu, na, s), cp = __shfl_down_sync(0xffffffffu, nc, s);
-        double dp = __shfl_down_sync(0xffffffffu, nd, s);
-        if (lane < s) { am = 0.0; cm = 0.0; dm = 0.0; }
-        if (lane + s > 31) { ap = 0.0; cp = 0.0; dp = 0.0; }
-        eb = fma(-na, cm, fma(-nc, ap, 1.0));
-        const double a2 = -na * am, c2 = -nc * cp;
-        const double d2 = fma(-na, dm, fma(-nc, dp, nd));
-        ib = rcp<double>(eb);
-        na = a2 * ib;
-        nc = c2 * ib;
-        nd = d2 * ib;
-    }
-    const double xe = nd;
-    // odd rows: x_o = (d_o - a_o x_e - c_o x_{e+2}) / b_o
-    double xe2 = __shfl_down_sync(0xffffffffu, xe, 1);
-    if (lane == 31) xe2 = 0.0;
-    R_.d[0] = xe;
-    R_.d[1] = (R_.d[1] - R_.a[1] * xe - R_.c[1] * xe2) * ibo;
-    R_.b[0] = eb;                      // the pivots, for the zero-pivot check (b[1] is b_o)
-}
+template <int G>
+__device__ __forceinline__ double up1(double v, int s = 1) { return __shfl_up_sync(0xffffffffu, v, s, G); }
+template <int G>
+__device__ __forceinline__ double dn1(double v, int s = 1) { return __shfl_down_sync(0xffffffffu, v, s, G); }
 
-// PCR over one row per lane (lane l holds row l of a 32-row system coupled to lanes l +- s),
+// PCR over one row per lane (lane ln of a group holds row ln of a G-row system coupled to ln +- s),
 // every row scaled to a unit diagonal so that a level fetches three values from each neighbour;
 // returns the last level's diagonal (the pivot, before scaling) in eb and x in ed.
-__device__ __forceinline__ void pcr_lanes(double &ea, double &eb, double &ec, double &ed, int lane) {
+template <int G>
+__device__ __forceinline__ void pcr_lanes(double ea, double &eb, double ec, double &ed, int ln) {
     double ib = rcp<double>(eb);
     double na = ea * ib, nc = ec * ib, nd = ed * ib;
 #pragma unroll
-    for (int s = 1; s < 32; s <<= 1) {
-        double am = __shfl_up_sync(0xffffffffu, na, s), cm = __shfl_up_sync(0xffffffffu, nc, s);
-        double dm = __shfl_up_sync(0xffffffffu, nd, s);
-        double ap = __shfl_down_sync(0xffffffffu, na, s), cp = __shfl_down_sync(0xffffffffu, nc, s);
-        double dp = __shfl_down_sync(0xffffffffu, nd, s);
-        if (lane < s) { am = 0.0; cm = 0.0; dm = 0.0; }
-        if (lane + s > 31) { ap = 0.0; cp = 0.0; dp = 0.0; }
+    for (int s = 1; s < G; s <<= 1) {
+        double am = up1<G>(na, s), cm = up1<G>(nc, s), dm = up1<G>(nd, s);
+        double ap = dn1<G>(na, s), cp = dn1<G>(nc, s), dp = dn1<G>(nd, s);
+        if (ln < s) { am = 0.0; cm = 0.0; dm = 0.0; }
+        if (ln + s > G - 1) { ap = 0.0; cp = 0.0; dp = 0.0; }
         eb = fma(-na, cm, fma(-nc, ap, 1.0));
         const double a2 = -na * am, c2 = -nc * cp;
         const double d2 = fma(-na, dm, fma(-nc, dp, nd));
@@ -1256,19 +1214,73 @@ __device__ __forceinline__ void pcr_lanes(double &ea, double &eb, double &ec, do
         nc = c2 * ib;
         nd = d2 * ib;
     }
-    ea = na;
-    ec = nc;
     ed = nd;
 }
 
+template <int G>
+__device__ __forceinline__ void cr_pcr_solve(Row<1> &R_, int ln) {
+    pcr_lanes<G>(R_.a[0], R_.b[0], R_.c[0], R_.d[0], ln);
+}
+
+// Two rows per lane (rows 2l and 2l+1): one cyclic-reduction step eliminates the odd rows, leaving
+// one row per lane, which PCR across the group solves; the odd rows then follow by
+// back-substitution. Half the divisions and shuffles of PCR on all rows, the same arithmetic per
+// eliminated row. Returns x in d; b holds the pivots for the zero-pivot check.
+template <int G>
+__device__ __forceinline__ void cr_pcr_solve(Row<2> &R_, int ln) {
+    // odd row o = 2l+1 of this lane; o- = 2l-1 is the previous lane's odd row
+    const double ibo = rcp<double>(R_.b[1]);
+    double a_om = up1<G>(R_.a[1]), c_om = up1<G>(R_.c[1]), d_om = up1<G>(R_.d[1]), ib_om = up1<G>(ibo);
+    if (ln == 0) { a_om = 0.0; c_om = 0.0; d_om = 0.0; ib_om = 1.0; }
+    // even row e = 2l: eliminate x_{e-1} (row o-) and x_{e+1} (row o)
+    const double al = -R_.a[0] * ib_om, ga = -R_.c[0] * ibo;
+    const double ea = al * a_om, ec = ga * R_.c[1];
+    double eb = R_.b[0] + al * c_om + ga * R_.a[1];
+    double ed = R_.d[0] + al * d_om + ga * R_.d[1];
+    pcr_lanes<G>(ea, eb, ec, ed, ln);
+    // odd rows: x_o = (d_o - a_o x_e - c_o x_{e+2}) / b_o
+    double xe2 = dn1<G>(ed);
+    if (ln == G - 1) xe2 = 0.0;
+    R_.d[0] = ed;
+    R_.d[1] = (R_.d[1] - R_.a[1] * ed - R_.c[1] * xe2) * ibo;
+    R_.b[0] = eb;
+}
+
+// Three rows per lane (rows 3l .. 3l+2): rows 3l+1 and 3l+2 eliminated down the lane, which leaves
+// row 3l coupled to the neighbouring lanes' rows 3l -+ 3 for the PCR; then back-substitution.
+template <int G>
+__device__ __forceinline__ void cr_pcr_solve(Row<3> &R_, int ln) {
+    const double ib1 = rcp<double>(R_.b[1]);
+    const double f = -R_.a[2] * ib1;
+    const double a2 = f * R_.a[1], b2 = fma(f, R_.c[1], R_.b[2]), d2 = fma(f, R_.d[1], R_.d[2]);
+    const double ib2 = rcp<double>(b2);
+    // x2 = A2 + B2 x0 + C2 x3, x1 = A1 + B1 x0 + C1 x3
+    const double A2 = d2 * ib2, B2 = -a2 * ib2, C2 = -R_.c[2] * ib2;
+    const double g = -R_.c[1] * ib1;
+    const double A1 = fma(g, A2, R_.d[1] * ib1), B1 = fma(g, B2, -R_.a[1] * ib1), C1 = g * C2;
+    double A2m = up1<G>(A2), B2m = up1<G>(B2), C2m = up1<G>(C2);
+    if (ln == 0) { A2m = 0.0; B2m = 0.0; C2m = 0.0; }
+    const double ea = R_.a[0] * B2m, ec = R_.c[0] * C1;
+    double eb = fma(R_.a[0], C2m, fma(R_.c[0], B1, R_.b[0]));
+    double ed = fma(-R_.a[0], A2m, fma(-R_.c[0], A1, R_.d[0]));
+    pcr_lanes<G>(ea, eb, ec, ed, ln);
+    double x3 = dn1<G>(ed);
+    if (ln == G - 1) x3 = 0.0;
+    R_.d[0] = ed;
+    R_.d[1] = fma(C1, x3, fma(B1, ed, A1));
+    R_.d[2] = fma(C2, x3, fma(B2, ed, A2));
+    R_.b[0] = eb;
+    R_.b[2] = b2;
+}
+
 // Four rows per lane (rows 4l .. 4l+3): two cyclic-reduction steps (the odd rows, then rows
-// 4l+2) leave row 4l, solved by PCR across the warp; rows 4l+2, then the odd rows follow by
-// back-substitution. Returns x in d; b holds the pivots for the zero-pivot check.
-__device__ __forceinline__ void cr_pcr_solve4(Row<4> &R_, int lane) {
+// 4l+2) leave row 4l, solved by PCR across the group; rows 4l+2, then the odd rows follow by
+// back-substitution.
+template <int G>
+__device__ __forceinline__ void cr_pcr_solve(Row<4> &R_, int ln) {
     const double ib1 = rcp<double>(R_.b[1]), ib3 = rcp<double>(R_.b[3]);
-    double a3p = __shfl_up_sync(0xffffffffu, R_.a[3], 1), c3p = __shfl_up_sync(0xffffffffu, R_.c[3], 1);
-    double d3p = __shfl_up_sync(0xffffffffu, R_.d[3], 1), ib3p = __shfl_up_sync(0xffffffffu, ib3, 1);
-    if (lane == 0) { a3p = 0.0; c3p = 0.0; d3p = 0.0; ib3p = 1.0; }
+    double a3p = up1<G>(R_.a[3]), c3p = up1<G>(R_.c[3]), d3p = up1<G>(R_.d[3]), ib3p = up1<G>(ib3);
+    if (ln == 0) { a3p = 0.0; c3p = 0.0; d3p = 0.0; ib3p = 1.0; }
     // level 1: rows 4l (eliminate 4l-1, 4l+1) and 4l+2 (eliminate 4l+1, 4l+3)
     double al = -R_.a[0] * ib3p, ga = -R_.c[0] * ib1;
     double a0 = al * a3p, b0 = R_.b[0] + al * c3p + ga * R_.a[1], c0 = ga * R_.c[1];
@@ -1279,16 +1291,15 @@ __device__ __forceinline__ void cr_pcr_solve4(Row<4> &R_, int lane) {
     double d2 = R_.d[2] + al * R_.d[1] + ga * R_.d[3];
     // level 2: row 4l eliminates 4l-2 (previous lane's row 2) and 4l+2
     const double ib2 = rcp<double>(b2);
-    double a2p = __shfl_up_sync(0xffffffffu, a2, 1), c2p = __shfl_up_sync(0xffffffffu, c2, 1);
-    double d2p = __shfl_up_sync(0xffffffffu, d2, 1), ib2p = __shfl_up_sync(0xffffffffu, ib2, 1);
-    if (lane == 0) { a2p = 0.0; c2p = 0.0; d2p = 0.0; ib2p = 1.0; }
+    double a2p = up1<G>(a2), c2p = up1<G>(c2), d2p = up1<G>(d2), ib2p = up1<G>(ib2);
+    if (ln == 0) { a2p = 0.0; c2p = 0.0; d2p = 0.0; ib2p = 1.0; }
     al = -a0 * ib2p;
     ga = -c0 * ib2;
-    double ea = al * a2p, eb = b0 + al * c2p + ga * a2, ec = ga * c2, ed = d0 + al * d2p + ga * d2;
-    pcr_lanes(ea, eb, ec, ed, lane);
+    double eb = b0 + al * c2p + ga * a2, ed = d0 + al * d2p + ga * d2;
+    pcr_lanes<G>(al * a2p, eb, ga * c2, ed, ln);
     const double x0 = ed;
-    double x4 = __shfl_down_sync(0xffffffffu, x0, 1);
-    if (lane == 31) x4 = 0.0;
+    double x4 = dn1<G>(x0);
+    if (ln == G - 1) x4 = 0.0;
     const double x2 = (d2 - a2 * x0 - c2 * x4) * ib2;
     R_.d[1] = (R_.d[1] - R_.a[1] * x0 - R_.c[1] * x2) * ib1;
     R_.d[3] = (R_.d[3] - R_.a[3] * x2 - R_.c[3] * x4) * ib3;
@@ -1303,6 +1314,13 @@ __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
+// over a group of G lanes
+template <int G>
+__device__ __forceinline__ double group_sum(double v) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
 
 // Per-bin constants of UpdateFreqFactors! staged in shared memory once per CTA. With the half-widths
 // dl = nuC - nu (left) and dr = nu_{k+1} - nuC (right) of a bin, the Peclet number at one of the three
@@ -1310,7 +1328,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 // i.e. P = vel (nuC d) / K + (h/kT) d - 2 d / nuC: KC_A* = nuC d, KC_D* = d, KC_B* = -2 d / nuC (zero without
 // recoil). *P: the left half of bin k+1, stored at k; *R: the right half of bin k (and, read at k-1,
 // of bin k-1). KC_EXP2: the 32 entries of exp_tab's table.
-enum { KC_AP, KC_DP, KC_BP, KC_AR, KC_DR, KC_BR, KC_IDNU, KC_DNU, KC_EXP2, KC_N };
+enum { KC_AP, KC_DP, KC_BP, KC_AR, KC_DR, KC_BR, KC_IDNU, KC_DNU, KC_EXP2 };
 
 // Per-cell inputs staged in shared memory, 32 cells at a time per warp, one cell per lane, already in
 // the combinations the cell loop uses: opacities times c~ dt, the source, the prefactor of K, h/kT, the
@@ -1337,40 +1355,32 @@ __device__ __forceinline__ void lds_row(const double *p, double (&v)[M]) {
     }
 }
 
-// The next cell's bin rows (J, H_r, H_Z, H_voigt, J_old) are prefetched into a per-warp double
-// buffer while the current cell computes, up to two bins per lane (four or more would leave
-// shared memory for one CTA per SM).
-template <int M> __host__ __device__ constexpr bool freq_prefetch() { return M <= 2; }
-
-// Shared memory of the frequency kernel, in doubles: FP64 per-k constants, the per-warp
-// reduction rows (without prefetch; with it, each warp's row lies in its own prefetch area,
-// free once the warp's cells are done), per-warp staged cell inputs, the per-warp prefetch
-// buffers (two slots of `ns` rows: 4, or 5 when J_old is not J's own buffer), and the
-// lane-serial solver rows when that solver runs: 71 KB per CTA at two bins per lane with J_old
-// aliased, which leaves L1 the difference. A
-// third CTA per SM would fit, but its 80-register bound spills in the cell loop (FP64 at
-// 256^2 x 64: 0.258 ms against 0.184 ms at two CTAs).
-template <int M>
-__host__ __device__ constexpr int freq_smem_off_cs(int nwarps) {
-    return KC_N * 32 * M + (freq_prefetch<M>() ? 0 : nwarps * (32 * M + 8));
+// Shared memory of the frequency kernel, in doubles: the FP64 per-bin constants (NP = G M padded bins);
+// per warp the staged cell inputs; up to 64 bins, per warp two slots (the cells at hand and the next
+// ones, whose rows are copied in meanwhile) of `ns` rows: J, H_r, H_Z, H_voigt, and with G = 32 J_old when
+// it is not J's own buffer; and the lane-serial solver's rows when it runs. A warp's reduction row
+// overlays its slots, which are free once its cells are done. 71 KB per CTA at 64 bins, 87 KB at 48:
+// two CTAs per SM. A third CTA per SM would fit at 64 bins, but its 80-register bound spills in the cell
+// loop (FP64 at 256^2 x 64: 0.258 ms against 0.184 ms at two CTAs).
+template <int M, int G> __host__ __device__ constexpr bool freq_prefetch() { return G * M <= 64; }
+template <int M, int G>
+__host__ __device__ constexpr int freq_rows_warp(int ns) {      // doubles per warp
+    return freq_prefetch<M, G>() ? 2 * ns * 32 * M : 32 * M + 8;
 }
-template <int M>
-__host__ __device__ constexpr int freq_smem_off_pf(int nwarps) { return freq_smem_off_cs<M>(nwarps) + nwarps * CS_N * 32; }
-template <int M>
-__host__ __device__ constexpr int freq_pf_warp(int ns) { return 2 * ns * 32 * M; }   // doubles per warp
-template <int M>
+template <int M, int G>
+__host__ __device__ constexpr int freq_smem_off_cs() { return KC_EXP2 * G * M + 32; }
+template <int M, int G>
+__host__ __device__ constexpr int freq_smem_off_rows(int nwarps) { return freq_smem_off_cs<M, G>() + nwarps * CS_N * 32; }
+template <int M, int G>
 __host__ __device__ constexpr int freq_smem_off_tsm(int nwarps, int ns) {
-    return freq_smem_off_pf<M>(nwarps) + (freq_prefetch<M>() ? nwarps * freq_pf_warp<M>(ns) : 0);
+    return freq_smem_off_rows<M, G>(nwarps) + nwarps * freq_rows_warp<M, G>(ns);
 }
-template <int M>
+template <int M, int G>
 __host__ __device__ constexpr int freq_smem_doubles(int nwarps, bool thomas, int ns) {
-    return freq_smem_off_tsm<M>(nwarps, ns) + (thomas ? nwarps * 4 * 32 * M : 0);
+    return freq_smem_off_tsm<M, G>(nwarps, ns) + (thomas ? nwarps * 4 * 32 * M : 0);
 }
-template <int M>
-__host__ __device__ inline double *freq_red_row(double *fsm, int nwarps, int ns, int w) {
-    return freq_prefetch<M>() ? fsm + freq_smem_off_pf<M>(nwarps) + w * freq_pf_warp<M>(ns)
-                              : fsm + KC_N * 32 * M + w * (32 * M + 8);
-}
+// rows of a slot
+template <int G> __host__ __device__ constexpr int freq_ns(bool jo_alias) { return G == 32 && !jo_alias ? 5 : 4; }
 
 // A lane's M contiguous bins of one row as whole 16-byte words, when the row layout allows it
 // (k_freq's `vec` path): loads from shared memory and stores to global memory.
@@ -1400,16 +1410,20 @@ struct LaneRow {
 };
 
 // The cells [wbeg, wend) of a work item that warp `warp` of `nw` handles: one contiguous run
-// per warp (k_freq and k_find_active sum their partials in this order).
-__device__ __forceinline__ void warp_cell_run(int4 it, int warp, int nw, int &wbeg, int &wend) {
-    const int per = (it.z - it.y + nw - 1) / nw;
+// per warp, of a multiple of `cpw` cells.
+__device__ __forceinline__ void warp_cell_run(int4 it, int warp, int nw, int cpw, int &wbeg, int &wend) {
+    const int per = ((it.z - it.y + nw - 1) / nw + cpw - 1) / cpw * cpw;
     wbeg = it.y + warp * per;
     wend = min(it.z, wbeg + per);
 }
 
-// Up to four bins per lane the kernel is held to 2 CTAs per SM (128 registers). Four bins:
-// ~230 B of spills, measured 1.4x faster than 1 CTA at 172 registers. Two bins: 1.8x faster
-// than the 164 registers ptxas picks when only the block size bounds it.
+// Up to four bins per lane the kernel is held to 2 CTAs per SM (128 registers).
+// A cell's bins lie across a group of G lanes, M contiguous bins to a lane: up to 48 bins half a warp
+// (two cells per warp, 1, 2 or 3 bins per lane), beyond a whole warp. With whole warps 48 bins left 8 of
+// 32 lanes idle and the solve took five levels across 32 lanes for each cell; by halves every lane has
+// work, a level serves two cells and there are four: 24 clouds x 48 bins 123 -> 86 us per launch. At 64
+// bins half warps (4 bins per lane) spill: 149 us against 140 at 256^2 in FP64, so they keep the
+// whole warp.
 // RC is the arithmetic of the cell-centre closure D(J, H) and of D:grad u that enter the Doppler
 // term of the frequency factors: R in the FP64 and FP32-storage forms, FP32 in the mixed form.
 // The closure only sets the velocity of the Peclet numbers; every factor is then formed in FP64
@@ -1429,15 +1443,17 @@ __device__ __forceinline__ void warp_cell_run(int4 it, int warp, int nw, int &wb
 // freq_item is one work item (`item` of `nitems`) by the calling CTA, whose first `nw` warps take
 // its cells (the others only meet its barriers), in dynamic shared memory `fsm`: the body of
 // k_freq, also run by the persistent batch kernel.
-template <typename S, typename R, int M, typename RC>
+template <typename S, typename R, int M, int G, typename RC>
 __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int nitems, double *fsm, int nw) {
-    constexpr int NP = 32 * M;
-    constexpr bool PF = freq_prefetch<M>();
+    constexpr int NP = G * M, WN = 32 * M, CPW = 32 / G;   // a cell's padded bins, a warp's, a warp's cells
+    constexpr bool PF = freq_prefetch<M, G>(), PARK = M == 3;
+    static_assert(freq_rows_warp<M, G>(4) >= NP + 8, "a warp's reduction row fits its rows");
     const bool jo_alias = a.Jold == a.Jin;
-    const int ns = jo_alias ? 4 : 5;               // prefetched rows per cell
-    double *kc = fsm;                                  // [KC_N][NP]
-    double *tsm = fsm + freq_smem_off_tsm<M>(nw, ns);  // [nwarps][4][NP] (lane-serial solver)
+    const int ns = freq_ns<G>(jo_alias);                  // rows of a slot
+    double *kc = fsm;                                     // [KC_EXP2][NP], then the exponentials' table
+    double *tsm = fsm + freq_smem_off_tsm<M, G>(nw, ns);  // [nwarps][CPW][4][NP] (lane-serial solver)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ln = lane & (G - 1), sub = lane / G;        // place in the cell's group, the group's cell
     const int nnu = a.nnu;
     for (int t = threadIdx.x; t < NP; t += blockDim.x) {
         const bool up = t + 1 < nnu, in = t < nnu;
@@ -1450,8 +1466,8 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
         kc[KC_BR * NP + t] = in && a.recoil ? -2.0 * dr * a.inv_nuC[t] : 0.0;
         kc[KC_IDNU * NP + t] = in ? a.inv_dnu[t] : 0.0;
         kc[KC_DNU * NP + t] = in ? a.dnu[t] : 0.0;
-        kc[KC_EXP2 * NP + t] = (t < 32) ? kExp2Tab[t] : 0.0;
     }
+    if (threadIdx.x < 32) kc[KC_EXP2 * NP + threadIdx.x] = kExp2Tab[threadIdx.x];
     __syncthreads();
 
     const int4 it = a.items[item];
@@ -1468,48 +1484,90 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
     int bad = 0;
 
     int wbeg, wend;
-    warp_cell_run(it, warp, nw, wbeg, wend);
-    double *cs = fsm + freq_smem_off_cs<M>(nw) + warp * CS_N * 32;      // [CS_N][32]
-    S *pf = reinterpret_cast<S *>(fsm + freq_smem_off_pf<M>(nw) + warp * freq_pf_warp<M>(ns));  // [2][ns][NP]
+    warp_cell_run(it, warp, nw, CPW, wbeg, wend);
+    double *cs = fsm + freq_smem_off_cs<M, G>() + warp * CS_N * 32;      // [CS_N][32]
+    S *rows = reinterpret_cast<S *>(fsm + freq_smem_off_rows<M, G>(nw) + warp * freq_rows_warp<M, G>(ns));
     const bool need_ff = a.do_freq && a.update_ff, need_js = a.do_emission || (a.parts & PART_DIAG);
-    // With `vec`, every lane's M bins of a row are whole 16-byte words in global and shared
-    // memory (row starts 16-byte aligned, n_nu a multiple of M): rows move as 16-byte copies,
-    // loads and stores, bin m of lane l at l*M + m. Otherwise element by element, bin m of
-    // lane l at m*32 + l.
+    // With `vec`, every lane's M bins of a row are whole 16-byte words in global and shared memory
+    // (row starts 16-byte aligned, n_nu a multiple of M). A group of a whole warp (G = 32) then moves its
+    // rows lane by lane, bin m of lane l at l*M + m, else element by element, bin m of lane l at
+    // m*32 + l; groups of 16 copy their two cells' rows as the one run they are in memory.
     using LR = LaneRow<S, M>;
-    const bool vec = LR::ok && a.vec16;
-    // copies of cell cl's bin rows into prefetch buffer b
+    const bool vec = LR::ok && a.vec16 && nnu % M == 0;
+    // copies of the rows of cells cl .. into slot b
     auto issue = [&](int cl, int b) {
         const long long base = o3 + (long long)cl * nnu;
-        S *d = pf + b * ns * NP;
-        if constexpr (LR::ok) {
-            if (vec) {
-                if (lane * M < nnu) {
-                    const long long g = base + lane * M;
-                    const int q = lane * M;
-                    constexpr int per = 16 / sizeof(S);
+        S *d = rows + b * ns * WN;
+        constexpr int per = 16 / sizeof(S);
+        if constexpr (G == 32) {
+            if constexpr (LR::ok) {
+                if (vec) {
+                    if (lane * M < nnu) {
+                        const long long g = base + lane * M;
+                        const int q = lane * M;
 #pragma unroll
-                    for (int w = 0; w < LR::words; w++) {
-                        cp_async_16(d + q + w * per, a.Jin + g + w * per);
-                        cp_async_16(d + NP + q + w * per, a.Hrin + g + w * per);
-                        cp_async_16(d + 2 * NP + q + w * per, a.HZin + g + w * per);
-                        cp_async_16(d + 3 * NP + q + w * per, a.Hv + g + w * per);
-                        if (!jo_alias) cp_async_16(d + 4 * NP + q + w * per, a.Jold + g + w * per);
+                        for (int w = 0; w < LR::words; w++) {
+                            cp_async_16(d + q + w * per, a.Jin + g + w * per);
+                            cp_async_16(d + WN + q + w * per, a.Hrin + g + w * per);
+                            cp_async_16(d + 2 * WN + q + w * per, a.HZin + g + w * per);
+                            cp_async_16(d + 3 * WN + q + w * per, a.Hv + g + w * per);
+                            if (!jo_alias) cp_async_16(d + 4 * WN + q + w * per, a.Jold + g + w * per);
+                        }
                     }
+                    return;
                 }
-                return;
+            }
+#pragma unroll
+            for (int m = 0; m < M; m++) {
+                const int k = lane * M + m, q = m * 32 + lane;
+                if (k < nnu) {
+                    cp_async_el(d + q, a.Jin + base + k);
+                    cp_async_el(d + WN + q, a.Hrin + base + k);
+                    cp_async_el(d + 2 * WN + q, a.HZin + base + k);
+                    cp_async_el(d + 3 * WN + q, a.Hv + base + k);
+                    if (!jo_alias) cp_async_el(d + 4 * WN + q, a.Jold + base + k);
+                }
+            }
+        } else {
+            const int n = min(CPW, wend - cl) * nnu;
+            if (a.vec16) {
+                for (int e = lane * per; e < n; e += 32 * per) {
+                    cp_async_16(d + e, a.Jin + base + e);
+                    cp_async_16(d + WN + e, a.Hrin + base + e);
+                    cp_async_16(d + 2 * WN + e, a.HZin + base + e);
+                    cp_async_16(d + 3 * WN + e, a.Hv + base + e);
+                }
+            } else {
+                for (int e = lane; e < n; e += 32) {
+                    cp_async_el(d + e, a.Jin + base + e);
+                    cp_async_el(d + WN + e, a.Hrin + base + e);
+                    cp_async_el(d + 2 * WN + e, a.HZin + base + e);
+                    cp_async_el(d + 3 * WN + e, a.Hv + base + e);
+                }
             }
         }
+    };
+    // a lane's bins of a row that starts at p (in shared or global memory), zeros beyond n_nu
+    auto row_get = [&](const S *p, bool ok, S (&v)[M]) {
+        if (vec) {
+            if (ok && ln * M < nnu) {
+                LR::load(p + ln * M, v);
+            } else {
 #pragma unroll
-        for (int m = 0; m < M; m++) {
-            const int k = lane * M + m, q = m * 32 + lane;
-            if (k < nnu) {
-                cp_async_el(d + q, a.Jin + base + k);
-                cp_async_el(d + NP + q, a.Hrin + base + k);
-                cp_async_el(d + 2 * NP + q, a.HZin + base + k);
-                cp_async_el(d + 3 * NP + q, a.Hv + base + k);
-                if (!jo_alias) cp_async_el(d + 4 * NP + q, a.Jold + base + k);
+                for (int m = 0; m < M; m++) v[m] = S(0);
             }
+        } else {
+#pragma unroll
+            for (int m = 0; m < M; m++) v[m] = (ok && ln * M + m < nnu) ? p[ln * M + m] : S(0);
+        }
+    };
+    auto row_put = [&](S *p, bool ok, const S (&v)[M]) {
+        if (vec) {
+            if (ok && ln * M < nnu) LR::store(p + ln * M, v);
+        } else {
+#pragma unroll
+            for (int m = 0; m < M; m++)
+                if (ok && ln * M + m < nnu) p[ln * M + m] = v[m];
         }
     };
     const double k4 = kFourPiOverC * (1.0 / c_tilde) * a.j_scale;
@@ -1552,20 +1610,20 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
         cp_async_commit();
     }
     int g0 = wbeg;
-    int i = wbeg % nr - 1, j = wbeg / nr;      // the cell's column and row, advanced with it
+    int i = (wbeg + sub) % nr, j = (wbeg + sub) / nr;     // the cell's column and row, advanced with it
     S nonfin = S(0);                           // 0 x everything written: NaN once something is not finite
-    for (int cl = wbeg; cl < wend; cl++) {
-        if (++i == nr) { i = 0; j++; }
-        const long long c = oc + cl;
+    for (int c0 = wbeg; c0 < wend; c0 += CPW) {
+        const int cl = c0 + sub;               // this group's cell (a last odd one leaves groups idle)
+        const bool ok = G == 32 || cl < wend;
         const long long base = o3 + (long long)cl * nnu;
-        if (((cl - wbeg) & 31) == 0) {
-            if (cl > wbeg) flush(g0, cl);
+        if (((c0 - wbeg) & 31) == 0) {
+            if (c0 > wbeg) flush(g0, c0);
             // stage the per-cell inputs of the next 32 cells of the run (one coalesced load per
             // field instead of a dependent load per cell)
-            g0 = cl;
+            g0 = c0;
             __syncwarp();
-            const bool v = cl + lane < wend;
-            const long long cc = c + lane;
+            const bool v = c0 + lane < wend;
+            const long long cc = oc + c0 + lane;
             auto ld = [&](const double *p, bool need) { return (v && need && p) ? __ldg(p + cc) : 0.0; };
             const double alv = ld(a.alpha, a.do_emission || need_ff), js = ld(a.js, need_js);
             const double dV = ld(a.dV, a.parts != 0);
@@ -1595,12 +1653,13 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
         S J[M], Hr[M], HZ[M];
         R Hv[M];
         double Jo[M];
-        if constexpr (PF) {
-            const int b = (cl - wbeg) & 1;
-            if (cl + 1 < wend) issue(cl + 1, b ^ 1);
+        S *rH = rows;                             // where H_r, H_Z wait: rows WN apart
+        if constexpr (G == 32 && PF) {
+            const int b = (c0 - wbeg) & 1;
+            if (c0 + 1 < wend) issue(c0 + 1, b ^ 1);
             cp_async_commit();
             cp_async_wait<1>();                   // this cell's copies (each lane reads its own)
-            const S *d = pf + b * ns * NP;
+            const S *d = rows + b * ns * WN;
             bool done = false;
             if constexpr (LR::ok) {
                 if (vec) {
@@ -1608,10 +1667,10 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
                         const int q = lane * M;
                         S hv[M], jo[M];
                         LR::load(d + q, J);
-                        LR::load(d + NP + q, Hr);
-                        LR::load(d + 2 * NP + q, HZ);
-                        LR::load(d + 3 * NP + q, hv);
-                        LR::load(d + (jo_alias ? 0 : 4 * NP) + q, jo);
+                        LR::load(d + WN + q, Hr);
+                        LR::load(d + 2 * WN + q, HZ);
+                        LR::load(d + 3 * WN + q, hv);
+                        LR::load(d + (jo_alias ? 0 : 4 * WN) + q, jo);
 #pragma unroll
                         for (int m = 0; m < M; m++) { Hv[m] = R(hv[m]); Jo[m] = double(jo[m]); }
                     } else {
@@ -1627,13 +1686,13 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
                     const int k = lane * M + m, q = m * 32 + lane;
                     const bool vld = k < nnu;
                     J[m] = vld ? d[q] : S(0);
-                    Hr[m] = vld ? d[NP + q] : S(0);
-                    HZ[m] = vld ? d[2 * NP + q] : S(0);
-                    Hv[m] = vld ? R(d[3 * NP + q]) : R(0);
-                    Jo[m] = vld ? double(jo_alias ? d[q] : d[4 * NP + q]) : 0.0;
+                    Hr[m] = vld ? d[WN + q] : S(0);
+                    HZ[m] = vld ? d[2 * WN + q] : S(0);
+                    Hv[m] = vld ? R(d[3 * WN + q]) : R(0);
+                    Jo[m] = vld ? double(jo_alias ? d[q] : d[4 * WN + q]) : 0.0;
                 }
             }
-        } else {
+        } else if constexpr (G == 32) {
 #pragma unroll
             for (int m = 0; m < M; m++) {
                 int k = lane * M + m;
@@ -1644,6 +1703,26 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
                 Hv[m] = vld ? R(__ldg(a.Hv + base + k)) : R(0);
                 Jo[m] = vld ? double(a.Jold[base + k]) : 0.0;
             }
+        } else {
+            S hv[M], jo[M];
+            if (!jo_alias) row_get(a.Jold + base, ok, jo);
+            const int b = ((c0 - wbeg) / CPW) & 1;
+            __syncwarp();                         // every lane is done with the other slot
+            if (c0 + CPW < wend) issue(c0 + CPW, b ^ 1);
+            cp_async_commit();
+            cp_async_wait<1>();                   // these cells' copies
+            __syncwarp();
+            S *d = rows + b * ns * WN + sub * nnu;
+            row_get(d, ok, J);
+            row_get(d + WN, ok, Hr);
+            row_get(d + 2 * WN, ok, HZ);
+            row_get(d + 3 * WN, ok, hv);
+            rH = d + WN;
+#pragma unroll
+            for (int m = 0; m < M; m++) {
+                Hv[m] = R(hv[m]);
+                Jo[m] = double(jo_alias ? J[m] : jo[m]);
+            }
         }
         double dr_sum = 0.0, dz_sum = 0.0;
         // ---- LyaEmissionAbsorptionUpdate! (src/ConstantsAndFunctions.jl:526-567) ----
@@ -1651,14 +1730,14 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
             const R al = R(cv[CS_AL * 32]), ac = R(cv[CS_AC * 32]), apd = R(cv[CS_APD * 32]);
             const R acF = R(cv[CS_ACF * 32]), src = R(cv[CS_SRC * 32]);
             double dn[M];
-            lds_row<M>(kc + KC_DNU * NP + lane * M, dn);
+            lds_row<M>(kc + KC_DNU * NP + ln * M, dn);
 #pragma unroll
             for (int m = 0; m < M; m++) {
-                const int k = lane * M + m;
+                const int k = ln * M + m;
                 R phi = (k >= a.phi_kmin && k <= a.phi_kmax) ? Hv[m] : R(0);
                 R aH = al * Hv[m] + acF;
-                if (a.phi) phi = k < nnu ? R(__ldg(a.phi + base + k)) : R(0);
-                if (a.aF) aH = k < nnu ? R(__ldg(a.aF + base + k)) * R(ctdt_e) : R(0);
+                if (a.phi) phi = ok && k < nnu ? R(__ldg(a.phi + base + k)) : R(0);
+                if (a.aF) aH = ok && k < nnu ? R(__ldg(a.aF + base + k)) * R(ctdt_e) : R(0);
                 // (bins beyond n_nu hold zeros and have no width)
                 const R Jn = (R(Jo[m]) + src * phi) * rcp<R>(R(1) + (ac + apd * Hv[m]));
                 const R iden = rcp<R>(R(1) + aH);
@@ -1670,10 +1749,10 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
                 J[m] = S(Jn);
                 Jo[m] = double(J[m]);
             }
-            dr_sum = warp_sum(dr_sum);
-            dz_sum = warp_sum(dz_sum);
+            dr_sum = group_sum<G>(dr_sum);
+            dz_sum = group_sum<G>(dz_sum);
         }
-        if (lane == 0) {     // turned into the cell's momentum and diagnostics by flush()
+        if (ln == 0) {       // turned into the cell's momentum and diagnostics by flush()
             cs[CS_SUM_R * 32 + (cl - g0)] = dr_sum;
             cs[CS_SUM_Z * 32 + (cl - g0)] = dz_sum;
         }
@@ -1695,13 +1774,24 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
                 double iK[M];
 #pragma unroll
                 for (int m = 0; m < M; m++) iK[m] = rcp<double>(pref * double(Hv[m]));
-                const double iK_up = __shfl_up_sync(0xffffffffu, iK[M - 1], 1);
-                const double iK_dn = __shfl_down_sync(0xffffffffu, iK[0], 1);
-                const double *kl = kc + lane * M, *etab = kc + KC_EXP2 * NP;
+                const double iK_up = up1<G>(iK[M - 1]), iK_dn = dn1<G>(iK[0]);
+                const double *kl = kc + ln * M, *etab = kc + KC_EXP2 * NP;
                 // the right half of the bin below the lane's first
-                const int kb = lane > 0 ? -1 : 0;
+                const int kb = ln > 0 ? -1 : 0;
                 double ar = kl[KC_AR * NP + kb], drr = kl[KC_DR * NP + kb], br = kl[KC_BR * NP + kb];
-                constexpr int W = M >= 2 ? 2 : 1;       // bins whose constants are held at a time
+                // three bins per lane: H_r and H_Z wait in their rows while the factors and the solve use the
+                // registers (24 clouds x 48 bins 94 -> 86 us)
+                double vel[M];
+                auto vel_of = [&](int m) {
+                    return double(work_rate<RC>(RC(J[m]), RC(Hr[m]), RC(HZ[m]), RC(jeps), RC(a.heps2), g0, g12, g3, tr));
+                };
+                if constexpr (PARK) {
+#pragma unroll
+                    for (int m = 0; m < M; m++) vel[m] = vel_of(m);
+                    row_put(rH, ok, Hr);
+                    row_put(rH + WN, ok, HZ);
+                }
+                constexpr int W = M % 2 == 0 ? 2 : 1;   // bins whose constants are held at a time
 #pragma unroll
                 for (int mb = 0; mb < M; mb += W) {
                     double AP[W], DP[W], BP[W], AR[W], DR[W], BR[W], idn[W];
@@ -1715,14 +1805,13 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
 #pragma unroll
                     for (int w = 0; w < W; w++) {
                         const int m = mb + w;
-                        const double vel = double(work_rate<RC>(RC(J[m]), RC(Hr[m]), RC(HZ[m]), RC(jeps), RC(a.heps2),
-                                                                g0, g12, g3, tr));
+                        if constexpr (!PARK) vel[m] = vel_of(m);
                         const double iKm = (m > 0) ? iK[m > 0 ? m - 1 : 0] : iK_up;
                         const double iKp = (m < M - 1) ? iK[m < M - 1 ? m + 1 : 0] : iK_dn;
                         const double rkp = DP[w] * iKp, rk = DR[w] * iK[m], rkm = drr * iKm;
-                        const double Pkp = clamp_P(fma(vel * AP[w], iKp, fma(rec0, DP[w], BP[w])));
-                        const double Pk = clamp_P(fma(vel * AR[w], iK[m], fma(rec0, DR[w], BR[w])));
-                        const double Pkm = clamp_P(fma(vel * ar, iKm, fma(rec0, drr, br)));
+                        const double Pkp = clamp_P(fma(vel[m] * AP[w], iKp, fma(rec0, DP[w], BP[w])));
+                        const double Pk = clamp_P(fma(vel[m] * AR[w], iK[m], fma(rec0, DR[w], BR[w])));
+                        const double Pkm = clamp_P(fma(vel[m] * ar, iKm, fma(rec0, drr, br)));
                         double oRkp, xRkp, oLk, xLk, oRk, xRk, oLkm, xLkm;
                         omphi_R(Pkp, oRkp, xRkp, etab);
                         omphi_LR(Pk, oLk, xLk, oRk, xRk, etab);
@@ -1738,9 +1827,9 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
                 if (a.Fkp) {
 #pragma unroll
                     for (int m = 0; m < M; m++) {
-                        int k = lane * M + m;
+                        int k = ln * M + m;
                         const bool in = k >= 1 && k <= nnu - 2;
-                        if (k < nnu) {
+                        if (ok && k < nnu) {
                             a.Fkp[base + k] = in ? Fp[m] : 0.0;
                             a.Fk[base + k] = in ? F0[m] : 0.0;
                             a.Fkm[base + k] = in ? Fm[m] : 0.0;
@@ -1750,8 +1839,8 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
             } else {
 #pragma unroll
                 for (int m = 0; m < M; m++) {
-                    int k = lane * M + m;
-                    bool in = (k >= 1 && k <= nnu - 2);
+                    int k = ln * M + m;
+                    bool in = (ok && k >= 1 && k <= nnu - 2);
                     Fp[m] = in ? a.Fkp[base + k] : 0.0;
                     F0[m] = in ? a.Fk[base + k] : 0.0;
                     Fm[m] = in ? a.Fkm[base + k] : 0.0;
@@ -1761,23 +1850,28 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
             // first and last rows to k = 0 and k = nnu-1 are dropped (TridiagonalSolver.jl:45-46)
 #pragma unroll
             for (int m = 0; m < M; m++) {
-                int k = lane * M + m;
-                bool in = (k >= 1 && k <= nnu - 2);
+                int k = ln * M + m;
+                bool in = (ok && k >= 1 && k <= nnu - 2);
                 sys.a[m] = (in && k >= 2) ? Fm[m] : 0.0;
                 sys.b[m] = in ? -(F0[m] + dw) : 1.0;
                 sys.c[m] = (in && k <= nnu - 3) ? Fp[m] : 0.0;
                 sys.d[m] = in ? -dw * Jo[m] : 0.0;
             }
             if (a.solver == SOLVER_THOMAS)
-                thomas_solve<M>(sys, lane, tsm + warp * 4 * NP);
+                thomas_solve<M, G>(sys, ln, tsm + (warp * CPW + sub) * 4 * NP);
             else
-                if constexpr (M == 2) cr_pcr_solve2(sys, lane);
-                else if constexpr (M == 4) cr_pcr_solve4(sys, lane);
+                if constexpr (M <= 4) cr_pcr_solve<G>(sys, ln);
                 else pcr_solve<M>(sys, lane);
+            if constexpr (PARK) {
+                if (a.update_ff) {
+                    row_get(rH, ok, Hr);
+                    row_get(rH + WN, ok, HZ);
+                }
+            }
             // flux correction, src/UpdateLyaJandH.jl:341-377
 #pragma unroll
             for (int m = 0; m < M; m++) {
-                int k = lane * M + m;
+                int k = ln * M + m;
                 bool in = (k >= 1 && k <= nnu - 2);
                 double Jn = in ? sys.d[m] : double(J[m]);
                 if (!(sys.b[m] != 0.0)) bad |= ERRB_SOLVE;
@@ -1795,32 +1889,18 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
                 HZ[m] = S(hz);
             }
         }
-        // ---- store ----
-        if (LR::ok && vec) {
-            if (lane * M < nnu) {
+        // ---- store (bins beyond n_nu hold the floor and zeros) ----
 #pragma unroll
-                for (int m = 0; m < M; m++) nonfin += J[m] * S(0) + Hr[m] * S(0) + HZ[m] * S(0);
-                LR::store(a.Jout + base + lane * M, J);
-                LR::store(a.Hrout + base + lane * M, Hr);
-                LR::store(a.HZout + base + lane * M, HZ);
-            }
-        } else {
-#pragma unroll
-            for (int m = 0; m < M; m++) {
-                int k = lane * M + m;
-                if (k >= nnu) continue;
-                nonfin += J[m] * S(0) + Hr[m] * S(0) + HZ[m] * S(0);
-                a.Jout[base + k] = J[m];
-                a.Hrout[base + k] = Hr[m];
-                a.HZout[base + k] = HZ[m];
-            }
-        }
+        for (int m = 0; m < M; m++) nonfin += J[m] * S(0) + Hr[m] * S(0) + HZ[m] * S(0);
+        row_put(a.Jout + base, ok, J);
+        row_put(a.Hrout + base, ok, Hr);
+        row_put(a.HZout + base, ok, HZ);
         // ---- epilogue partials ----
         if (a.parts & PART_ACTIVE) {
             // (bins beyond n_nu have no width)
             const double dV = cv[CS_DV * 32];
             double dn[M];
-            lds_row<M>(kc + KC_DNU * NP + lane * M, dn);
+            lds_row<M>(kc + KC_DNU * NP + ln * M, dn);
 #pragma unroll
             for (int m = 0; m < M; m++) {
                 const double Jv = double(J[m]), w = dn[m] * dV;
@@ -1832,14 +1912,14 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
         if (a.parts & PART_DIAG) {
             // escaping flux through the outer r face, the top face and (outflow) the bottom face
             double esc = 0.0;
-            const bool rb = (i == nr - 1), zt = (j == nz - 1), zb = (j == 0 && bzb == 1);
+            const bool rb = ok && i == nr - 1, zt = ok && j == nz - 1, zb = ok && j == 0 && bzb == 1;
             if (rb || zt || zb) {
                 const double Arr = rb ? __ldg(a.A_r + cd.orf + nr + (long long)(nr + 1) * j) * kFourPi : 0.0;
                 const double AZt = zt ? __ldg(a.A_Z + cd.ozf + i + (long long)nr * nz) * kFourPi : 0.0;
                 const double AZb = zb ? __ldg(a.A_Z + cd.ozf + i) * kFourPi : 0.0;
 #pragma unroll
                 for (int m = 0; m < M; m++) {
-                    int k = lane * M + m;
+                    int k = ln * M + m;
                     if (k >= nnu) continue;
                     double dn = kc[KC_DNU * NP + k];
                     double hr = double(S(Hr[m])) * a.j_scale, hz = double(S(HZ[m])) * a.j_scale;
@@ -1850,6 +1930,7 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
             }
             acc_esc += esc;
         }
+        for (i += CPW; i >= nr; i -= nr) j++;
     }
     if (wbeg < wend) flush(g0, wend);
     if (nonfin != S(0)) bad |= ERRB_NONFINITE;
@@ -1857,11 +1938,15 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
     if (bad) atomicOr(a.err, bad);
     if (!a.parts) return;
     // ---- CTA reduction of the partials, fixed order ----
-    // (the warp's own row: with prefetch it overlays the warp's prefetch area, whose last copies
-    // landed above)
-    double *red = freq_red_row<M>(fsm, nw, ns, warp);
+    // (the warp's reduction row overlays its rows, whose last copies landed above)
+    auto red_row = [&](int w) { return fsm + freq_smem_off_rows<M, G>(nw) + w * freq_rows_warp<M, G>(ns); };
+    double *red = red_row(warp);
     __syncwarp();
-    if (warp < nw) {
+#pragma unroll
+    for (int m = 0; m < M; m++)
+#pragma unroll
+        for (int o = G; o < 32; o <<= 1) acc_e[m] += __shfl_xor_sync(0xffffffffu, acc_e[m], o);
+    if (warp < nw && lane < G) {
 #pragma unroll
         for (int m = 0; m < M; m++) red[lane * M + m] = acc_e[m];
     }
@@ -1884,20 +1969,20 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
     for (int col = threadIdx.x; col < ncols; col += blockDim.x) {
         int src = col < nnu ? col : NP + (col - nnu);
         double s = 0.0;
-        for (int w2 = 0; w2 < nw; w2++) s += freq_red_row<M>(fsm, nw, ns, w2)[src];
+        for (int w2 = 0; w2 < nw; w2++) s += red_row(w2)[src];
         a.partials[(size_t)col * nitems + item] = s;
     }
 }
 
-template <typename S, typename R, int M, typename RC = R>
+template <typename S, typename R, int M, int G, typename RC = R>
 __global__ void __launch_bounds__(FREQ_THREADS, M <= 4 ? 2 : 1) k_freq(FreqArgs<S> a) {
     extern __shared__ __align__(16) double fsm[];
-    freq_item<S, R, M, RC>(a, a.item0 + (int)blockIdx.x, a.nitems_all ? a.nitems_all : (int)gridDim.x, fsm,
+    freq_item<S, R, M, G, RC>(a, a.item0 + (int)blockIdx.x, a.nitems_all ? a.nitems_all : (int)gridDim.x, fsm,
                            blockDim.x >> 5);
 }
 
-// FindActiveBins partials of the current J (src/UpdateLyaJandH.jl:47-97): one warp per cell,
-// the same work items (and so the same summation order) as k_freq.
+// FindActiveBins partials of the current J (src/UpdateLyaJandH.jl:47-97): one warp per cell, over
+// the work items of k_freq.
 template <typename S, int M>
 __global__ void __launch_bounds__(FREQ_THREADS) k_find_active(const S *J, int nnu, const double *dnu,
                                                               const double *dV, const CloudDesc *cl, const int4 *items,
@@ -1912,7 +1997,7 @@ __global__ void __launch_bounds__(FREQ_THREADS) k_find_active(const S *J, int nn
     for (int m = 0; m < M; m++) acc_e[m] = 0.0;
     double acc_tot = 0.0;
     int wbeg, wend;
-    warp_cell_run(it, warp, nw, wbeg, wend);
+    warp_cell_run(it, warp, nw, 1, wbeg, wend);
     for (int c = wbeg; c < wend; c++) {
         const double v = __ldg(dV + oc + c);
 #pragma unroll
@@ -2092,7 +2177,7 @@ struct PersistArgs {
 };
 
 // RA: arithmetic of the advection; RF, RC: of the frequency step and its closure (as k_freq).
-template <typename S, typename RA, typename RF, typename RC, int FLUX, int M>
+template <typename S, typename RA, typename RF, typename RC, int FLUX, int M, int G>
 __global__ void __launch_bounds__(PT, 2) k_step_persistent(PersistArgs<S> p) {
     extern __shared__ __align__(128) unsigned char psm[];
     for (int t = blockIdx.x; t < p.ntiles; t += gridDim.x) {
@@ -2101,7 +2186,7 @@ __global__ void __launch_bounds__(PT, 2) k_step_persistent(PersistArgs<S> p) {
     }
     if (!grid_barrier(p.bar, gridDim.x, p.polls, p.err)) return;
     for (int it = blockIdx.x; it < p.nitems; it += gridDim.x) {
-        freq_item<S, RF, M, RC>(p.freq, it, p.nitems, reinterpret_cast<double *>(psm), FREQ_THREADS / 32);
+        freq_item<S, RF, M, G, RC>(p.freq, it, p.nitems, reinterpret_cast<double *>(psm), FREQ_THREADS / 32);
         __syncthreads();
     }
     if (!grid_barrier(p.bar, gridDim.x, p.polls, p.err)) return;
@@ -2181,34 +2266,45 @@ int freq_blocks(int ncell, int dev) {
 
 static bool al16(const void *p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-template <typename S, typename R, int M, typename RC>
+// Every row of every cloud starts on a 16-byte boundary when the buffers do and a row (n_nu elements) is
+// a multiple of 16 bytes: cloud offsets are sums of whole rows.
+template <typename S>
+static int rows_vec16(const FreqArgs<S> &f) {
+    return (f.nnu * sizeof(S)) % 16 == 0 && al16(f.Jin) && al16(f.Hrin) && al16(f.HZin) && al16(f.Jold) && al16(f.Hv) &&
+           al16(f.Jout) && al16(f.Hrout) && al16(f.HZout);
+}
+
+template <typename S, typename R, int M, int G, typename RC>
 static void freq_launch(const void *args, int nitems, cudaStream_t st) {
     FreqArgs<S> fa = *static_cast<const FreqArgs<S> *>(args);
-    // every row of every cloud starts on a 16-byte boundary when the buffers do and a row
-    // (n_nu elements) is a multiple of 16 bytes: cloud offsets are sums of whole rows
-    fa.vec16 = LaneRow<S, M>::ok && fa.nnu % M == 0 && (fa.nnu * sizeof(S)) % 16 == 0 && al16(fa.Jin) &&
-               al16(fa.Hrin) && al16(fa.HZin) && al16(fa.Jold) && al16(fa.Hv) && al16(fa.Jout) && al16(fa.Hrout) &&
-               al16(fa.HZout);
-    const int ns = fa.Jold == fa.Jin ? 4 : 5;
-    const size_t sm = sizeof(double) * freq_smem_doubles<M>(FREQ_THREADS / 32, fa.solver == SOLVER_THOMAS, ns);
+    fa.vec16 = rows_vec16(fa);
+    const size_t sm = sizeof(double) * freq_smem_doubles<M, G>(FREQ_THREADS / 32, fa.solver == SOLVER_THOMAS,
+                                                               freq_ns<G>(fa.Jold == fa.Jin));
     static bool attr = false;
     if (!attr) {
-        const size_t smax = sizeof(double) * freq_smem_doubles<M>(FREQ_THREADS / 32, true, 5);
-        cudaFuncSetAttribute(k_freq<S, R, M, RC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
+        const size_t smax = sizeof(double) * freq_smem_doubles<M, G>(FREQ_THREADS / 32, true, 5);
+        cudaFuncSetAttribute(k_freq<S, R, M, G, RC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
         attr = true;
     }
-    k_freq<S, R, M, RC><<<nitems, FREQ_THREADS, sm, st>>>(fa);
+    k_freq<S, R, M, G, RC><<<nitems, FREQ_THREADS, sm, st>>>(fa);
 }
+
+// How a cell's bins lie across lanes: groups of G lanes, M bins to a lane (see freq_item).
+static int freq_shape(int nnu) {
+    return nnu <= 16 ? 0 : nnu <= 32 ? 1 : nnu <= 48 ? 2 : nnu <= 64 ? 3 : nnu <= 128 ? 4 : 5;
+}
+int freq_cells_per_warp(int nnu) { return nnu <= 48 ? 2 : 1; }
 
 void launch_freq(int prec, const void *args, int nnu, int nitems, cudaStream_t st) {
     if (nitems <= 0) return;
-    int M = bins_per_lane(nnu);
-#define LYD_FQ(S_, R_, RC_)                                              \
-    switch (M) {                                                         \
-    case 1: freq_launch<S_, R_, 1, RC_>(args, nitems, st); break;        \
-    case 2: freq_launch<S_, R_, 2, RC_>(args, nitems, st); break;        \
-    case 4: freq_launch<S_, R_, 4, RC_>(args, nitems, st); break;        \
-    default: freq_launch<S_, R_, 8, RC_>(args, nitems, st); break;       \
+#define LYD_FQ(S_, R_, RC_)                                                  \
+    switch (freq_shape(nnu)) {                                               \
+    case 0: freq_launch<S_, R_, 1, 16, RC_>(args, nitems, st); break;        \
+    case 1: freq_launch<S_, R_, 2, 16, RC_>(args, nitems, st); break;        \
+    case 2: freq_launch<S_, R_, 3, 16, RC_>(args, nitems, st); break;        \
+    case 3: freq_launch<S_, R_, 2, 32, RC_>(args, nitems, st); break;        \
+    case 4: freq_launch<S_, R_, 4, 32, RC_>(args, nitems, st); break;        \
+    default: freq_launch<S_, R_, 8, 32, RC_>(args, nitems, st); break;       \
     }
     // the mixed variant keeps the frequency step in FP64 (its state, factors and solve need
     // it) except the closure that sets the Doppler velocity (see k_freq)
@@ -2245,15 +2341,13 @@ void launch_find_active(int sprec, const void *J, int nnu, const double *dnu, co
 #undef LYD_ACT
 }
 
-template <typename S, typename RA, typename RF, typename RC, int FLUX, int M>
+template <typename S, typename RA, typename RF, typename RC, int FLUX, int M, int G>
 static cudaError_t persist_launch(const void *adv, const void *freq, const RedArgs &red, int nitems,
                                   unsigned *bar, long long polls, int *err, cudaStream_t st) {
     PersistArgs<S> p;
     p.adv = *static_cast<const AdvArgs<S> *>(adv);
     p.freq = *static_cast<const FreqArgs<S> *>(freq);
-    p.freq.vec16 = LaneRow<S, M>::ok && p.freq.nnu % M == 0 && (p.freq.nnu * sizeof(S)) % 16 == 0 && al16(p.freq.Jin) &&
-                   al16(p.freq.Hrin) && al16(p.freq.HZin) && al16(p.freq.Jold) && al16(p.freq.Hv) &&
-                   al16(p.freq.Jout) && al16(p.freq.Hrout) && al16(p.freq.HZout);
+    p.freq.vec16 = rows_vec16(p.freq);
     p.red = red;
     if (!red.colsum) p.red.cnt = nullptr;
     const int ncols = red.nnu + kExtraCols, rw = PT / 32;
@@ -2263,10 +2357,10 @@ static cudaError_t persist_launch(const void *adv, const void *freq, const RedAr
     p.bar = bar;
     p.polls = polls;
     p.err = err;
-    auto kern = k_step_persistent<S, RA, RF, RC, FLUX, M>;
+    auto kern = k_step_persistent<S, RA, RF, RC, FLUX, M, G>;
     const size_t sa = adv_pack_smem<S, RA>();
-    const size_t sf = sizeof(double) * freq_smem_doubles<M>(FREQ_THREADS / 32, p.freq.solver == SOLVER_THOMAS,
-                                                            p.freq.Jold == p.freq.Jin ? 4 : 5);
+    const size_t sf = sizeof(double) * freq_smem_doubles<M, G>(FREQ_THREADS / 32, p.freq.solver == SOLVER_THOMAS,
+                                                               freq_ns<G>(p.freq.Jold == p.freq.Jin));
     const size_t sm = sa > sf ? sa : sf;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
@@ -2293,16 +2387,17 @@ static cudaError_t persist_launch(const void *adv, const void *freq, const RedAr
 
 cudaError_t launch_persistent(int prec, int flux, const void *adv, const void *freq, const RedArgs &red, int nnu,
                               int nitems, unsigned *bar, long long polls, int *err, cudaStream_t st) {
-    const int M = bins_per_lane(nnu);
-#define LYD_PS1(S_, RA_, RF_, RC_, M_)                                                                     \
-    return flux == 0 ? persist_launch<S_, RA_, RF_, RC_, 0, M_>(adv, freq, red, nitems, bar, polls, err, st) \
-                     : persist_launch<S_, RA_, RF_, RC_, 1, M_>(adv, freq, red, nitems, bar, polls, err, st);
+#define LYD_PS1(S_, RA_, RF_, RC_, M_, G_)                                                                 \
+    return flux == 0 ? persist_launch<S_, RA_, RF_, RC_, 0, M_, G_>(adv, freq, red, nitems, bar, polls, err, st) \
+                     : persist_launch<S_, RA_, RF_, RC_, 1, M_, G_>(adv, freq, red, nitems, bar, polls, err, st);
 #define LYD_PS(S_, RA_, RF_, RC_)                                                                         \
-    switch (M) {                                                                                          \
-    case 1: LYD_PS1(S_, RA_, RF_, RC_, 1)                                                                 \
-    case 2: LYD_PS1(S_, RA_, RF_, RC_, 2)                                                                 \
-    case 4: LYD_PS1(S_, RA_, RF_, RC_, 4)                                                                 \
-    default: LYD_PS1(S_, RA_, RF_, RC_, 8)                                                                \
+    switch (freq_shape(nnu)) {                                                                            \
+    case 0: LYD_PS1(S_, RA_, RF_, RC_, 1, 16)                                                             \
+    case 1: LYD_PS1(S_, RA_, RF_, RC_, 2, 16)                                                             \
+    case 2: LYD_PS1(S_, RA_, RF_, RC_, 3, 16)                                                             \
+    case 3: LYD_PS1(S_, RA_, RF_, RC_, 2, 32)                                                             \
+    case 4: LYD_PS1(S_, RA_, RF_, RC_, 4, 32)                                                             \
+    default: LYD_PS1(S_, RA_, RF_, RC_, 8, 32)                                                            \
     }
     // the arithmetic of each phase as in launch_advect and launch_freq
     if (prec == PREC_K_FP32) {
