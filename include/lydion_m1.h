@@ -210,7 +210,7 @@ int  lyd_f_esc(lyd_ctx *ctx, double L_allspace, int32_t bc_z_bot, double *f_esc)
 /* Reset_Delta_rho_u!, src/ConstantsAndFunctions.jl:809-816 */
 int  lyd_reset_dru(lyd_ctx *ctx);
 /* n_steps iterations of the static-cloud driver loop, src/StaticCloudTest.jl:357-392, as
- * fused kernels replayed from a CUDA graph. diag_hist (may be NULL) receives one lyd_diag
+ * fused kernels, chained from step to step. diag_hist (may be NULL) receives one lyd_diag
  * per step; with diag_hist == NULL the call returns once the steps are enqueued and any
  * error is reported by the next synchronising call. */
 int  lyd_static_steps(lyd_ctx *ctx, const lyd_step_params *p, lyd_diag *diag_hist);
@@ -238,8 +238,8 @@ int  lyd_get_timing(lyd_ctx *ctx, double ms[3]);
 /* A context may hold many independent clouds of different (n_r, n_z) sharing one frequency
  * grid and one configuration: the batched form of the static-cloud run (512 clouds of
  * uneven size advancing together). Every step kernel covers all clouds in one launch (a work
- * list of per-cloud tiles), each cloud with its own time step and boundary conditions, and
- * the step is replayed from one CUDA graph. lyd_create is a batch of one cloud.
+ * list of per-cloud tiles), each cloud with its own time step and boundary conditions.
+ * lyd_create is a batch of one cloud.
  *
  * On a context of several clouds: lyd_upload / lyd_download move every cloud's values,
  * concatenated cloud after cloud; lyd_find_active_bins writes n_clouds entries to each of

@@ -4,8 +4,7 @@
 // A context holds a batch of independent clouds (one cloud for lyd_create). Every field of
 // every cloud lives in one concatenated device array per field, cloud after cloud; the
 // per-cloud offsets, sizes, boundary conditions and time step are CloudDesc records in
-// device memory that the kernels read, so changing a time step is a 100-byte copy and the
-// captured step graph stays valid.
+// device memory that the kernels read, so changing a time step is a 100-byte copy.
 //
 // Device state. J, H_r, H_Z live in two buffer sets. `cur` holds the current values; the
 // other set holds J_old, H_r_old, H_Z_old unless `old_alias` is set, in which case the old
@@ -106,7 +105,7 @@ struct lyd_ctx {
     double *small = nullptr;           // device scratch (512 doubles)
     cudaGraphExec_t gexec = nullptr;
     int gkey_cur = -1;
-    long long gkey_polls = 0;          // 0: the three-launch step graph; else the persistent step's poll limit
+    long long gkey_polls = 0;          // poll limit of the captured persistent step
     // the host-state step (lyd_static_step_host): the state as uploaded, the window check, the
     // work lists grouped by row chunk, its copy streams and events
     double *hin = nullptr;             // [3][n3] J, H_r, H_Z as uploaded
@@ -1174,6 +1173,8 @@ static int enqueue_step(lyd_ctx *c, bool timed, double *tape = nullptr, const S 
     RedArgs ra = red_args(c, PART_ACTIVE | PART_DIAG);
     ra.diag = c->hist; ra.step_counter = c->step_ctr; ra.done = c->step_ctr + 1; ra.hist_capacity = c->hist_cap;
     ra.kwin_copy = win_next;
+    // the three kernels, and the next step's after them, overlap their ends and beginnings
+    aa.chained = fa.chained = ra.chained = !timed;
     const int prec = c->prec;
     if (polls > 0) {
         if (timed) cudaEventRecord(c->ev[0], c->st);
@@ -1243,14 +1244,18 @@ static int run_steps(lyd_ctx *c, int n_steps, lyd_diag *hist_out, long long poll
             }
         }
         for (int q = 0; q < 3; q++) c->ms[q] = acc[q];
-    } else if (polls > 0 && c->persist_graph < 0) {
-        // the runtime refused to capture the cooperative launch: one launch per step
+    } else if (polls == 0 || c->persist_graph < 0) {
+        // Three launches per step, chained from step to step (see pdl_wait). A graph of one step cannot
+        // overlap the next one's: 24 x 20 x 16 29.0 us per step from the graph, 26.3 launched; 64^2 x 64 45.2
+        // and 43.8; 256^2 x 64 339.4 and 337.0; a graph of four steps is no faster than launching them, and
+        // has to be made first. (Persistent step: the runtime refused to capture the cooperative launch.)
         for (int n = 0; n < n_steps; n++) {
             int r = c->sprec == 0 ? enqueue_step<double>(c, false, nullptr, nullptr, nullptr, nullptr, true, nullptr, polls)
                                   : enqueue_step<float>(c, false, nullptr, nullptr, nullptr, nullptr, true, nullptr, polls);
             if (r != LYD_OK) return r;
         }
     } else {
+        // the persistent step from a captured graph
         if (!c->gexec || c->gkey_cur != c->cur || c->gkey_polls != polls) {
             drop_graph(c);
             cudaGraph_t g = nullptr;
@@ -1263,17 +1268,15 @@ static int run_steps(lyd_ctx *c, int n_steps, lyd_diag *hist_out, long long poll
                 if (e != cudaSuccess) c->gexec = nullptr;
             }
             if (g) cudaGraphDestroy(g);
-            if (polls > 0 && (r != LYD_OK || e != cudaSuccess)) {
+            if (r != LYD_OK || e != cudaSuccess) {
                 // capture of the cooperative launch refused: launch it directly from now on
                 cudaGetLastError();
                 c->persist_graph = -1;
                 return run_steps(c, n_steps, hist_out, polls);
             }
-            if (r != LYD_OK) return r;
-            if (e != cudaSuccess) return fail(c, LYD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
             c->gkey_cur = c->cur;
             c->gkey_polls = polls;
-            if (polls > 0) c->persist_graph = 1;
+            c->persist_graph = 1;
         }
         for (int n = 0; n < n_steps; n++) LYD_CU(c, cudaGraphLaunch(c->gexec, c->st));
     }

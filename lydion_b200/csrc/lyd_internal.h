@@ -73,6 +73,7 @@ struct AdvArgs {
     const unsigned char *tmaps;  // tensor maps of the input J, H_r, H_Z, [cloud][3] of
                                  // kTensorMapBytes each in device memory, or nullptr: packed tiles
     int *err;                    // device error bits (ERRB_TIMEOUT)
+    int chained;                 // the launch overlaps the end of the kernel before it (all three: see pdl_wait)
 };
 
 // Emission/absorption + frequency step + flux correction (+ partial reductions).
@@ -105,6 +106,7 @@ struct FreqArgs {
     int nnu;
     int solver;                  // SOLVER_*
     int vec16;                   // set by the launcher: rows move as whole 16-byte words
+    int chained;
     int item0, nitems_all;       // a launch over items item0 .. of a list of nitems_all (0: the grid's)
 };
 
@@ -131,6 +133,7 @@ struct RedArgs {
     // counters (zero between launches). Both null: one CTA per cloud sums every column.
     double *colsum;
     int *cnt;
+    int chained;
     int *kwin_copy;              // optional second destination of the decided window [cloud][2]
 };
 

@@ -24,6 +24,30 @@ namespace lyd {
 
 constexpr int FREQ_THREADS = 256;
 
+// The step's kernels follow one another with programmatic dependent launches: each lets the next one's
+// CTAs in as soon as all of its own have started (they fill the slots its last wave leaves empty and do
+// what needs nothing from it), and every CTA waits for the kernels before it to have finished, and
+// their writes to be visible, before it reads or writes anything of theirs. Every CTA of every kernel
+// of the chain waits, so a kernel that has finished vouches for all before it. Launched without the
+// attribute the two do nothing.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename K, typename A>
+static void launch_chained(bool chained, K kern, int grid, int block, size_t sm, cudaStream_t st, const A &a) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, a);
+}
+
 // Per-CTA view of one cloud of a batch.
 struct View {
     long long o3, oc, orf, ozf;
@@ -647,6 +671,8 @@ __device__ __forceinline__ void advect_tile_tma(const AdvArgs<S> &a, int tile, u
 template <typename S, typename R, int FLUX, int MINB>
 __global__ void __launch_bounds__(MTHREADS, MINB) k_advect_tma(AdvArgs<S> a) {
     extern __shared__ __align__(128) unsigned char adv_smem[];
+    pdl_trigger();
+    pdl_wait();
     advect_tile_tma<S, R, FLUX>(a, blockIdx.x, adv_smem);
 }
 
@@ -1076,6 +1102,8 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
 template <typename S, typename R, int FLUX, int MINB>
 __global__ void __launch_bounds__(PT, MINB) k_advect(AdvArgs<S> a) {
     extern __shared__ __align__(128) unsigned char adv_smem[];
+    pdl_trigger();
+    pdl_wait();                                             // (the tile's very shape is the last step's decision)
     advect_tile<S, R, FLUX>(a, blockIdx.x, adv_smem);
 }
 
@@ -1468,6 +1496,7 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
         kc[KC_DNU * NP + t] = in ? a.dnu[t] : 0.0;
     }
     if (threadIdx.x < 32) kc[KC_EXP2 * NP + threadIdx.x] = kExp2Tab[threadIdx.x];
+    pdl_wait();                               // (the constants above are none of the step's own)
     __syncthreads();
 
     const int4 it = a.items[item];
@@ -1977,6 +2006,7 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
 template <typename S, typename R, int M, int G, typename RC = R>
 __global__ void __launch_bounds__(FREQ_THREADS, M <= 4 ? 2 : 1) k_freq(FreqArgs<S> a) {
     extern __shared__ __align__(16) double fsm[];
+    pdl_trigger();
     freq_item<S, R, M, G, RC>(a, a.item0 + (int)blockIdx.x, a.nitems_all ? a.nitems_all : (int)gridDim.x, fsm,
                            blockDim.x >> 5);
 }
@@ -2050,7 +2080,14 @@ __device__ __forceinline__ void reduce_block(const RedArgs &a, int vb) {
         double s = 0.0;
         if (need) {
             const double *p = pbase + (size_t)cc * a.nblocks;
-            for (int b = lane; b < npb; b += 32) s += p[b];
+            // (eight loads in flight, added in order)
+            for (int b0 = lane; b0 < npb; b0 += 256) {
+                double v[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) v[q] = b0 + 32 * q < npb ? __ldcg(p + b0 + 32 * q) : 0.0;
+#pragma unroll
+                for (int q = 0; q < 8; q++) s += v[q];
+            }
         }
         s = warp_sum(s);
         if (lane == 0) {
@@ -2070,28 +2107,34 @@ __device__ __forceinline__ void reduce_block(const RedArgs &a, int vb) {
         if (threadIdx.x == 0) a.cnt[cloud] = 0;
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
+    // the decisions: one warp looks the bins over, its first lane writes
+    if (warp != 0) return;
     int *kw = a.kwin + 2 * cloud;
-    int used_kmin = kw[0], used_kmax = kw[1];
+    const int used_kmin = kw[0], used_kmax = kw[1];
+    __syncwarp();
     if (a.parts & PART_ACTIVE) {
         double Etot = col[a.nnu];
         int kmin = a.nnu - 1, kmax = 0;
-        for (int k = 0; k < a.nnu; k++) {
+        for (int k = lane; k < a.nnu; k += 32) {
             if (col[k] > kEpsActive * Etot) {
                 kmin = k < kmin ? k : kmin;
                 kmax = k > kmax ? k : kmax;
             }
         }
+        kmin = __reduce_min_sync(0xffffffffu, kmin);
+        kmax = __reduce_max_sync(0xffffffffu, kmax);
         kmax = kmax > a.kcore_max ? kmax : a.kcore_max;
         kmin = kmin < a.kcore_min ? kmin : a.kcore_min;
-        kw[0] = kmin;
-        kw[1] = kmax;
-        if (a.kwin_copy) {
-            a.kwin_copy[2 * cloud] = kmin;
-            a.kwin_copy[2 * cloud + 1] = kmax;
+        if (lane == 0) {
+            kw[0] = kmin;
+            kw[1] = kmax;
+            if (a.kwin_copy) {
+                a.kwin_copy[2 * cloud] = kmin;
+                a.kwin_copy[2 * cloud + 1] = kmax;
+            }
         }
     }
-    if (a.parts & PART_DIAG) {
+    if (lane == 0 && (a.parts & PART_DIAG)) {
         double MF = col[a.nnu + 1], net = col[a.nnu + 2], outw = col[a.nnu + 3];
         double L = col[a.nnu + 4];
         if (L > 0.0) {
@@ -2120,7 +2163,11 @@ __device__ __forceinline__ void reduce_block(const RedArgs &a, int vb) {
     }
 }
 
-__global__ void __launch_bounds__(1024) k_reduce(RedArgs a) { reduce_block(a, blockIdx.x); }
+__global__ void __launch_bounds__(1024) k_reduce(RedArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    reduce_block(a, blockIdx.x);
+}
 
 // ---- the persistent step: one cooperative launch runs the three phases -----------------------
 //
@@ -2209,7 +2256,7 @@ static void adv_launch(const void *args, cudaStream_t st) {
             cudaFuncSetAttribute(k_advect_tma<S, R, FLUX, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             attr_t = true;
         }
-        k_advect_tma<S, R, FLUX, MINB><<<a.ntiles, MTHREADS, sm, st>>>(a);
+        launch_chained(a.chained, k_advect_tma<S, R, FLUX, MINB>, a.ntiles, MTHREADS, sm, st, a);
         return;
     }
     constexpr size_t sm = adv_pack_smem<S, R>();
@@ -2217,7 +2264,7 @@ static void adv_launch(const void *args, cudaStream_t st) {
         cudaFuncSetAttribute(k_advect<S, R, FLUX, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         attr = true;
     }
-    k_advect<S, R, FLUX, MINB><<<a.ntiles, PT, sm, st>>>(a);
+    launch_chained(a.chained, k_advect<S, R, FLUX, MINB>, a.ntiles, PT, sm, st, a);
 }
 
 template <typename S, typename R, int FLUX>
@@ -2286,7 +2333,7 @@ static void freq_launch(const void *args, int nitems, cudaStream_t st) {
         cudaFuncSetAttribute(k_freq<S, R, M, G, RC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
         attr = true;
     }
-    k_freq<S, R, M, G, RC><<<nitems, FREQ_THREADS, sm, st>>>(fa);
+    launch_chained(fa.chained, k_freq<S, R, M, G, RC>, nitems, FREQ_THREADS, sm, st, fa);
 }
 
 // How a cell's bins lie across lanes: groups of G lanes, M bins to a lane (see freq_item).
@@ -2415,11 +2462,11 @@ void launch_reduce(const RedArgs &a, cudaStream_t st) {
     if (a.nclouds <= 0) return;
     if (a.cnt && a.colsum) {
         const int nchunks = (a.nnu + kExtraCols + 7) / 8;
-        k_reduce<<<a.nclouds * nchunks, 256, 0, st>>>(a);
+        launch_chained(a.chained, k_reduce, a.nclouds * nchunks, 256, 0, st, a);
     } else {
         RedArgs b = a;
         b.cnt = nullptr;
-        k_reduce<<<a.nclouds, 1024, 0, st>>>(b);
+        launch_chained(a.chained, k_reduce, a.nclouds, 1024, 0, st, b);
     }
 }
 
