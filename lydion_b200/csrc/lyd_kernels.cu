@@ -793,10 +793,10 @@ __device__ __forceinline__ CellSrc cell_src(const View &v, int col, int row) {
 }
 template <typename S>
 __device__ __forceinline__ S bc_rule(S h, int rule) {
+    if (rule == 0) return h;                  // (all but the ghosts: one branch past the rules)
     if (rule == 1) return -h;
     if (rule == 2) return h < S(0) ? h : S(0);
-    if (rule == 3) return h > S(0) ? h : S(0);
-    return h;
+    return h > S(0) ? h : S(0);
 }
 
 // Every staged input a row ahead: when the landing rows fit, i.e. when S and R agree.
@@ -850,19 +850,35 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
     const int kbeg = kmin + kb * nbk;
     const R jeps = R(a.jeps);
 
-    // bins outside the window pass through: the rows of the tile in turn over its chunks
-    if (nact < a.nnu) {
-        const int nin = a.nnu - nact, n = ncol * nin;
-        for (int j = j0 + kb; j < j1; j += pk.nb) {
-            const long long row = v.o3 + (long long)a.nnu * (i0 + (long long)v.nr * j);
-            for (int e = t; e < n; e += PT) {
-                const int c = e / nin, m = e - c * nin;
-                const long long x = row + (long long)a.nnu * c + (m < kmin ? m : m + nact);
-                a.Jo[x] = a.J[x]; a.Hro[x] = a.Hr[x]; a.HZo[x] = a.HZ[x];
-            }
+    // Bins outside the window pass through, the rows of the tile in turn over its chunks. A thread's first
+    // two are loaded here and stored once the prologue's own loads have gone out.
+    const int nin = a.nnu - nact, prow = ncol * nin;
+    const int npass = prow * ((j1 - j0 - kb + pk.nb - 1) / pk.nb);
+    auto pass_at = [&](int e) {
+        const int q = e / prow, f = e - q * prow, cc = f / nin, m = f - cc * nin;
+        return v.o3 + (long long)a.nnu * (i0 + cc + (long long)v.nr * (j0 + kb + q * pk.nb)) + (m < kmin ? m : m + nact);
+    };
+    Cell<S> pv[2];
+    long long px[2] = {-1, -1};
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+        if (t + q * PT < npass) {
+            px[q] = pass_at(t + q * PT);
+            pv[q].J = a.J[px[q]]; pv[q].Hr = a.Hr[px[q]]; pv[q].HZ = a.HZ[px[q]];
         }
+    auto pass_rest = [&]() {
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+            if (px[q] >= 0) { a.Jo[px[q]] = pv[q].J; a.Hro[px[q]] = pv[q].Hr; a.HZo[px[q]] = pv[q].HZ; }
+        for (int e = t + 2 * PT; e < npass; e += PT) {
+            const long long x = pass_at(e);
+            a.Jo[x] = a.J[x]; a.Hro[x] = a.Hr[x]; a.HZo[x] = a.HZ[x];
+        }
+    };
+    if (nact == 0 || kbeg > kmax) {
+        pass_rest();
+        return;
     }
-    if (nact == 0 || kbeg > kmax) return;
 
     // this thread's item: column i0 + c (c = ncol: the column right of the tile, for its r face)
     const int c = t / nbk, k = kbeg + (t - c * nbk), col = i0 + c;
@@ -1030,6 +1046,7 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
         if (f <= v.nr) riv[e] = __ldg(a.rint + v.orint + 5 * f + e % 5);
     }
     if (t < PNC && i0 + t < v.nr) irc[t] = __ldg(a.inv_r_cell + v.ocol + i0 + t);
+    pass_rest();
     cp_async_wait<0>();
     __syncthreads();
     auto zface = [&](int f, const double *ivz, double us, R *F) {

@@ -61,3 +61,27 @@ def test_tile_heights_change_nothing(oracle_mod, rows):
         np.testing.assert_array_equal(a.download(f), b.download(f))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("staging", [0, 2])
+def test_repeated_band_advections_keep_the_old_state(oracle_mod, staging):
+    """AdvectJandH! again and again from a J_old that is not J: the buffers trade places, J_old stays, and
+    a fused step afterwards (with tensor maps or without) starts from the advected state."""
+    cl = W.small_cloud(nr=17, nz=11, n_nu=24, x_max=200.0)
+    st, ctx = matched_pair(oracle_mod, cl, seed=13)
+    ctx.set_tuning(8, 0, 0, 0, staging)
+    ctdt = cl.c_tilde * cl.dt
+    old = 0.5 * st.J
+    st.J_old[...] = old
+    ctx.upload("J_old", old)
+    for n in range(4):
+        st.advect_jh(ctdt, 0, 23, n == 3)
+        ctx.advect_jh(ctdt, 0, 23, n == 3, cl.bc_r_right, cl.bc_z_bot, cl.bc_z_top)
+        for f in ("J", "H_r", "H_Z", "J_old"):
+            assert norm_err(ctx.download(f), getattr(st, f)) < 4e-12, (n, f)
+    h = ctx.static_steps(2, cl.c_tilde, cl.dt, cl.z_center, cl.bc_r_right, cl.bc_z_bot, cl.bc_z_top)
+    d = st.run(2)
+    np.testing.assert_array_equal(h[:, 5:7], d[:, 5:7])
+    for f in ("J", "H_r", "H_Z"):
+        assert norm_err(ctx.download(f), getattr(st, f)) < 1e-9, f
+    ctx.close()
