@@ -37,6 +37,8 @@ constexpr int kLutN = 200001;        // src/FastInterpolations.jl:175-176
 constexpr double kLutXmax = 1000.0;
 constexpr int kTileCols = 8;         // columns per advection tile (the kernel's MT)
 constexpr int kDefaultRows = 16;
+constexpr int kGraphSteps = 4;       // steps of the captured graph
+constexpr int kGraphAfter = 64;      // steps of a context before one is captured
 
 // per-cloud "was provided" bits: per-cell fields use their index (field - LYD_F_ALPHA)
 enum { CF_ALPHA = 0, CF_ALPHA_C, CF_ALPHA_CF, CF_PD, CF_JS, CF_T, CF_DUR_DR, CF_DUR_DZ, CF_DUZ_DR, CF_DUZ_DZ,
@@ -105,7 +107,8 @@ struct lyd_ctx {
     double *small = nullptr;           // device scratch (512 doubles)
     cudaGraphExec_t gexec = nullptr;
     int gkey_cur = -1;
-    long long gkey_polls = 0;          // poll limit of the captured persistent step
+    long long gkey_polls = 0;          // 0: a graph of kGraphSteps steps; else the persistent step's poll limit
+    int steps_run = 0;                 // fused steps so far, up to kGraphAfter
     // the host-state step (lyd_static_step_host): the state as uploaded, the window check, the
     // work lists grouped by row chunk, its copy streams and events
     double *hin = nullptr;             // [3][n3] J, H_r, H_Z as uploaded
@@ -1244,41 +1247,49 @@ static int run_steps(lyd_ctx *c, int n_steps, lyd_diag *hist_out, long long poll
             }
         }
         for (int q = 0; q < 3; q++) c->ms[q] = acc[q];
-    } else if (polls == 0 || c->persist_graph < 0) {
-        // Three launches per step, chained from step to step (see pdl_wait). A graph of one step cannot
-        // overlap the next one's: 24 x 20 x 16 29.0 us per step from the graph, 26.3 launched; 64^2 x 64 45.2
-        // and 43.8; 256^2 x 64 339.4 and 337.0; a graph of four steps is no faster than launching them, and
-        // has to be made first. (Persistent step: the runtime refused to capture the cooperative launch.)
-        for (int n = 0; n < n_steps; n++) {
-            int r = c->sprec == 0 ? enqueue_step<double>(c, false, nullptr, nullptr, nullptr, nullptr, true, nullptr, polls)
-                                  : enqueue_step<float>(c, false, nullptr, nullptr, nullptr, nullptr, true, nullptr, polls);
-            if (r != LYD_OK) return r;
-        }
     } else {
-        // the persistent step from a captured graph
-        if (!c->gexec || c->gkey_cur != c->cur || c->gkey_polls != polls) {
+        auto steps = [&](int n) -> int {
+            for (int q = 0; q < n; q++)
+                LYD_TRY(c->sprec == 0
+                            ? enqueue_step<double>(c, false, nullptr, nullptr, nullptr, nullptr, true, nullptr, polls)
+                            : enqueue_step<float>(c, false, nullptr, nullptr, nullptr, nullptr, true, nullptr, polls));
+            return LYD_OK;
+        };
+        // Steps are launched one by one, each kernel chained to the one before, until the context has run
+        // enough of them to pay for a captured graph of kGraphSteps, which a slow host cannot hold up
+        // (24 x 20 x 16: launched 26 us per step, 29 on a slower box; the graph 26; a graph of one step, which
+        // cannot overlap the next one's first kernel, 29). The persistent step has one launch to capture.
+        const int gs = polls > 0 ? 1 : kGraphSteps;
+        const bool graph = polls > 0 ? c->persist_graph >= 0
+                                     : n_steps >= gs && (c->gexec || c->steps_run + n_steps >= kGraphAfter);
+        if (graph && (!c->gexec || c->gkey_cur != c->cur || c->gkey_polls != polls)) {
             drop_graph(c);
             cudaGraph_t g = nullptr;
             LYD_CU(c, cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-            int r = c->sprec == 0 ? enqueue_step<double>(c, false, nullptr, nullptr, nullptr, nullptr, true, nullptr, polls)
-                                  : enqueue_step<float>(c, false, nullptr, nullptr, nullptr, nullptr, true, nullptr, polls);
+            const int r = steps(gs);
             cudaError_t e = cudaStreamEndCapture(c->st, &g);
             if (e == cudaSuccess && r == LYD_OK) {
                 e = cudaGraphInstantiate(&c->gexec, g, 0);
                 if (e != cudaSuccess) c->gexec = nullptr;
             }
             if (g) cudaGraphDestroy(g);
-            if (r != LYD_OK || e != cudaSuccess) {
+            if (polls > 0 && (r != LYD_OK || e != cudaSuccess)) {
                 // capture of the cooperative launch refused: launch it directly from now on
                 cudaGetLastError();
                 c->persist_graph = -1;
                 return run_steps(c, n_steps, hist_out, polls);
             }
+            if (r != LYD_OK) return r;
+            if (e != cudaSuccess) return fail(c, LYD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
             c->gkey_cur = c->cur;
             c->gkey_polls = polls;
-            c->persist_graph = 1;
+            if (polls > 0) c->persist_graph = 1;
         }
-        for (int n = 0; n < n_steps; n++) LYD_CU(c, cudaGraphLaunch(c->gexec, c->st));
+        int n = 0;
+        if (graph)
+            for (; n + gs <= n_steps; n += gs) LYD_CU(c, cudaGraphLaunch(c->gexec, c->st));
+        LYD_TRY(steps(n_steps - n));
+        c->steps_run = std::min(c->steps_run + n_steps, kGraphAfter);
     }
     c->old_alias = true;
     c->active_valid = true;
