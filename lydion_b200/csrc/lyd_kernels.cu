@@ -1,17 +1,17 @@
 // lyd_kernels.cu -- the hot kernels of the Lyman-alpha M1 step on sm_100a.
 //
 //  k_advect   AdvectJandH_Cylindrical! (src/AdvectJandH.jl:526-1390) as ONE kernel. A CTA owns a
-//             tile of 8 columns (r) x `rows` rows (Z) x 32 bins (one bin per lane, k innermost,
-//             so every warp load is a contiguous 256 B / 128 B run) of one cloud and marches up
-//             the tile row by row. Face fluxes never touch HBM: the six face-flux arrays and the
-//             two K_phiphi arrays of the reference are replaced by shared memory and registers.
-//             Ghost cells of the four boundaries are produced on the fly from the boundary
-//             conditions.
+//             tile of columns (r) x rows (Z) x active bins of one cloud, its threads dealt out over
+//             (column, bin) pairs (k innermost, so a warp's loads are runs of neighbouring bins),
+//             and marches up the tile row by row. Face fluxes never touch HBM: the six face-flux
+//             arrays and the two K_phiphi arrays of the reference are replaced by shared memory and
+//             registers. Ghost cells of the four boundaries are produced on the fly from the
+//             boundary conditions. k_advect_tma is the form with bulk tensor copies.
 //  k_freq     LyaEmissionAbsorptionUpdate! + UpdateFreqFactors! + the per-cell tridiagonal solve
-//             + the flux correction of FrequencyUpdateJLya_AllCells!, fused per cell: one warp
-//             owns one cell's whole spectrum (M contiguous bins per lane), the k +- 1 couplings
-//             travel by warp shuffles, and the tridiagonal system is solved in FP64, by parallel
-//             cyclic reduction across the warp or by a lane-serial elimination. The epilogue
+//             + the flux correction of FrequencyUpdateJLya_AllCells!, fused per cell: a warp or half
+//             a warp owns one cell's whole spectrum (M contiguous bins per lane), the k +- 1 couplings
+//             travel by shuffles, and the tridiagonal system is solved in FP64, by parallel
+//             cyclic reduction across the lanes or by a lane-serial elimination. The epilogue
 //             accumulates the next step's FindActiveBins energies and the step diagnostics into
 //             per-CTA partials (fixed order, so results are run-to-run deterministic).
 //  k_reduce   one CTA per cloud sums that cloud's partials and derives kmin/kmax, M_F, L, f_esc.
@@ -205,19 +205,16 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const void *map, int x, i
         : "memory");
 }
 
-// ---- k_advect: one CTA = 8 columns (r) x `rows` rows (Z) x 32 bins, marching up in Z --------
+// ---- k_advect_tma: one CTA = 8 columns (r) x `rows` rows (Z) x 32 bins, marching up in Z ----
 //
 // A ring of four rows holds, for the 8 own columns and the 2 + 2 halo columns of each row, the
-// cell values every face needs: J, the reduced fluxes H/max(J, Jeps) (so the reciprocal of J is
-// taken once per cell, not once per face) and alpha_F (formed once per cell, not at each of the
-// four face sides that read it); a ring of three rows holds the state of the own columns for
-// the cell update. With FP64 arithmetic and per-lane staging the halo columns keep one row and
-// every staged input comes a row ahead by cp.async (PFR below): the tile (76 KB) runs at three
-// CTAs per SM. Warp w (0..7) owns
-// column i0+w; warp 8 stages the halo columns and computes the tile's rightmost r face. Per row: stage row j+2 -> sync -> every warp
-// computes the r face on its left (warp 8: the right edge) into shared memory and its Z face
-// j+1/2 into registers -> sync -> the cell update of row j uses the two r faces from shared
-// memory and the Z faces j-1/2 (carried from the previous row) and j+1/2.
+// cell values every face needs: J, the reduced fluxes H/max(J, Jeps) and alpha_F, each formed once
+// per cell; a ring of three rows holds the state of the own columns for the cell update. Warp w
+// (0..7) owns column i0+w; warp 8 stages the halo columns and computes the tile's rightmost r face.
+// Per row: stage row j+2 -> sync -> every warp computes the r face on its left (warp 8: the right
+// edge) into shared memory and its Z face j+1/2 into registers -> sync -> the cell update of row j
+// uses the two r faces from shared memory and the Z faces j-1/2 (carried from the previous row) and
+// j+1/2.
 constexpr int MT = 8;                  // own columns per CTA
 constexpr int MWARPS = MT + 1;
 constexpr int MTHREADS = 32 * MWARPS;
@@ -327,9 +324,9 @@ __device__ __forceinline__ CellF<R> staged(const R *p, int ps, R &aF) {
 
 // The face between staged cells pi and pp (pm, p2: the stencil's outer cells) with the PLM intervals
 // ivp and u* (src/AdvectJandH.jl:641-968, 978-1289).
-template <typename R, int FLUX, bool ZDIR>
+template <typename R, int FLUX, bool ZDIR, typename I>
 __device__ __forceinline__ void face_cells(const R *pm, const R *pi, const R *pp, const R *p2, int ps, R jeps,
-                                           double us, const double *ivp, R *F, R &kL, R &kR, R &JR, R &HZR) {
+                                           double us, const I *ivp, R *F, R &kL, R &kR, R &JR, R &HZR) {
     R d0, aFi, aFp, d3;
     const CellF<R> cm1 = staged<R>(pm, ps, d0);
     const CellF<R> ci = staged<R>(pi, ps, aFi);
@@ -347,9 +344,9 @@ __device__ __forceinline__ void face_z_cells(const R *pm, const R *pi, const R *
     face_cells<R, FLUX, true>(pm, pi, pp, p2, ps, jeps, us, ivp, F, kL, kR, JR, HZR);
 }
 // r face: K_phiphi of both sides too; on the axis (f = 0) the right side's is that of the axis.
-template <typename R, int FLUX>
+template <typename R, int FLUX, typename I>
 __device__ __forceinline__ void face_r_cells(const R *pm, const R *pi, const R *pp, const R *p2, int ps, bool axis,
-                                             R jeps, double us, const double *ivp, R *F, R &kL, R &kR) {
+                                             R jeps, double us, const I *ivp, R *F, R &kL, R &kR) {
     R JR, HZR;
     face_cells<R, FLUX, false>(pm, pi, pp, p2, ps, jeps, us, ivp, F, kL, kR, JR, HZR);
     if (axis) kR = k_phiphi_axis<R>(JR, HZR, jeps);
@@ -694,8 +691,9 @@ __global__ void __launch_bounds__(MTHREADS, MINB) k_advect_tma(AdvArgs<S> a) {
 // row: stage row j+2 -> barrier -> each thread computes the r face on its left into shared memory
 // and its Z face j+1/2 into registers -> barrier -> the cell update of row j from the two r faces in
 // shared memory and the Z faces j-1/2 (carried) and j+1/2. Faces never touch HBM. Every staged
-// input comes a row ahead by cp.async when S and R agree (FP64, FP32 storage); the mixed form has no
-// room for the landing rows at four CTAs per SM and loads its rows where it stages them.
+// input comes a row ahead by cp.async; the mixed form has no room for the halo's landing row at
+// four CTAs per SM and loads the halo where it stages it (with its own columns' rows loaded so too
+// 256^2 x 64 took 171 us, with those a row ahead 167).
 // Bound by dependent FP64 latency and instruction issue (24 warps per SM, 80 registers: FP64 pipe 36 %,
 // issue 60 %). Per launch, against tiles of 8 columns x 32 fixed bins with one warp per column and
 // branches in the faces: 256^2 x 64 with 53 active bins 262 -> 202 us (FP64), 187 -> 176 us (mixed),
@@ -799,7 +797,8 @@ __device__ __forceinline__ S bc_rule(S h, int rule) {
     return h > S(0) ? h : S(0);
 }
 
-// Every staged input a row ahead: when the landing rows fit, i.e. when S and R agree.
+// The own columns' rows land a row ahead in every form; the halo columns' when their landing row fits
+// beside it, i.e. when S and R agree.
 template <typename S, typename R> __host__ __device__ constexpr bool adv_ahead() { return sizeof(S) == sizeof(R); }
 // The halo's landing row fills the gaps of its staged row's planes (96 of 256 values) in FP64;
 // with FP32 it has its own space.
@@ -808,7 +807,7 @@ template <typename S, typename R>
 __host__ __device__ constexpr size_t adv_pack_smem() {
     size_t b = sizeof(R) * ((RING + 1) * 4 * PT + 5 * PT);           // ring, halo row, r faces
     b += sizeof(S) * RING * (adv_ahead<S, R>() ? 2 : 3) * PT;        // the state's rows
-    if (adv_ahead<S, R>()) b += sizeof(S) * 2 * PT;                  // landing row: J, H_voigt
+    b += sizeof(S) * (adv_ahead<S, R>() ? 2 : 1) * PT;               // landing row: J (mixed: lands in the state's), H_voigt
     if (adv_ahead<S, R>() && !adv_overlay<S, R>()) b += sizeof(S) * 4 * PHALO + sizeof(double) * 2 * PHALO;
     return b + sizeof(double) * (2 * PGEO + PNC * 5 + PNC);
 }
@@ -823,11 +822,12 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
     R *HB = A + RING * 4 * PT;                              // [4][PT]: the halo columns' current row
     R *Fr = HB + 4 * PT;                                    // [5][PT]
     S *Hs = reinterpret_cast<S *>(Fr + 5 * PT);             // [RING][HF][PT]: H_r, H_Z (, J) as stored
-    S *raw = Hs + RING * HF * PT;                           // AHEAD: [2][PT]: J, H_voigt (or alpha_F) landing
-    double *geo = reinterpret_cast<double *>(raw + (AHEAD ? 2 * PT : 0));   // [2][PGEO]
-    double *riv = geo + 2 * PGEO;                           // [PNC][5]: the r faces' intervals
-    double *irc = riv + PNC * 5;                            // [PNC]: <1/r>
-    double *hal = irc + PNC;                                // AHEAD, not OVER: [2][PHALO], then [4][PHALO] of S
+    S *raw = Hs + RING * HF * PT;                           // [HF == 3 ? 1 : 2][PT]: (J,) H_voigt (or alpha_F) landing
+    constexpr int RJ = HF == 3 ? 0 : PT;                    // where H_voigt lands in it
+    double *geo = reinterpret_cast<double *>(raw + RJ + PT);                // [2][PGEO]
+    double *irc = geo + 2 * PGEO;                           // [PNC]: <1/r>
+    R *riv = reinterpret_cast<R *>(irc + PNC);              // [PNC][5] of a double's room: the r faces' intervals
+    double *hal = irc + PNC + PNC * 5;                      // AHEAD, not OVER: [2][PHALO], then [4][PHALO] of S
     const int t = threadIdx.x;
     const int4 it = a.tiles[tile];                          // cloud, rows [y, w), place z in their list
     View v;
@@ -933,14 +933,14 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
     };
     long long xo = 0, xoa = 0, xh = 0, xha = 0;
     int orule = 0, hrule = 0;
-    if (AHEAD && item) col_base(col, k, xo, xoa, orule);
+    if (item) col_base(col, k, xo, xoa, orule);
     if (AHEAD && halo) col_base(hcol, hk, xh, xha, hrule);
     // rows the own columns stage: up to j1 + 1 and the second ghost row; no corner ghosts
     auto stages = [&](int r) { return item && r <= j1 + 1 && r <= v.nz + 1 && !(col >= v.nr && r >= v.nz); };
     auto issue_own = [&](int r) {
         if (stages(r)) {
             S *h = Hs + (r & (RING - 1)) * HF * PT + t;
-            copy_cell(xo, xoa, r, raw + t, h, h + PT, raw + PT + t);
+            copy_cell(xo, xoa, r, HF == 3 ? h + 2 * PT : raw + t, h, h + PT, raw + RJ + t);
         }
     };
     auto issue_halo = [&](int r) {
@@ -997,8 +997,8 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
                 case P_DUZDZ: gsrc = a.duZ_dZ + v.oc + gcol; break;
                 case P_UROR: gsrc = a.ur_over_r + v.oc + gcol; break;
                 case P_UZ: gsrc = a.u_Z_star + v.ozf + gcol + v.nr; break;       // face j + 1
-                case P_AL: gsrc = AHEAD && !a.aF ? a.alpha + v.oc + cc : nullptr; break;
-                default: gsrc = AHEAD && !a.aF && a.alpha_cF ? a.alpha_cF + v.oc + cc : nullptr; break;
+                case P_AL: gsrc = !a.aF ? a.alpha + v.oc + cc : nullptr; break;
+                default: gsrc = !a.aF && a.alpha_cF ? a.alpha_cF + v.oc + cc : nullptr; break;
             }
         }
     } else if (t < PGEO) {
@@ -1013,10 +1013,8 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
     };
 
     // ---- prologue: the first copies, then rows j0-2 .. j0+1 by loads ----
-    if constexpr (AHEAD) {
-        issue_own(j0 + 2);
-        issue_halo(j0);
-    }
+    issue_own(j0 + 2);
+    if constexpr (AHEAD) issue_halo(j0);
     geo_copy(j0);
     if (g_al) geo_copy(j0 - 1);
     cp_async_commit();
@@ -1043,7 +1041,7 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
     }
     for (int e = t; e < PNC * 5; e += PT) {
         const int f = i0 + e / 5;
-        if (f <= v.nr) riv[e] = __ldg(a.rint + v.orint + 5 * f + e % 5);
+        if (f <= v.nr) riv[e] = R(__ldg(a.rint + v.orint + 5 * f + e % 5));
     }
     if (t < PNC && i0 + t < v.nr) irc[t] = __ldg(a.inv_r_cell + v.ocol + i0 + t);
     pass_rest();
@@ -1060,26 +1058,24 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
     for (int j = j0; j < j1; j++) {
         const double *g = geo + (j & 1) * PGEO;
         // (A) row j+2 of the own columns and row j of the halo columns
+        const int r = j + 2;
+        if constexpr (!AHEAD) {
+            if (halo) stage_direct(hp, nullptr, hcol, j, hk);
+        }
+        if (stages(r)) {
+            const int zrule = r < v.nz ? 0 : (v.bzt == 0 ? 1 : 3);
+            const S *h = Hs + (r & (RING - 1)) * HF * PT + t;
+            const double *gp = geo + ((j - 1) & 1) * PGEO + c;
+            put(A + (r & (RING - 1)) * 4 * PT + t, HF == 3 ? h[2 * PT] : raw[t], bc_rule(h[0], orule),
+                bc_rule(h[PT], zrule), aF_of(raw[RJ + t], gp[P_AL * PNC], gp[P_ACF * PNC]));
+        }
+        issue_own(r + 1);
         if constexpr (AHEAD) {
-            const int r = j + 2;
-            if (stages(r)) {
-                const int zrule = r < v.nz ? 0 : (v.bzt == 0 ? 1 : 3);
-                const S *h = Hs + (r & (RING - 1)) * HF * PT + t;
-                const double *gp = geo + ((j - 1) & 1) * PGEO + c;
-                put(A + (r & (RING - 1)) * 4 * PT + t, raw[t], bc_rule(h[0], orule), bc_rule(h[PT], zrule),
-                    aF_of(raw[PT + t], gp[P_AL * PNC], gp[P_ACF * PNC]));
-            }
-            issue_own(r + 1);
             if (halo) {
                 put(hp, hraw[0], bc_rule(hraw[hps], hrule), hraw[2 * hps],
                     aF_of(hraw[3 * hps], *hal0, *hal1));
                 issue_halo(j + 1);
             }
-        } else {
-            const int r = j + 2;
-            if (stages(r))
-                stage_direct(A + (r & (RING - 1)) * 4 * PT + t, Hs + (r & (RING - 1)) * HF * PT + t, col, r, k);
-            if (halo) stage_direct(hp, nullptr, hcol, j, hk);
         }
         __syncthreads();
         geo_copy(j + 1);
