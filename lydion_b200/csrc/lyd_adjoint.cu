@@ -134,14 +134,14 @@ __device__ __forceinline__ void pcr(RowA<M> &R_, int lane) {
 
 // Two rows per lane: one cyclic-reduction step over the odd rows, PCR across the warp on the
 // even rows, back-substitution of the odd rows (the same scheme as the forward frequency
-// kernel's two-bins-per-lane solve).
-__device__ __forceinline__ void cr_pcr2(RowA<2> &R_, int lane) {
+// kernel's two-bins-per-lane solve: a lane without a neighbour gets its own values back, times a
+// coupling of zero).
+__device__ __forceinline__ void cr_pcr2(RowA<2> &R_) {
     const double ibo = rcp<double>(R_.b[1]);
     double a_om = __shfl_up_sync(0xffffffffu, R_.a[1], 1);
     double c_om = __shfl_up_sync(0xffffffffu, R_.c[1], 1);
     double d_om = __shfl_up_sync(0xffffffffu, R_.d[1], 1);
     double ib_om = __shfl_up_sync(0xffffffffu, ibo, 1);
-    if (lane == 0) { a_om = 0.0; c_om = 0.0; d_om = 0.0; ib_om = 1.0; }
     double al = -R_.a[0] * ib_om, ga = -R_.c[0] * ibo;
     double ea = al * a_om;
     double eb = R_.b[0] + al * c_om + ga * R_.a[1];
@@ -156,8 +156,6 @@ __device__ __forceinline__ void cr_pcr2(RowA<2> &R_, int lane) {
         double dm = __shfl_up_sync(0xffffffffu, nd, s);
         double ap = __shfl_down_sync(0xffffffffu, na, s), cp = __shfl_down_sync(0xffffffffu, nc, s);
         double dp = __shfl_down_sync(0xffffffffu, nd, s);
-        if (lane < s) { am = 0.0; cm = 0.0; dm = 0.0; }
-        if (lane + s > 31) { ap = 0.0; cp = 0.0; dp = 0.0; }
         eb = fma(-na, cm, fma(-nc, ap, 1.0));
         const double a2 = -na * am, c2 = -nc * cp;
         const double d2 = fma(-na, dm, fma(-nc, dp, nd));
@@ -167,15 +165,14 @@ __device__ __forceinline__ void cr_pcr2(RowA<2> &R_, int lane) {
         nd = d2 * ib;
     }
     const double xe = nd;
-    double xe2 = __shfl_down_sync(0xffffffffu, xe, 1);
-    if (lane == 31) xe2 = 0.0;
+    const double xe2 = __shfl_down_sync(0xffffffffu, xe, 1);
     R_.d[0] = xe;
     R_.d[1] = (R_.d[1] - R_.a[1] * xe - R_.c[1] * xe2) * ibo;
 }
 
 template <int M>
 __device__ __forceinline__ void solve(RowA<M> &R_, int lane) {
-    if constexpr (M == 2) cr_pcr2(reinterpret_cast<RowA<2> &>(R_), lane);
+    if constexpr (M == 2) cr_pcr2(reinterpret_cast<RowA<2> &>(R_));
     else pcr<M>(R_, lane);
 }
 

@@ -1236,17 +1236,18 @@ __device__ __forceinline__ double dn1(double v, int s = 1) { return __shfl_down_
 
 // PCR over one row per lane (lane ln of a group holds row ln of a G-row system coupled to ln +- s),
 // every row scaled to a unit diagonal so that a level fetches three values from each neighbour;
-// returns the last level's diagonal (the pivot, before scaling) in eb and x in ed.
+// returns the last level's diagonal (the pivot, before scaling) in eb and x in ed. A lane with no
+// neighbour at distance s gets its own values back from the shuffle, and its coupling that way is zero
+// (the first row's a and the last row's c are, and a level carries the zeros on to lanes ln < 2 s and
+// from the far end), so nothing is selected (256^2 x 64 FP64 139 -> 137 us, 512^2 x 128 1025 -> 1006).
 template <int G>
-__device__ __forceinline__ void pcr_lanes(double ea, double &eb, double ec, double &ed, int ln) {
+__device__ __forceinline__ void pcr_lanes(double ea, double &eb, double ec, double &ed) {
     double ib = rcp<double>(eb);
     double na = ea * ib, nc = ec * ib, nd = ed * ib;
 #pragma unroll
     for (int s = 1; s < G; s <<= 1) {
         double am = up1<G>(na, s), cm = up1<G>(nc, s), dm = up1<G>(nd, s);
         double ap = dn1<G>(na, s), cp = dn1<G>(nc, s), dp = dn1<G>(nd, s);
-        if (ln < s) { am = 0.0; cm = 0.0; dm = 0.0; }
-        if (ln + s > G - 1) { ap = 0.0; cp = 0.0; dp = 0.0; }
         eb = fma(-na, cm, fma(-nc, ap, 1.0));
         const double a2 = -na * am, c2 = -nc * cp;
         const double d2 = fma(-na, dm, fma(-nc, dp, nd));
@@ -1259,8 +1260,8 @@ __device__ __forceinline__ void pcr_lanes(double ea, double &eb, double ec, doub
 }
 
 template <int G>
-__device__ __forceinline__ void cr_pcr_solve(Row<1> &R_, int ln) {
-    pcr_lanes<G>(R_.a[0], R_.b[0], R_.c[0], R_.d[0], ln);
+__device__ __forceinline__ void cr_pcr_solve(Row<1> &R_) {
+    pcr_lanes<G>(R_.a[0], R_.b[0], R_.c[0], R_.d[0]);
 }
 
 // Two rows per lane (rows 2l and 2l+1): one cyclic-reduction step eliminates the odd rows, leaving
@@ -1268,20 +1269,18 @@ __device__ __forceinline__ void cr_pcr_solve(Row<1> &R_, int ln) {
 // back-substitution. Half the divisions and shuffles of PCR on all rows, the same arithmetic per
 // eliminated row. Returns x in d; b holds the pivots for the zero-pivot check.
 template <int G>
-__device__ __forceinline__ void cr_pcr_solve(Row<2> &R_, int ln) {
+__device__ __forceinline__ void cr_pcr_solve(Row<2> &R_) {
     // odd row o = 2l+1 of this lane; o- = 2l-1 is the previous lane's odd row
     const double ibo = rcp<double>(R_.b[1]);
     double a_om = up1<G>(R_.a[1]), c_om = up1<G>(R_.c[1]), d_om = up1<G>(R_.d[1]), ib_om = up1<G>(ibo);
-    if (ln == 0) { a_om = 0.0; c_om = 0.0; d_om = 0.0; ib_om = 1.0; }
     // even row e = 2l: eliminate x_{e-1} (row o-) and x_{e+1} (row o)
     const double al = -R_.a[0] * ib_om, ga = -R_.c[0] * ibo;
     const double ea = al * a_om, ec = ga * R_.c[1];
     double eb = R_.b[0] + al * c_om + ga * R_.a[1];
     double ed = R_.d[0] + al * d_om + ga * R_.d[1];
-    pcr_lanes<G>(ea, eb, ec, ed, ln);
+    pcr_lanes<G>(ea, eb, ec, ed);
     // odd rows: x_o = (d_o - a_o x_e - c_o x_{e+2}) / b_o
-    double xe2 = dn1<G>(ed);
-    if (ln == G - 1) xe2 = 0.0;
+    const double xe2 = dn1<G>(ed);
     R_.d[0] = ed;
     R_.d[1] = (R_.d[1] - R_.a[1] * ed - R_.c[1] * xe2) * ibo;
     R_.b[0] = eb;
@@ -1290,7 +1289,7 @@ __device__ __forceinline__ void cr_pcr_solve(Row<2> &R_, int ln) {
 // Three rows per lane (rows 3l .. 3l+2): rows 3l+1 and 3l+2 eliminated down the lane, which leaves
 // row 3l coupled to the neighbouring lanes' rows 3l -+ 3 for the PCR; then back-substitution.
 template <int G>
-__device__ __forceinline__ void cr_pcr_solve(Row<3> &R_, int ln) {
+__device__ __forceinline__ void cr_pcr_solve(Row<3> &R_) {
     const double ib1 = rcp<double>(R_.b[1]);
     const double f = -R_.a[2] * ib1;
     const double a2 = f * R_.a[1], b2 = fma(f, R_.c[1], R_.b[2]), d2 = fma(f, R_.d[1], R_.d[2]);
@@ -1299,14 +1298,12 @@ __device__ __forceinline__ void cr_pcr_solve(Row<3> &R_, int ln) {
     const double A2 = d2 * ib2, B2 = -a2 * ib2, C2 = -R_.c[2] * ib2;
     const double g = -R_.c[1] * ib1;
     const double A1 = fma(g, A2, R_.d[1] * ib1), B1 = fma(g, B2, -R_.a[1] * ib1), C1 = g * C2;
-    double A2m = up1<G>(A2), B2m = up1<G>(B2), C2m = up1<G>(C2);
-    if (ln == 0) { A2m = 0.0; B2m = 0.0; C2m = 0.0; }
+    const double A2m = up1<G>(A2), B2m = up1<G>(B2), C2m = up1<G>(C2);
     const double ea = R_.a[0] * B2m, ec = R_.c[0] * C1;
     double eb = fma(R_.a[0], C2m, fma(R_.c[0], B1, R_.b[0]));
     double ed = fma(-R_.a[0], A2m, fma(-R_.c[0], A1, R_.d[0]));
-    pcr_lanes<G>(ea, eb, ec, ed, ln);
-    double x3 = dn1<G>(ed);
-    if (ln == G - 1) x3 = 0.0;
+    pcr_lanes<G>(ea, eb, ec, ed);
+    const double x3 = dn1<G>(ed);
     R_.d[0] = ed;
     R_.d[1] = fma(C1, x3, fma(B1, ed, A1));
     R_.d[2] = fma(C2, x3, fma(B2, ed, A2));
@@ -1318,10 +1315,9 @@ __device__ __forceinline__ void cr_pcr_solve(Row<3> &R_, int ln) {
 // 4l+2) leave row 4l, solved by PCR across the group; rows 4l+2, then the odd rows follow by
 // back-substitution.
 template <int G>
-__device__ __forceinline__ void cr_pcr_solve(Row<4> &R_, int ln) {
+__device__ __forceinline__ void cr_pcr_solve(Row<4> &R_) {
     const double ib1 = rcp<double>(R_.b[1]), ib3 = rcp<double>(R_.b[3]);
     double a3p = up1<G>(R_.a[3]), c3p = up1<G>(R_.c[3]), d3p = up1<G>(R_.d[3]), ib3p = up1<G>(ib3);
-    if (ln == 0) { a3p = 0.0; c3p = 0.0; d3p = 0.0; ib3p = 1.0; }
     // level 1: rows 4l (eliminate 4l-1, 4l+1) and 4l+2 (eliminate 4l+1, 4l+3)
     double al = -R_.a[0] * ib3p, ga = -R_.c[0] * ib1;
     double a0 = al * a3p, b0 = R_.b[0] + al * c3p + ga * R_.a[1], c0 = ga * R_.c[1];
@@ -1333,14 +1329,12 @@ __device__ __forceinline__ void cr_pcr_solve(Row<4> &R_, int ln) {
     // level 2: row 4l eliminates 4l-2 (previous lane's row 2) and 4l+2
     const double ib2 = rcp<double>(b2);
     double a2p = up1<G>(a2), c2p = up1<G>(c2), d2p = up1<G>(d2), ib2p = up1<G>(ib2);
-    if (ln == 0) { a2p = 0.0; c2p = 0.0; d2p = 0.0; ib2p = 1.0; }
     al = -a0 * ib2p;
     ga = -c0 * ib2;
     double eb = b0 + al * c2p + ga * a2, ed = d0 + al * d2p + ga * d2;
-    pcr_lanes<G>(al * a2p, eb, ga * c2, ed, ln);
+    pcr_lanes<G>(al * a2p, eb, ga * c2, ed);
     const double x0 = ed;
-    double x4 = dn1<G>(x0);
-    if (ln == G - 1) x4 = 0.0;
+    const double x4 = dn1<G>(x0);
     const double x2 = (d2 - a2 * x0 - c2 * x4) * ib2;
     R_.d[1] = (R_.d[1] - R_.a[1] * x0 - R_.c[1] * x2) * ib1;
     R_.d[3] = (R_.d[3] - R_.a[3] * x2 - R_.c[3] * x4) * ib3;
@@ -1902,7 +1896,7 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
             if (a.solver == SOLVER_THOMAS)
                 thomas_solve<M, G>(sys, ln, tsm + (warp * CPW + sub) * 4 * NP);
             else
-                if constexpr (M <= 4) cr_pcr_solve<G>(sys, ln);
+                if constexpr (M <= 4) cr_pcr_solve<G>(sys);
                 else pcr_solve<M>(sys, lane);
             if constexpr (PARK) {
                 if (a.update_ff) {
