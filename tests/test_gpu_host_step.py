@@ -19,7 +19,8 @@ def _pair(cl, precision=0, seed=5, rows=8):
     ctxs = []
     for _ in range(2):
         ctx = context_for_cloud(cl, precision=precision)
-        ctx.set_tuning(rows, 0, 0)
+        if rows:
+            ctx.set_tuning(rows, 0, 0)
         for name, a in (("J", J), ("H_r", Hr), ("H_Z", HZ)):
             ctx.upload(name, a)
             ctx.upload(name + "_old", a)
@@ -152,3 +153,23 @@ def test_host_step_rejects_what_it_does_not_cover():
     with pytest.raises(_lib.LydionError):
         b.static_step_host(J, Hr, HZ, *p)
     b.close()
+
+
+@pytest.mark.parametrize("nr,nz,chunks", [(20, 59, 4), (33, 33, 8), (7, 3, 2)])
+def test_host_step_chunks_end_at_any_row_bitwise(nr, nz, chunks):
+    """Chunk ends between the rows of the tiles, with the tile rows picked automatically, then
+    set between two steps (the chunks' tile lists follow)."""
+    cl = W.static_cloud(nr=nr, nz=nz, n_nu=32, tau0=1e6, T0=1e4, umax_kms=100.0, rs=0.5, tau_abs=0.5)
+    dev, host, (J, Hr, HZ) = _pair(cl, rows=None)
+    p = _params(cl)
+    for rows in (None, 4, 16):
+        if rows:
+            host.set_tuning(rows, 0, 0)
+        rec_d = dev.static_steps(1, *p)[0]
+        J, Hr, HZ, rec_h = host.static_step_host(J, Hr, HZ, *p, out=(J, Hr, HZ), chunks=chunks)
+        np.testing.assert_array_equal(rec_h, rec_d, err_msg=f"rows {rows}")
+        np.testing.assert_array_equal(J, dev.download("J"), err_msg=f"rows {rows}")
+        np.testing.assert_array_equal(Hr, dev.download("H_r"))
+        np.testing.assert_array_equal(HZ, dev.download("H_Z"))
+    dev.close()
+    host.close()
