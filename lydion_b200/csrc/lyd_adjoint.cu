@@ -36,14 +36,14 @@ __device__ __forceinline__ double wsum_d(double v) {
 // Segmented warp sum: the lanes form runs of equal `key` (keys are contiguous runs across the
 // warp). Returns, in the first lane of each run (head), the run's sum; other lanes get partial
 // sums. Every lane of the warp must call it.
-__device__ __forceinline__ double seg_sum(double v, long long key, int lane, bool &head) {
+__device__ __forceinline__ double seg_sum(double v, int key, int lane, bool &head) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double w = __shfl_down_sync(0xffffffffu, v, o);
-        const long long kk = __shfl_down_sync(0xffffffffu, key, o);
+        const int kk = __shfl_down_sync(0xffffffffu, key, o);
         if (lane + o < 32 && kk == key) v += w;
     }
-    const long long kp = __shfl_up_sync(0xffffffffu, key, 1);
+    const int kp = __shfl_up_sync(0xffffffffu, key, 1);
     head = lane == 0 || kp != key;
     return v;
 }
@@ -305,14 +305,14 @@ template <int M>
 __global__ void __launch_bounds__(ADJ_THREADS, 2) k_freq_adj(FreqAdjArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int nnu = a.nnu;
-    const int4 it = a.items[blockIdx.x];
-    const CloudDesc &cd = a.cl[it.x];
+    const CloudDesc &cd = a.cl[0];
+    const int first = a.cell0 + blockIdx.x * a.per_block, end = min(first + a.per_block, a.cell1);
     const double c_tilde = cd.c_tilde, dt = cd.dt, ctdt = cd.ctdt;
     const double jeps = a.jeps, dw = 1.0 / ctdt;
     __shared__ double etab[32];
     if (threadIdx.x < 32) etab[threadIdx.x] = kExp2Tab[threadIdx.x];
     __syncthreads();
-    for (int cl = it.y + warp; cl < it.z; cl += nw) {
+    for (int cl = first + warp; cl < end; cl += nw) {
         const long long c = cd.oc + cl;
         const long long base = cd.o3 + (long long)cl * nnu;
         double JA[M], HrA[M], HZA[M], Hv[M], dn[M];
@@ -622,7 +622,7 @@ __device__ __forceinline__ GCell gcell(const AdjAdvArgs &a, int i, int j, int k)
     if (j < 0) { if (a.bc_z_bot == 0) { g.j = -1 - j; g.sHZ = -1.0; } else { g.j = 0; g.sHZ = -2.0; } }
     else if (j >= nz) { if (a.bc_z_top == 0) { g.j = 2 * nz - 1 - j; g.sHZ = -1.0; } else { g.j = nz - 1; g.sHZ = 2.0; } }
     else g.j = j;
-    long long x = (long long)k + (long long)a.nnu * ((long long)g.i + (long long)nr * g.j);
+    const int x = k + a.nnu * (g.i + nr * g.j);
     g.J = a.J[x];
     double hr = a.Hr[x], hz = a.HZ[x];
     // outflow ghosts keep only the outgoing sign: 2.0 marks max(H, 0), -2.0 min(H, 0)
@@ -636,24 +636,25 @@ __device__ __forceinline__ GCell gcell(const AdjAdvArgs &a, int i, int j, int k)
 }
 
 __device__ __forceinline__ double alpha_F_at(const AdjAdvArgs &a, int i, int j, int k) {
-    long long c = (long long)i + (long long)a.nr * j;
-    double v = a.alpha[c] * a.Hv[(long long)k + (long long)a.nnu * c];
+    const int c = i + a.nr * j;
+    double v = a.alpha[c] * a.Hv[k + a.nnu * c];
     if (a.alpha_cF) v += a.alpha_cF[c];
     return v;
 }
 
 // Cell update adjoint (src/AdvectJandH.jl:1302-1382 reversed): warp = one cell x 32 bins.
-// One thread per cell-bin, cell-major (a warp may span two or three cells).
+// One thread per cell-bin, cell-major (a warp may span two or three cells). The indices of the
+// advection's adjoint are 32 bits: its 17 fields of n3 doubles hold n3 far below 2^31 (the three
+// kernels at 128^2 x 48: 166 us a step with 64-bit indices and divisions, 159 without).
 __global__ void __launch_bounds__(ADJ_THREADS) k_adv_adj_cell(AdjAdvArgs a) {
     const int lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long ncell = (long long)a.nr * a.nz;
-    const bool valid = item < ncell * a.nnu;
-    const long long c = valid ? item / a.nnu : -1;
-    const int k = valid ? (int)(item % a.nnu) : 0;
-    const int i = valid ? (int)(c % a.nr) : 0;
+    const unsigned item = blockIdx.x * blockDim.x + threadIdx.x;
+    const int ncell = a.nr * a.nz;
+    const bool valid = item < (unsigned)ncell * a.nnu;
+    const int c = valid ? (int)(item / (unsigned)a.nnu) : -1;
+    const int k = valid ? (int)(item % (unsigned)a.nnu) : 0;
     const bool act = valid && k >= a.kmin && k <= a.kmax;
-    const long long x = (long long)k + (long long)a.nnu * c;
+    const int x = k + a.nnu * c;
     double gu[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (valid && !act) {
         a.lJ[x] = a.gJ[x]; a.lHr[x] = a.gHr[x]; a.lHZ[x] = a.gHZ[x];
@@ -704,7 +705,6 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adv_adj_cell(AdjAdvArgs a) {
         a.lJ[x] = gsJ; a.lHr[x] = gsHr; a.lHZ[x] = gsHZ;
         a.pJ[x] = gJn0; a.pHr[x] = gHrp; a.pHZ[x] = gHZp;
     }
-    (void)i;
     bool head = false;
 #pragma unroll
     for (int q = 0; q < 5; q++) gu[q] = seg_sum(gu[q], c, lane, head);
@@ -720,32 +720,32 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adv_adj_cell(AdjAdvArgs a) {
 template <bool ZDIR, int FLUX>
 __global__ void __launch_bounds__(ADJ_THREADS, 2) k_adv_adj_face(AdjAdvArgs a) {
     const int lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned item = blockIdx.x * blockDim.x + threadIdx.x;
     const int nact = a.kmax - a.kmin + 1;          // the step's active bins, packed densely
     const int nr = a.nr, nz = a.nz;
-    const long long nfaces = ZDIR ? (long long)nr * (nz + 1) : (long long)(nr + 1) * nz;
-    const bool act = nact > 0 && item < nfaces * nact;
-    const long long fi = act ? item / nact : -1;
-    const int k = act ? a.kmin + (int)(item % nact) : 0;
+    const int nfaces = ZDIR ? nr * (nz + 1) : (nr + 1) * nz;
+    const bool act = nact > 0 && item < (unsigned)nfaces * nact;
+    const int fi = act ? (int)(item / (unsigned)nact) : -1;
+    const int k = act ? a.kmin + (int)(item % (unsigned)nact) : 0;
     // r face: fi = f + (nr+1) j ; Z face: fi = i + nr f
-    const int f = !act ? 0 : (ZDIR ? (int)(fi / nr) : (int)(fi % (nr + 1)));
-    const int line = !act ? 0 : (ZDIR ? (int)(fi % nr) : (int)(fi / (nr + 1)));
+    const int f = !act ? 0 : (ZDIR ? fi / nr : fi % (nr + 1));
+    const int line = !act ? 0 : (ZDIR ? fi % nr : fi / (nr + 1));
     double guc = 0.0;
     if (act) {
         const double ctdt = a.ctdt;
         // the two cells sharing the face: lower (f-1) and upper (f) along the sweep direction
         const bool lo = f >= 1, hi = ZDIR ? f <= nz - 1 : f <= nr - 1;
-        auto cidx = [&](int p) -> long long { return ZDIR ? (long long)line + (long long)nr * p : (long long)p + (long long)nr * line; };
+        auto cidx = [&](int p) { return ZDIR ? line + nr * p : p + nr * line; };
         const double Af = ZDIR ? a.A_Z[fi] : a.A_r[fi];
         double gF[3] = {0.0, 0.0, 0.0}, gkL = 0.0, gkR = 0.0;
         if (lo) {
-            long long cl = cidx(f - 1), xl = (long long)k + (long long)a.nnu * cl;
+            const int cl = cidx(f - 1), xl = k + a.nnu * cl;
             double w = -ctdt * a.inv_dV[cl] * Af;
             gF[0] += w * a.pJ[xl]; gF[1] += w * a.pHr[xl]; gF[2] += w * a.pHZ[xl];
             if (!ZDIR) gkL = 0.5 * ctdt * a.inv_r_cell[f - 1] * a.pHr[xl];
         }
         if (hi) {
-            long long cu = cidx(f), xu = (long long)k + (long long)a.nnu * cu;
+            const int cu = cidx(f), xu = k + a.nnu * cu;
             double w = ctdt * a.inv_dV[cu] * Af;
             gF[0] += w * a.pJ[xu]; gF[1] += w * a.pHr[xu]; gF[2] += w * a.pHZ[xu];
             if (!ZDIR) gkR = 0.5 * ctdt * a.inv_r_cell[f] * a.pHr[xu];
@@ -776,15 +776,12 @@ __global__ void __launch_bounds__(ADJ_THREADS, 2) k_adv_adj_face(AdjAdvArgs a) {
         for (int s = 0; s < 4; s++) {
             double gJ = 0.0, gHr = 0.0, gHZ = 0.0;
             adj_cell_f(g4[s].J, g4[s].Hr, g4[s].HZ, a.jeps, gc[s], gJ, gHr, gHZ);
-            long long xs = (long long)k + (long long)a.nnu * ((long long)g4[s].i + (long long)nr * g4[s].j);
+            const int xs = k + a.nnu * (g4[s].i + nr * g4[s].j);
             if (gJ != 0.0) atomicAdd(a.lJ + xs, gJ);
             if (gHr != 0.0 && g4[s].sHr != 0.0) atomicAdd(a.lHr + xs, gHr * g4[s].sHr);
             if (gHZ != 0.0 && g4[s].sHZ != 0.0) atomicAdd(a.lHZ + xs, gHZ * g4[s].sHZ);
         }
-        long long xi = ZDIR ? (long long)k + (long long)a.nnu * ((long long)line + (long long)nr * pi)
-                            : (long long)k + (long long)a.nnu * ((long long)pi + (long long)nr * line);
-        long long xp = ZDIR ? (long long)k + (long long)a.nnu * ((long long)line + (long long)nr * pp)
-                            : (long long)k + (long long)a.nnu * ((long long)pp + (long long)nr * line);
+        const int xi = k + a.nnu * cidx(pi), xp = k + a.nnu * cidx(pp);
         if (gaFi != 0.0) atomicAdd(a.g_aF + xi, gaFi);
         if (gaFp != 0.0) atomicAdd(a.g_aF + xp, gaFp);
     }
@@ -913,17 +910,23 @@ __global__ void k_hvoigt_adj(const double *g_Hv, const double *T, const double *
 
 // ---- launch wrappers ---------------------------------------------------------------------------
 template <int M>
-static void fa_launch(const FreqAdjArgs &a, int nitems, cudaStream_t st) {
-    k_freq_adj<M><<<nitems, ADJ_THREADS, 0, st>>>(a);
+static void fa_launch(const FreqAdjArgs &a, cudaStream_t st) {
+    k_freq_adj<M><<<(a.cell1 - a.cell0 + a.per_block - 1) / a.per_block, ADJ_THREADS, 0, st>>>(a);
 }
 
-void launch_freq_adj(const FreqAdjArgs &a, int nitems, cudaStream_t st) {
-    if (nitems <= 0) return;
+// One wave of CTAs (two per SM): every warp takes the same number of cells, or one less. With the
+// forward kernel's list, four blocks per SM, the second wave ran part empty: 128^2 x 48 142 us a step,
+// so 127 (prefetching the next cell's rows into L1 instead of waiting for them: 133).
+void launch_freq_adj(FreqAdjArgs &a, int sms, cudaStream_t st) {
+    constexpr int W = ADJ_THREADS / 32;
+    const int n = a.cell1 - a.cell0, slots = 2 * sms;
+    if (n <= 0) return;
+    a.per_block = ((n + slots - 1) / slots + W - 1) / W * W;
     switch (bins_per_lane(a.nnu)) {
-    case 1: fa_launch<1>(a, nitems, st); break;
-    case 2: fa_launch<2>(a, nitems, st); break;
-    case 4: fa_launch<4>(a, nitems, st); break;
-    default: fa_launch<8>(a, nitems, st); break;
+    case 1: fa_launch<1>(a, st); break;
+    case 2: fa_launch<2>(a, st); break;
+    case 4: fa_launch<4>(a, st); break;
+    default: fa_launch<8>(a, st); break;
     }
 }
 

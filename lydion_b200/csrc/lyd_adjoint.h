@@ -23,7 +23,7 @@ struct FreqAdjArgs {
     const double *dur_dr, *dur_dZ, *duZ_dr, *duZ_dZ, *ur_over_r;
     const double *nu, *nuC, *dnu, *inv_dnu, *inv_nuC, *dV;
     const CloudDesc *cl;
-    const int4 *items;
+    int cell0, cell1, per_block;        // the cells to step, and how many of them a CTA takes
     double alpha_floor, jeps, heps2, j_scale;
     int recoil, nnu;
     long long ncell;
@@ -56,7 +56,7 @@ struct AdjAdvArgs {
     double ctdt, jeps, heps2;
 };
 
-void launch_freq_adj(const FreqAdjArgs &a, int nitems, cudaStream_t st);
+void launch_freq_adj(FreqAdjArgs &a, int sms, cudaStream_t st);   // sets per_block
 void launch_adv_adj(const AdjAdvArgs &a, cudaStream_t st);
 void launch_seed_spectrum(double *gJ, const double *w, int nnu, int nr, int nz, cudaStream_t st);
 void launch_af_params(const double *g_aF, const double *alpha, const double *Hv, int nnu, long long ncell,

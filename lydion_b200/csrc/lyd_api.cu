@@ -2170,7 +2170,8 @@ int lyd_adjoint_run(lyd_ctx *c, const lyd_adjoint_cfg *cfg, lyd_adjoint_out *out
         fa.dur_dr = c->cellf[CF_DUR_DR]; fa.dur_dZ = c->cellf[CF_DUR_DZ]; fa.duZ_dr = c->cellf[CF_DUZ_DR];
         fa.duZ_dZ = c->cellf[CF_DUZ_DZ]; fa.ur_over_r = c->cellf[CF_UR_OVER_R];
         fa.nu = c->nu; fa.nuC = c->nuC; fa.dnu = c->dnu; fa.inv_dnu = c->inv_dnu; fa.inv_nuC = c->inv_nuC;
-        fa.dV = c->dV; fa.cl = c->cl; fa.items = c->items;
+        fa.dV = c->dV; fa.cl = c->cl;
+        fa.cell0 = c->nr[0] * c->desc[0].j_own0; fa.cell1 = c->nr[0] * c->desc[0].j_own1;
         fa.alpha_floor = c->cfg.alpha_floor; fa.jeps = c->jeps_s; fa.heps2 = c->heps2_s; fa.j_scale = c->jscale;
         fa.recoil = c->cfg.recoil; fa.nnu = nnu; fa.ncell = (long long)nc;
         fa.gJ = lam; fa.gHr = lam + n3; fa.gHZ = lam + 2 * n3;
@@ -2178,7 +2179,7 @@ int lyd_adjoint_run(lyd_ctx *c, const lyd_adjoint_cfg *cfg, lyd_adjoint_out *out
         fa.g_alpha = g_alpha; fa.g_alpha_c = g_alpha_c; fa.g_T = g_T; fa.g_u = g_u; fa.g_Hv = gHv;
         fa.mf_seed = (n == N - 1) && mf_w != 0.0;
         fa.mf_w = mf_w;
-        launch_freq_adj(fa, c->nitems, c->st);
+        launch_freq_adj(fa, c->sms, c->st);
         tick(4);
         // advection adjoint: lambda of x_A -> lambda_n
         AdjAdvArgs ad;
