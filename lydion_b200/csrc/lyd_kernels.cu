@@ -716,25 +716,28 @@ static_assert(PGEO <= PT, "one copy per thread");
 // ncol columns (ncol + 1 columns of nbk bins fit the CTA's threads), the fewest tiles of four
 // candidates; then the columns are shared out evenly over the tiles.
 struct Pack { int nb, nbk, ncol, nct; };
-__host__ __device__ __forceinline__ int pack_cost(int nact, int nr, int nb) {
-    const int nbk = (nact + nb - 1) / nb;
-    int nc = PT / nbk - 1;
-    nc = nc < PNC - 1 ? nc : PNC - 1;
-    return nb * ((nr + nc - 1) / nc);
-}
+__host__ __device__ __forceinline__ int up_div(int a, int b) { return (int)((unsigned)(a + b - 1) / (unsigned)b); }
 __host__ __device__ __forceinline__ Pack pack_of(int nact, int nr, int nb) {
     Pack p;
     p.nb = nb;
-    p.nbk = (nact + nb - 1) / nb;
-    p.nct = pack_cost(nact, nr, nb) / nb;
-    p.ncol = (nr + p.nct - 1) / p.nct;
+    p.nbk = up_div(nact, nb);
+    const int nc = (int)((unsigned)PT / (unsigned)p.nbk) - 1;
+    p.nct = up_div(nr, nc < PNC - 1 ? nc : PNC - 1);
+    p.ncol = up_div(nr, p.nct);
     return p;
 }
-// device: lane q of every warp weighs candidate nb0 + q
+// device: lane q of every warp weighs candidate nb0 + q, and every lane takes the best one's quotients. Every tile
+// waits for this arithmetic: with thirteen divisions in series, the height's loop and its late load of
+// `share` instead of eight and none, 256^2 x 64 took 197.4 us against 195.1 (FP32 storage 135 against 132).
 __device__ __forceinline__ Pack pack_bins(int nact, int nr) {
     const int q = threadIdx.x & 3, nb0 = (nact + 31) / 32;
-    const unsigned key = (unsigned)pack_cost(nact, nr, nb0 + q) * 4u + (unsigned)q;
-    return pack_of(nact, nr, nb0 + (int)(__reduce_min_sync(0xffffffffu, key) & 3u));
+    Pack p = pack_of(nact, nr, nb0 + q);
+    const int best = (int)(__reduce_min_sync(0xffffffffu, (unsigned)(p.nb * p.nct) * 4u + (unsigned)q) & 3u);
+    p.nb = nb0 + best;
+    p.nbk = __shfl_sync(0xffffffffu, p.nbk, best);
+    p.ncol = __shfl_sync(0xffffffffu, p.ncol, best);
+    p.nct = __shfl_sync(0xffffffffu, p.nct, best);
+    return p;
 }
 // Rows per tile when the caller leaves them open: nz rows, tpb tiles to a band of rows, for a
 // cloud whose share of the GPU's resident CTAs is `share`. A field that one wave of tiles of up to 12
@@ -746,15 +749,12 @@ __device__ __forceinline__ Pack pack_bins(int nact, int nr) {
 // 134 us with 8, 156 / 145 with 16 / 4; 512^2 x 128: 1099 us with 16, 1164 with 8).
 constexpr int kPackRows = 16;
 __host__ __device__ __forceinline__ int pack_rows(int tpb, int nz, int share) {
-    const int wave = (tpb * nz + share - 1) / share;          // rows per tile of a single wave
-    int rows = wave;
-    if (wave > 12) {
-        rows = 4;
-        while (rows < kPackRows && rows * rows < 2 * wave) rows++;
+    const int wave = up_div(tpb * nz, share);                 // rows per tile of a single wave
+    int rows = wave < 2 ? 2 : wave;
+    if (wave > 12) {                                          // at least 5, as 2 x 13 > 16
+        rows = wave > kPackRows * kPackRows / 2 ? kPackRows : (int)ceilf(sqrtf(2.0f * wave));
     }
-    rows = rows < 2 ? 2 : rows;
-    const int bands = (nz + rows - 1) / rows;
-    return (nz + bands - 1) / bands;
+    return up_div(nz, up_div(nz, rows));
 }
 // host: the most tiles any window of 1..nnu bins makes of `nz` rows
 int adv_tiles(int nnu, int nr, int nz, int rows, int share) {
@@ -762,8 +762,8 @@ int adv_tiles(int nnu, int nr, int nz, int rows, int share) {
     for (int n = 1; n <= nnu; n++) {
         int tpb = 1 << 30;
         for (int q = 0; q < 4; q++) {
-            const int c = pack_cost(n, nr, (n + 31) / 32 + q);
-            tpb = c < tpb ? c : tpb;
+            const Pack p = pack_of(n, nr, (n + 31) / 32 + q);
+            tpb = p.nb * p.nct < tpb ? p.nb * p.nct : tpb;
         }
         const int r = rows > 0 ? rows : pack_rows(tpb, nz, share);
         const int m = tpb * ((nz + r - 1) / r);
@@ -832,14 +832,15 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
     const int4 it = a.tiles[tile];                          // cloud, rows [y, w), place z in their list
     View v;
     load_view(a.cl[it.x], v);
+    const int share = a.cl[it.x].adv_share;                 // (asked for with the rest, not when it is needed)
     int kmin = a.kwin[2 * it.x], kmax = a.kwin[2 * it.x + 1];
     kmin = kmin > 0 ? kmin : 0;
     kmax = kmax < a.nnu - 1 ? kmax : a.nnu - 1;
     const int nact = kmax >= kmin ? kmax - kmin + 1 : 0;
     const Pack pk = pack_bins(nact > 0 ? nact : 1, v.nr);
-    const int tpb = pk.nb * pk.nct, band = it.z / tpb, e0 = it.z - band * tpb;
-    const int kb = e0 / pk.nct, ct = e0 - kb * pk.nct;
-    const int rows = a.rows > 0 ? a.rows : pack_rows(tpb, it.w - it.y, a.cl[it.x].adv_share);
+    const int tpb = pk.nb * pk.nct, band = (int)((unsigned)it.z / (unsigned)tpb), e0 = it.z - band * tpb;
+    const int kb = (int)((unsigned)e0 / (unsigned)pk.nct), ct = e0 - kb * pk.nct;
+    const int rows = a.rows > 0 ? a.rows : pack_rows(tpb, it.w - it.y, share);
     const int j0 = it.y + band * rows;
     if (j0 >= it.w) return;
     const int j1 = j0 + rows < it.w ? j0 + rows : it.w;
