@@ -218,7 +218,7 @@ int  lyd_static_steps(lyd_ctx *ctx, const lyd_step_params *p, lyd_diag *diag_his
  * layout of lyd_upload) go up, the step runs, the new J, H_r, H_Z come back into the *_out
  * arrays (which may be the inputs themselves) and diag receives its record (may be NULL).
  * p->n_steps is ignored. The copies and the step are pipelined over `chunks` row chunks
- * (1..16; 8 is a good choice): a chunk's rows advect once the next chunk has landed, its cells
+ * (1..16; 8 is a good choice): a chunk's rows advect once they and two more rows have landed, its cells
  * take the frequency step and go back down while later chunks still go up. For that the step
  * uses the active window the previous step decided, and checks it against FindActiveBins of the
  * uploaded J; when they differ (the caller changed J in between, or on the first call) the call
@@ -280,10 +280,11 @@ int  lyd_persistent_info(lyd_ctx *ctx, int32_t *graph);
 
 /* Launch-shape knobs chosen by the autotuner (lydion_b200/autotune.py): rows of the
  * advection tile (4..64; a context that was never tuned picks the height from its size and
- * active window, and lyd_get_tuning then reports the tallest, 16), cells per frequency-kernel block (8..1024, or 0 for automatic), the
- * frequency solver (0: parallel cyclic reduction across the warp; 1: lane-serial
- * elimination), the advection kernel's resident CTAs per SM (2..4 with FP32 arithmetic,
- * 2..3 with FP64, or 0 for the default: 4 and 3), and how the advection stages its rows
+ * active window, and lyd_get_tuning then reports the tallest, 16), cells per frequency-kernel
+ * block (8..1024, or 0 for automatic), the frequency solver (0: parallel cyclic reduction across
+ * the warp; 1: lane-serial elimination), the advection kernel's resident CTAs per SM (2..4 with
+ * FP32 arithmetic, 2..3 with FP64, or 0 for the default: 4 with FP32 storage, else 3), and how the
+ * advection stages its rows
  * (LYD_STAGING_*). lyd_get_tuning reports an automatic cell count as its negative and the
  * staging actually used. */
 #define LYD_STAGING_AUTO   0   /* the library's choice: per-lane                                */

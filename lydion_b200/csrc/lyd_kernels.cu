@@ -696,9 +696,9 @@ __global__ void __launch_bounds__(MTHREADS, MINB) k_advect_tma(AdvArgs<S> a) {
 // 256^2 x 64 took 171 us, with those a row ahead 167).
 // Bound by dependent FP64 latency and instruction issue (24 warps per SM, 80 registers: FP64 pipe 36 %,
 // issue 60 %). Per launch, against tiles of 8 columns x 32 fixed bins with one warp per column and
-// branches in the faces: 256^2 x 64 with 53 active bins 262 -> 202 us (FP64), 187 -> 176 us (mixed),
-// 171 -> 140 us (FP32 storage); 512^2 x 128 with 85 active 1877 -> 1105 us; 24 clouds of 17..96
-// cells a side x 48 bins 254 -> 134 us; 131 x 203 x 50 with the HLL flux 155 -> 95 us. Executed warp
+// branches in the faces: 256^2 x 64 with 53 active bins 262 -> 195 us (FP64), 187 -> 158 us (mixed),
+// 171 -> 132 us (FP32 storage); 512^2 x 128 with 85 active 1877 -> 1088 us; 24 clouds of 17..96
+// cells a side x 48 bins 254 -> 125 us; 131 x 203 x 50 with the HLL flux 155 -> 95 us. Executed warp
 // instructions at 256^2 x 64: 153 -> 125 million from the branch-free faces. A ninth warp for the
 // halo columns and the right face (288 threads, 72 registers) was slower (210 us): it stages four
 // cells to the others' one and holds up the row's barrier.
@@ -744,16 +744,14 @@ __device__ __forceinline__ Pack pack_bins(int nact, int nr) {
 // rows covers is cut until its tiles just fill the wave, down to two rows: its time is a tile's
 // latency (64^2 x 64: 25 us with 2 rows, 28 / 36 / 58 us with 4 / 8 / 16; 131 x 203 x 50: 95 us with 10,
 // 105 / 112 with 8 / 16). Beyond, a tile's prologue (about 1.3 rows of work) pulls towards tall tiles
-// and the last wave, which runs partly empty, towards short ones: rows^2 = 2 x the rows of a single
-// wave balances the two (256^2 x 64: 200 us with 8 or 9 rows, 205 / 225 with 16 / 4; the 24 clouds
-// 134 us with 8, 156 / 145 with 16 / 4; 512^2 x 128: 1099 us with 16, 1164 with 8).
+// and the last wave, which runs partly empty, towards short ones: rows^2 = 4 x the rows of a single
+// wave balances the two (256^2 x 64: 194 us with 12 rows, 195 / 199 with 9 / 16, mixed 158 / 162 / 171;
+// the 24 clouds 134 us with 8, 156 / 145 with 16 / 4; 512^2 x 128: 1084 us with 16, 1097 / 1158 with 12 / 8).
 constexpr int kPackRows = 16;
 __host__ __device__ __forceinline__ int pack_rows(int tpb, int nz, int share) {
     const int wave = up_div(tpb * nz, share);                 // rows per tile of a single wave
     int rows = wave < 2 ? 2 : wave;
-    if (wave > 12) {                                          // at least 5, as 2 x 13 > 16
-        rows = wave > kPackRows * kPackRows / 2 ? kPackRows : (int)ceilf(sqrtf(2.0f * wave));
-    }
+    if (wave > 12) rows = wave > kPackRows * kPackRows / 4 ? kPackRows : (int)ceilf(sqrtf(4.0f * wave));
     return up_div(nz, up_div(nz, rows));
 }
 // host: the most tiles any window of 1..nnu bins makes of `nz` rows
@@ -2284,7 +2282,9 @@ static void adv_occ(const void *args, cudaStream_t st, int ctas) {
 
 int adv_ctas_per_sm(int prec, int want) {
     if (prec == PREC_K_FP64) return (want == 2) ? 2 : 3;   // FP64: 75 KB of shared memory, 80 registers
-    return (want >= 2 && want <= 4) ? want : 4;
+    // FP32 arithmetic: three CTAs of 80 registers against four of 64: mixed 158 against 161 us at 256^2 x 64,
+    // 533 / 541 at 512^2 x 64, level on small fields; FP32 storage 133 against 130
+    return (want >= 2 && want <= 4) ? want : prec == PREC_K_FP32 ? 4 : 3;
 }
 
 void launch_advect(int prec, int flux, const void *args, int ctas, cudaStream_t st) {
