@@ -106,8 +106,7 @@ struct lyd_ctx {
     size_t stage_n = 0;
     double *small = nullptr;           // device scratch (512 doubles)
     cudaGraphExec_t gexec = nullptr;
-    int gkey_cur = -1;
-    long long gkey_polls = 0;          // 0: a graph of kGraphSteps steps; else the persistent step's poll limit
+    std::vector<unsigned char> gkey;   // the kernels' arguments it was captured with (step_key)
     int steps_run = 0;                 // fused steps so far, up to kGraphAfter
     // the host-state step (lyd_static_step_host): the state as uploaded, the window check, the
     // work lists grouped by row chunk, its copy streams and events
@@ -283,7 +282,6 @@ static int build_work(lyd_ctx *c) {
     c->ntiles = (int)t.size();
     c->ntma = (int)tt.size();
     c->nitems = (int)it.size();
-    drop_graph(c);
     return sync_desc(c);
 }
 
@@ -990,7 +988,6 @@ int lyd_advect_jh(lyd_ctx *c, double ctdt, int32_t kmin, int32_t kmax, int32_t u
         c->cur = old;              // the set `in` keeps the state before the advection as J_old / H_old
     } else {
         for (int q = 0; q < 3; q++) std::swap(c->set[in][q], c->spare[q]);
-        drop_graph(c);             // its kernels' buffers have changed
         c->tmaps_stale = true;
         if (c->tma_tiles) LYD_TRY(encode_tmaps(c));
     }
@@ -1146,23 +1143,26 @@ int lyd_f_esc(lyd_ctx *c, double L_all, int32_t bc_z_bot, double *f) {
 
 // ---- fused static-cloud step -----------------------------------------------------------------
 template <typename S>
-// One step from set[cur] back into set[cur] (x_A in the other set). The adjoint's forward sweep
-// passes `tape` to record the advection's tape, `in` / `out` (three fields each, n3 apart) to
-// read s_n from and write s_{n+1} into its own storage instead, and `ff` to keep the frequency
-// factors F+, F, F- (n3 apart), and `win_next` to receive the window the step decides for the
-// next one.
-// `polls` > 0 runs the step as one cooperative launch of the persistent kernel whose grid
-// barriers give up after that many polls.
-static int enqueue_step(lyd_ctx *c, bool timed, double *tape = nullptr, const S *in = nullptr, S *out = nullptr,
-                        double *ff = nullptr, bool reduce = true, int *win_next = nullptr, long long polls = 0) {
+struct StepArgs {
+    AdvArgs<S> adv;
+    FreqArgs<S> freq;
+    RedArgs red;
+};
+
+// The three kernels' arguments for one step from set[cur] back into set[cur] (x_A in the other
+// set), as the context stands now; see enqueue_step for the options.
+template <typename S>
+static void step_args(lyd_ctx *c, StepArgs<S> &s, bool timed, double *tape, const S *in, S *out, double *ff,
+                      int *win_next, long long polls) {
     const int A = c->cur, B = 1 - c->cur;
-    AdvArgs<S> aa;
+    memset(&s, 0, sizeof(s));
+    AdvArgs<S> &aa = s.adv;
     fill_adv<S>(c, aa, A, B);
     aa.tape = tape;
     aa.tape_stride = (long long)c->n3;
     if (in) { aa.J = in; aa.Hr = in + c->n3; aa.HZ = in + 2 * c->n3; }
     if (in || polls > 0) packed_tiles(c, aa);
-    FreqArgs<S> fa;
+    FreqArgs<S> &fa = s.freq;
     if (out)
         fill_freq<S>(c, fa, c->set[B][0], c->set[B][1], c->set[B][2], c->set[B][0], out, out + c->n3,
                      out + 2 * c->n3);
@@ -1173,11 +1173,43 @@ static int enqueue_step(lyd_ctx *c, bool timed, double *tape = nullptr, const S 
     fa.parts = PART_ACTIVE | PART_DIAG;
     fa.f_r = c->cellf[CF_F_R]; fa.f_Z = c->cellf[CF_F_Z];
     if (ff) { fa.Fkp = ff; fa.Fk = ff + c->n3; fa.Fkm = ff + 2 * c->n3; }
-    RedArgs ra = red_args(c, PART_ACTIVE | PART_DIAG);
+    RedArgs &ra = s.red;
+    ra = red_args(c, PART_ACTIVE | PART_DIAG);
     ra.diag = c->hist; ra.step_counter = c->step_ctr; ra.done = c->step_ctr + 1; ra.hist_capacity = c->hist_cap;
     ra.kwin_copy = win_next;
     // the three kernels, and the next step's after them, overlap their ends and beginnings
     aa.chained = fa.chained = ra.chained = !timed;
+}
+
+// Everything a captured step holds: the kernels' arguments, byte for byte, the tuning that picks their
+// variants and launch shapes, and the poll limit (0: the three-launch step). A graph is replayed only while
+// all of it is as it was at the capture, so no input that appears, goes or moves needs to say so.
+template <typename S>
+static std::vector<unsigned char> step_key(lyd_ctx *c, long long polls) {
+    StepArgs<S> s;
+    step_args<S>(c, s, false, nullptr, nullptr, nullptr, nullptr, nullptr, polls);
+    std::vector<unsigned char> key(sizeof(s) + sizeof(c->tune) + sizeof(polls));
+    memcpy(key.data(), &s, sizeof(s));
+    memcpy(key.data() + sizeof(s), &c->tune, sizeof(c->tune));
+    memcpy(key.data() + sizeof(s) + sizeof(c->tune), &polls, sizeof(polls));
+    return key;
+}
+
+// One step from set[cur] back into set[cur]. The adjoint's forward sweep
+// passes `tape` to record the advection's tape, `in` / `out` (three fields each, n3 apart) to
+// read s_n from and write s_{n+1} into its own storage instead, and `ff` to keep the frequency
+// factors F+, F, F- (n3 apart), and `win_next` to receive the window the step decides for the
+// next one.
+// `polls` > 0 runs the step as one cooperative launch of the persistent kernel whose grid
+// barriers give up after that many polls.
+template <typename S>
+static int enqueue_step(lyd_ctx *c, bool timed, double *tape = nullptr, const S *in = nullptr, S *out = nullptr,
+                        double *ff = nullptr, bool reduce = true, int *win_next = nullptr, long long polls = 0) {
+    StepArgs<S> s;
+    step_args<S>(c, s, timed, tape, in, out, ff, win_next, polls);
+    AdvArgs<S> &aa = s.adv;
+    FreqArgs<S> &fa = s.freq;
+    RedArgs &ra = s.red;
     const int prec = c->prec;
     if (polls > 0) {
         if (timed) cudaEventRecord(c->ev[0], c->st);
@@ -1225,7 +1257,6 @@ static int run_steps(lyd_ctx *c, int n_steps, lyd_diag *hist_out, long long poll
         int cap = n_steps < 1024 ? 1024 : n_steps;
         LYD_TRY(dalloc(c, (void **)&c->hist, (size_t)cap * c->ncl * 7 * 8));
         c->hist_cap = cap;
-        drop_graph(c);
     }
     LYD_TRY(sync_desc(c));
     LYD_CU(c, cudaMemsetAsync(c->step_ctr, 0, 2 * sizeof(int), c->st));
@@ -1262,7 +1293,9 @@ static int run_steps(lyd_ctx *c, int n_steps, lyd_diag *hist_out, long long poll
         const int gs = polls > 0 ? 1 : kGraphSteps;
         const bool graph = polls > 0 ? c->persist_graph >= 0
                                      : n_steps >= gs && (c->gexec || c->steps_run + n_steps >= kGraphAfter);
-        if (graph && (!c->gexec || c->gkey_cur != c->cur || c->gkey_polls != polls)) {
+        std::vector<unsigned char> key;
+        if (graph) key = c->sprec == 0 ? step_key<double>(c, polls) : step_key<float>(c, polls);
+        if (graph && (!c->gexec || c->gkey != key)) {
             drop_graph(c);
             cudaGraph_t g = nullptr;
             LYD_CU(c, cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
@@ -1281,8 +1314,7 @@ static int run_steps(lyd_ctx *c, int n_steps, lyd_diag *hist_out, long long poll
             }
             if (r != LYD_OK) return r;
             if (e != cudaSuccess) return fail(c, LYD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-            c->gkey_cur = c->cur;
-            c->gkey_polls = polls;
+            c->gkey = key;
             if (polls > 0) c->persist_graph = 1;
         }
         int n = 0;
@@ -1979,7 +2011,6 @@ int lyd_adjoint_run(lyd_ctx *c, const lyd_adjoint_cfg *cfg, lyd_adjoint_out *out
         c->hist_cap = 0;
         LYD_TRY(dalloc(c, (void **)&c->hist, (size_t)N * 7 * 8));
         c->hist_cap = N;
-        drop_graph(c);
     }
     // One workspace, kept in the context between calls. It holds: the checkpoints (every
     // step's state when all are kept); per step of one segment the state (recomputation only);
