@@ -29,7 +29,9 @@ constexpr int FREQ_THREADS = 256;
 // what needs nothing from it), and every CTA waits for the kernels before it to have finished, and
 // their writes to be visible, before it reads or writes anything of theirs. Every CTA of every kernel
 // of the chain waits, so a kernel that has finished vouches for all before it. Launched without the
-// attribute the two do nothing.
+// attribute the two do nothing. What a kernel of the chain writes (J, H_r, H_Z, Delta rho u, the window, the
+// partials) is read by plain loads or asynchronous copies: a kernel may be resident while its
+// predecessors still write, and __ldg asks for data that nobody writes as long as the kernel lives.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -69,9 +71,9 @@ template <typename S, typename R>
 __device__ __forceinline__ Cell<R> ld_cell(const AdvArgs<S> &a, const View &v, int i, int j, int k) {
     long long x = v.o3 + (long long)k + (long long)a.nnu * ((long long)i + (long long)v.nr * j);
     Cell<R> c;
-    c.J = R(__ldg(a.J + x));
-    c.Hr = R(__ldg(a.Hr + x));
-    c.HZ = R(__ldg(a.HZ + x));
+    c.J = R(a.J[x]);
+    c.Hr = R(a.Hr[x]);
+    c.HZ = R(a.HZ[x]);
     return c;
 }
 
@@ -1680,8 +1682,9 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
             }
             cs[CS_DV * 32 + lane] = dV;
             cs[CS_POW * 32 + lane] = kFourPi * dV * js;
-            cs[CS_DRU_R * 32 + lane] = ld(a.dru_r, a.do_emission);
-            cs[CS_DRU_Z * 32 + lane] = ld(a.dru_Z, a.do_emission);
+            const bool du = v && a.do_emission && a.dru_r;       // (flush writes them: no __ldg)
+            cs[CS_DRU_R * 32 + lane] = du ? a.dru_r[cc] : 0.0;
+            cs[CS_DRU_Z * 32 + lane] = du ? a.dru_Z[cc] : 0.0;
             __syncwarp();
         }
         const double *cv = cs + (cl - g0);        // cv[f * 32]: field f of this cell
