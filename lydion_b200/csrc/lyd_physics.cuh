@@ -332,9 +332,16 @@ __device__ __forceinline__ void face_flux(const CellF<R> &cm1, const CellF<R> &c
     const Side<R> L = side_of<R, ZDIR>(J_L > jeps ? J_L : jeps, fr_L, fZ_L);
     const Side<R> Q = side_of<R, ZDIR>(J_R > jeps ? J_R : jeps, fr_R, fZ_R);
     const R tau = aF_i * dL + aF_ip1 * dR;
-    const R num = R(0.2) + tau;
-    const R r = rcp<R>(num + tau * tau);
-    const R eps = num * r, te = tau * r;
+    R num = R(0.2) + tau, tt = tau;
+    if constexpr (sizeof(R) == 4) {
+        // tau^2 leaves FP32's range (and its reciprocal is flushed from 9e18 on): beyond 1e18, where 0.2 and 1
+        // are lost beside tau, both weights are 1 / (1 + tau), of terms that stay in range up to FLT_MAX
+        const bool deep = tau > R(1e18);
+        num = deep ? R(0.125) : num;
+        tt = deep ? R(0.125) : tau;
+    }
+    const R r = rcp<R>(num + tt * tau);
+    const R eps = num * r, te = tt * r;
     const R diff = -Num<R>::third() * (cp1.J - ci.J) * te;
     const R Kr_L = ZDIR ? L.Kt : L.Kn, Kr_R = ZDIR ? Q.Kt : Q.Kn, KZ_L = ZDIR ? L.Kn : L.Kt, KZ_R = ZDIR ? Q.Kn : Q.Kt;
     const R Hn_L = ZDIR ? L.HZ : L.Hr, Hn_R = ZDIR ? Q.HZ : Q.Hr;
