@@ -279,14 +279,15 @@ int  lyd_batch_steps_persistent(lyd_ctx *ctx, const lyd_cloud_params *params, in
 int  lyd_persistent_info(lyd_ctx *ctx, int32_t *graph);
 
 /* Launch-shape knobs chosen by the autotuner (lydion_b200/autotune.py): rows of the
- * advection tile (4..64; a context that was never tuned picks the height from its size and
- * active window, and lyd_get_tuning then reports the tallest, 16), cells per frequency-kernel
+ * advection tile (4..64, or 0 for automatic: the height follows the size and the active window;
+ * a context starts so), cells per frequency-kernel
  * block (8..1024, or 0 for automatic), the frequency solver (0: parallel cyclic reduction across
  * the warp; 1: lane-serial elimination), the advection kernel's resident CTAs per SM (2..4 with
  * FP32 arithmetic, 2..3 with FP64, or 0 for the default: 4 with FP32 storage, else 3), and how the
  * advection stages its rows
- * (LYD_STAGING_*). lyd_get_tuning reports an automatic cell count as its negative and the
- * staging actually used. */
+ * (LYD_STAGING_*). lyd_get_tuning reports what is automatic as a negative (minus the tallest
+ * tile, 16; minus the cell count in force) and the staging actually used; lyd_set_tuning takes
+ * what lyd_get_tuning reports, an automatic knob staying automatic. */
 #define LYD_STAGING_AUTO   0   /* the library's choice: per-lane                                */
 #define LYD_STAGING_LANES  1   /* per-lane copies of every staged cell, in tiles packed over the
                                   active bins                                                   */

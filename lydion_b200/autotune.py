@@ -1,7 +1,7 @@
 """Launch-shape autotuner for the Lyman-alpha step.
 
 Five knobs of a context are tuned (lyd_set_tuning):
-  rows_per_tile    rows of the advection tile each CTA marches through (4..64);
+  rows_per_tile    rows of the advection tile each CTA marches through (4..64, or 0 = automatic);
   adv_ctas_per_sm  resident advection CTAs per SM (2..4 with FP32 arithmetic, 2..3 with FP64);
   adv_staging      how the advection stages its rows: per-lane loads (1) or bulk tensor copies
                    of each row's box completed on an mbarrier (2);
@@ -28,12 +28,17 @@ import tempfile
 
 import numpy as np
 
-ROWS = (4, 8, 12, 16, 20, 24, 32, 40, 48)
+ROWS = (0, 4, 8, 12, 16, 20, 24, 32, 40, 48)
 CTAS = (2, 3, 4)
 CELLS = (0, 16, 32, 64, 128, 256, 512)
 SOLVERS = (0, 1)
 STAGING = (1, 2)        # per-lane loads, bulk tensor copies (the library falls back to the first
                         # where the layout does not allow the second)
+
+
+# Part of a cached shape's key: raised when the kernels change so far that shapes tuned for the ones
+# before say nothing any more. 2: the packed advection tiles and the frequency kernel's lane groups.
+KERNELS = 2
 
 
 def cache_path():
@@ -55,7 +60,7 @@ def workload_key(ctx, device=0):
     """GPU name + bins + precision + cloud sizes (hashed for batches)."""
     sizes = getattr(ctx, "sizes", None) or [(ctx.n_r, ctx.n_z)]
     h = hashlib.sha1(np.asarray(sorted(sizes), dtype=np.int64).tobytes()).hexdigest()[:12]
-    return f"{device_name(device)}|nnu={ctx.n_nu}|prec={ctx.precision}|clouds={len(sizes)}|sizes={h}|knobs=5"
+    return f"{device_name(device)}|nnu={ctx.n_nu}|prec={ctx.precision}|clouds={len(sizes)}|sizes={h}|knobs=5|kernels={KERNELS}"
 
 
 def _load(path):

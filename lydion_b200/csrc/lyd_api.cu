@@ -282,6 +282,7 @@ static int build_work(lyd_ctx *c) {
     c->ntiles = (int)t.size();
     c->ntma = (int)tt.size();
     c->nitems = (int)it.size();
+    c->hs_req = 0;      // the host-state step's chunks are cut from these lists: again when it next runs
     return sync_desc(c);
 }
 
@@ -552,8 +553,12 @@ int lyd_synchronize(lyd_ctx *c) {
 
 int lyd_set_tuning(lyd_ctx *c, const lyd_tuning *t) {
     if (!c || !t) return LYD_ERR_ARG;
-    if (t->rows_per_tile < 4 || t->rows_per_tile > 64) return fail(c, LYD_ERR_ARG, "rows_per_tile outside 4..64");
-    if (t->cells_per_block != 0 && (t->cells_per_block < 8 || t->cells_per_block > 1024))
+    // automatic: 0, or the negative that lyd_get_tuning reports for it
+    const bool auto_rows = t->rows_per_tile == 0 || t->rows_per_tile == -kDefaultRows;
+    const bool auto_cells = t->cells_per_block == 0 || (t->cells_per_block <= -8 && t->cells_per_block >= -1024);
+    if (!auto_rows && (t->rows_per_tile < 4 || t->rows_per_tile > 64))
+        return fail(c, LYD_ERR_ARG, "rows_per_tile outside 4..64");
+    if (!auto_cells && (t->cells_per_block < 8 || t->cells_per_block > 1024))
         return fail(c, LYD_ERR_ARG, "cells_per_block outside 8..1024");
     if (t->solver != SOLVER_PCR && t->solver != SOLVER_THOMAS) return fail(c, LYD_ERR_ARG, "unknown solver");
     if (t->adv_ctas_per_sm != 0 && (t->adv_ctas_per_sm < 2 || t->adv_ctas_per_sm > 4))
@@ -563,14 +568,17 @@ int lyd_set_tuning(lyd_ctx *c, const lyd_tuning *t) {
     cudaSetDevice(c->dev);
     LYD_CU(c, cudaStreamSynchronize(c->st));
     c->tune = *t;
+    if (auto_rows) c->tune.rows_per_tile = 0;
+    if (auto_cells) c->tune.cells_per_block = 0;
     return build_work(c);
 }
 
 int lyd_get_tuning(lyd_ctx *c, lyd_tuning *t) {
     if (!c || !t) return LYD_ERR_ARG;
     *t = c->tune;
-    t->rows_per_tile = fixed_rows(c);
-    if (t->cells_per_block == 0) t->cells_per_block = -cells_per_block(c);   // negative: chosen automatically
+    // negative: chosen automatically
+    if (t->rows_per_tile == 0) t->rows_per_tile = -kDefaultRows;
+    if (t->cells_per_block == 0) t->cells_per_block = -cells_per_block(c);
     t->adv_ctas_per_sm = adv_ctas_per_sm(c->prec, t->adv_ctas_per_sm);
     t->adv_staging = staging_used(c);
     return LYD_OK;

@@ -102,3 +102,24 @@ def test_concurrent_cache_writes_keep_every_key(tmp_path):
     assert sorted(data) == sorted(f"rank{r}|k{k}" for r in range(4) for k in range(50))
     assert all(data[f"rank{r}|k{k}"] == {"rank": r, "k": k} for r in range(4) for k in range(50))
     assert sorted(os.listdir(tmp_path)) == ["tuning.json", "tuning.json.lock"]
+
+
+def test_search_tries_the_automatic_height():
+    class Auto(FakeCtx):
+        def timing(self):
+            adv, freq, red = super().timing()
+            return [adv * (0.5 if self.t[0] == 0 else 1.0), freq, red]
+
+    ctx = Auto()
+    best, _ = A.search(ctx, ctx.run, steps=5)
+    assert best[0] == 0
+
+
+def test_shapes_of_other_kernels_are_not_applied(tmp_path, monkeypatch):
+    monkeypatch.setattr(A, "device_name", lambda device=0: "g")
+    path = str(tmp_path / "tune.json")
+    ctx = FakeCtx()
+    old = A.workload_key(ctx).replace(f"|kernels={A.KERNELS}", "")
+    assert old.endswith("|knobs=5")
+    A._save(path, {old: {"tuning": [48, 0, 1, 2, 1]}})
+    assert A.autotune(ctx, ctx.run, steps=3, cache=path) == (8, 64, 0, 3, 2)
