@@ -184,7 +184,10 @@ int  lyd_advect(lyd_ctx *ctx, double ctdt, int32_t bc_r_left, int32_t bc_r_right
 /* AdvectJandH!, src/AdvectJandH.jl:2227-2464, with the caller's bin range [kmin, kmax]
  * (0-based) and J_old rule: update_jold != 0 sets J_old = J after the step, otherwise J_old
  * keeps its value; H_old is left alone. This is the form the stellar/IR bands use
- * (PhotoThermoChemistry.jl:3854-3868: all bands, UpdateJold = false, explicit alpha_F). */
+ * (PhotoThermoChemistry.jl:3854-3868: all bands, UpdateJold = false, explicit alpha_F).
+ * The call only enqueues; errors of its kernel surface at the next synchronising call. With J_old
+ * apart from J it takes memory for three more cell-bin fields, which the context keeps until another
+ * of its allocations or an adjoint run wants the room. */
 int  lyd_advect_jh(lyd_ctx *ctx, double ctdt, int32_t kmin, int32_t kmax, int32_t update_jold,
                    int32_t bc_r_left, int32_t bc_r_right, int32_t bc_z_bot, int32_t bc_z_top);
 /* LyaEmissionAbsorptionUpdate!, src/ConstantsAndFunctions.jl:483-573 (reads the uploaded

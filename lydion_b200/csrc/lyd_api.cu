@@ -64,7 +64,7 @@ struct lyd_ctx {
     void *set[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
     int cur = 0;
     bool old_alias = true;
-    void *spare[3] = {nullptr, nullptr, nullptr};   // third buffers of J, H_r, H_Z (lyd_advect_jh, on first need)
+    void *spare[3] = {nullptr, nullptr, nullptr};   // third buffers of J, H_r, H_Z (lyd_advect_jh): all or none
     bool tmaps_stale = false;          // a buffer set changed since the tensor maps were encoded
     void *Hv = nullptr;
     bool hv_from_T = false;            // H_voigt last computed on the device from T
@@ -144,9 +144,25 @@ static int fail(lyd_ctx *c, int code, const std::string &m) {
             return fail(ctx, LYD_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));    \
     } while (0)
 
+// The spare buffer set holds nothing between calls: it is given back when its memory is wanted.
+static bool free_spare(lyd_ctx *c) {
+    bool any = false;
+    for (void *&p : c->spare) {
+        any = any || p;
+        cudaFree(p);
+        p = nullptr;
+    }
+    return any;
+}
+
 static int dalloc(lyd_ctx *c, void **p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
+    if (e == cudaErrorMemoryAllocation && free_spare(c)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes ? bytes : 16);
+    }
     if (e != cudaSuccess) {
+        cudaGetLastError();      // (the next launch's check is not to find it)
         *p = nullptr;
         return fail(c, LYD_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
@@ -506,7 +522,7 @@ int lyd_destroy(lyd_ctx *c) {
     drop_graph(c);
     for (int s = 0; s < 2; s++)
         for (int q = 0; q < 3; q++) cudaFree(c->set[s][q]);
-    for (void *p : c->spare) cudaFree(p);
+    free_spare(c);
     cudaFree(c->tmaps);
     void *ps[] = {c->Hv, c->phi, c->phi_inv, c->aF, c->Ff[0], c->Ff[1], c->Ff[2], c->u_r_star, c->u_Z_star, c->dV,
                   c->inv_dV, c->A_r, c->A_Z, c->inv_r_cell, c->rCoM, c->ZCoM, c->rint, c->zint, c->r_if, c->Z_if,
@@ -976,9 +992,16 @@ int lyd_advect_jh(lyd_ctx *c, double ctdt, int32_t kmin, int32_t kmax, int32_t u
     // with J_old and H_old apart from J and H, the advected state goes into a third set of buffers, which
     // trades places with the current one: no copies (256^2 x 8 bands: 0.85 -> 0.06 ms per call, most of it
     // the allocation and the six copies that kept the old state before)
-    if (!alias)
-        for (void *&p : c->spare)
-            if (!p) LYD_TRY(dalloc(c, &p, c->n3 * c->ssz));
+    if (!alias && !c->spare[2]) {
+        void *p[3] = {nullptr, nullptr, nullptr};
+        int r = LYD_OK;
+        for (int q = 0; q < 3 && r == LYD_OK; q++) r = dalloc(c, &p[q], c->n3 * c->ssz);
+        if (r != LYD_OK) {
+            for (void *q : p) cudaFree(q);
+            return r;
+        }
+        for (int q = 0; q < 3; q++) c->spare[q] = p[q];
+    }
     std::vector<int> w((size_t)2 * c->ncl);
     for (int q = 0; q < c->ncl; q++) { w[2 * q] = kmin; w[2 * q + 1] = kmax; }
     LYD_CU(c, cudaMemcpyAsync(c->kwin, w.data(), w.size() * sizeof(int), cudaMemcpyHostToDevice, c->st));
@@ -1985,6 +2008,7 @@ int lyd_adjoint_run(lyd_ctx *c, const lyd_adjoint_cfg *cfg, lyd_adjoint_out *out
     // Otherwise a checkpoint every K steps (0: 100) and one recomputation of each segment.
     // When there is room, every step's frequency factors are kept too (3 more doubles per
     // cell-bin), and the frequency-step adjoint reads them instead of recomputing them.
+    free_spare(c);
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) { cudaGetLastError(); fr = 0; }
     const size_t avail = fr + c->adj_ws_bytes, margin = 16 * S * 8 + ((size_t)2 << 30);
