@@ -693,9 +693,10 @@ __global__ void __launch_bounds__(MTHREADS, MINB) k_advect_tma(AdvArgs<S> a) {
 // row: stage row j+2 -> barrier -> each thread computes the r face on its left into shared memory
 // and its Z face j+1/2 into registers -> barrier -> the cell update of row j from the two r faces in
 // shared memory and the Z faces j-1/2 (carried) and j+1/2. Faces never touch HBM. Every staged
-// input comes a row ahead by cp.async; the mixed form has no room for the halo's landing row at
-// four CTAs per SM and loads the halo where it stages it (with its own columns' rows loaded so too
-// 256^2 x 64 took 171 us, with those a row ahead 167).
+// input comes a row ahead by cp.async, but for the halo of the mixed form, which is loaded where it is
+// staged: with four CTAs per SM, which a caller may set, there is no room for its landing row (at the default
+// three there would be: not tried). Its own columns' rows loaded so too: 256^2 x 64 171 us, with
+// those a row ahead 167.
 // Bound by dependent FP64 latency and instruction issue (24 warps per SM, 80 registers: FP64 pipe 36 %,
 // issue 60 %). Per launch, against tiles of 8 columns x 32 fixed bins with one warp per column and
 // branches in the faces: 256^2 x 64 with 53 active bins 262 -> 195 us (FP64), 187 -> 158 us (mixed),
@@ -713,6 +714,7 @@ constexpr int PHALO = 96;              // 3 halo columns x 32 bins
 enum { P_AR, P_UR, P_AZL, P_AZR, P_IDV, P_DURDR, P_DURDZ, P_DUZDR, P_DUZDZ, P_UROR, P_UZ, P_AL, P_ACF, P_N };
 constexpr int PGEO = P_N * PNC + 5;
 static_assert(PGEO <= PT, "one copy per thread");
+static_assert(PT == FREQ_THREADS, "the persistent step's CTAs run tiles and items alike");
 
 // How a window of nact bins of a cloud of nr columns is cut: nb chunks of nbk <= 32 bins, tiles of
 // ncol columns (ncol + 1 columns of nbk bins fit the CTA's threads), the fewest tiles of four
@@ -772,22 +774,14 @@ int adv_tiles(int nnu, int nr, int nz, int rows, int share) {
     return most;
 }
 
-// The cell a staged stencil cell (col, row) copies, and the boundary rules that r_cell / z_cell
-// apply to the copy: rr for H_r, rz for H_Z (1: negate; 2: keep the part <= 0; 3: keep the
-// part >= 0). A corner cell (ghost in both directions) is never staged.
-struct CellSrc { int i, j, rr, rz; };
-__device__ __forceinline__ CellSrc cell_src(const View &v, int col, int row) {
-    CellSrc s{col, row, 0, 0};
-    if (col < 0) {
-        if (v.bcl == 0) { s.i = -1 - col; s.rr = 1; } else { s.i = 0; s.rr = 2; }
-    } else if (col >= v.nr) {
-        if (v.bcr == 0) { s.i = 2 * v.nr - 1 - col; s.rr = 1; } else { s.i = v.nr - 1; s.rr = 3; }
-    } else if (row < 0) {
-        if (v.bzb == 0) { s.j = -1 - row; s.rz = 1; } else { s.j = 0; s.rz = 2; }
-    } else if (row >= v.nz) {
-        if (v.bzt == 0) { s.j = 2 * v.nz - 1 - row; s.rz = 1; } else { s.j = v.nz - 1; s.rz = 3; }
-    }
-    return s;
+// The column a staged stencil column copies, and the boundary rule that r_cell applies to the copy's H_r
+// (1: negate; 2: keep the part <= 0; 3: keep the part >= 0). A ghost row's source and rule change from
+// row to row and are found where it is copied; a corner cell (ghost in both directions) is never staged.
+struct ColSrc { int i, rule; };
+__device__ __forceinline__ ColSrc col_src(const View &v, int col) {
+    if (col < 0) return v.bcl == 0 ? ColSrc{-1 - col, 1} : ColSrc{0, 2};
+    if (col >= v.nr) return v.bcr == 0 ? ColSrc{2 * v.nr - 1 - col, 1} : ColSrc{v.nr - 1, 3};
+    return ColSrc{col, 0};
 }
 template <typename S>
 __device__ __forceinline__ S bc_rule(S h, int rule) {
@@ -926,11 +920,11 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
     };
     // where a (possibly ghost) column's cells and opacities come from, and the rule of its H_r
     auto col_base = [&](int cc, int kk, long long &xc, long long &xac, int &rule) {
-        const CellSrc s = cell_src(v, cc, 0);
+        const ColSrc s = col_src(v, cc);
         const int ci = cc < 0 ? 0 : (cc >= v.nr ? v.nr - 1 : cc);
         xc = v.o3 + kk + (long long)a.nnu * s.i;
         xac = v.o3 + kk + (long long)a.nnu * ci;
-        rule = s.rr;
+        rule = s.rule;
     };
     long long xo = 0, xoa = 0, xh = 0, xha = 0;
     int orule = 0, hrule = 0;
@@ -965,16 +959,10 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
         if (a.alpha_cF) x = x + R(acF);
         return x;
     };
-    // cell (cc, row) by loads, with its state into Hs for the own columns
+    // an own cell's state as stored
     auto keep = [&](S *h, const Cell<S> &x) {
         h[0] = x.Hr; h[PT] = x.HZ;
         if (HF == 3) h[2 * PT] = x.J;
-    };
-    auto stage_direct = [&](R *p, S *h, int cc, int row, int kk) {
-        const Cell<S> x = raw_cell<S, S>(a, v, cc, row, kk);
-        const R aF = alpha_F_clamped<S, R>(a, v, cc, row, kk);
-        put(p, x.J, x.Hr, x.HZ, aF);
-        if (h) keep(h, x);
     };
 
     // ---- per-row scalars: entry t of a row's slot comes from gsrc + row * gstr ----
@@ -1061,7 +1049,10 @@ __device__ __forceinline__ void advect_tile(const AdvArgs<S> &a, int tile, unsig
         // (A) row j+2 of the own columns and row j of the halo columns
         const int r = j + 2;
         if constexpr (!AHEAD) {
-            if (halo) stage_direct(hp, nullptr, hcol, j, hk);
+            if (halo) {
+                const Cell<S> x = raw_cell<S, S>(a, v, hcol, j, hk);
+                put(hp, x.J, x.Hr, x.HZ, alpha_F_clamped<S, R>(a, v, hcol, j, hk));
+            }
         }
         if (stages(r)) {
             const int zrule = r < v.nz ? 0 : (v.bzt == 0 ? 1 : 3);
@@ -1163,8 +1154,8 @@ __device__ __forceinline__ void nbr(const double (&v)[M], double (&out)[M], int 
     }
 }
 
-// Parallel cyclic reduction of the 32*M-row tridiagonal system held by the warp
-// (row r = lane*M + m; a = sub-, b = main-, c = super-diagonal, d = right-hand side).
+// Parallel cyclic reduction of the 32*M-row tridiagonal system held by the warp (8 bins per lane; fewer
+// take cr_pcr_solve below) (row r = lane*M + m; a = sub-, b = main-, c = super-diagonal, d = right-hand side).
 // Decoupled rows are identity rows. Returns x in d.
 template <int M>
 __device__ __forceinline__ void pcr_solve(Row<M> &R_, int lane) {
@@ -1476,11 +1467,11 @@ __device__ __forceinline__ void warp_cell_run(int4 it, int warp, int nw, int cpw
 // per launch 178 -> 141 us (FP64), 174 -> 138 (mixed), 163 -> 129 (FP32 storage); 512^2 x 128 1474 ->
 // 1026 us, 24 clouds x 48 bins 158 -> 123 us, 64^2 x 64 27 -> 24 us.
 //
-// freq_item is one work item (`item` of `nitems`) by the calling CTA, whose first `nw` warps take
-// its cells (the others only meet its barriers), in dynamic shared memory `fsm`: the body of
-// k_freq, also run by the persistent batch kernel.
+// freq_item is one work item (`item` of `nitems`) by the calling CTA of FREQ_THREADS threads, in dynamic
+// shared memory `fsm`: the body of k_freq, also run by the persistent batch kernel.
 template <typename S, typename R, int M, int G, typename RC>
-__device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int nitems, double *fsm, int nw) {
+__device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int nitems, double *fsm) {
+    constexpr int nw = FREQ_THREADS / 32;
     constexpr int NP = G * M, WN = 32 * M, CPW = 32 / G;   // a cell's padded bins, a warp's, a warp's cells
     constexpr bool PF = freq_prefetch<M, G>(), PARK = M == 3;
     static_assert(freq_rows_warp<M, G>(4) >= NP + 8, "a warp's reduction row fits its rows");
@@ -1984,7 +1975,7 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
     for (int m = 0; m < M; m++)
 #pragma unroll
         for (int o = G; o < 32; o <<= 1) acc_e[m] += __shfl_xor_sync(0xffffffffu, acc_e[m], o);
-    if (warp < nw && lane < G) {
+    if (lane < G) {
 #pragma unroll
         for (int m = 0; m < M; m++) red[lane * M + m] = acc_e[m];
     }
@@ -1994,7 +1985,7 @@ __device__ __forceinline__ void freq_item(const FreqArgs<S> &a, int item, int ni
     acc_net = warp_sum(acc_net);
     acc_out = warp_sum(acc_out);
     acc_L = warp_sum(acc_L);
-    if (lane == 0 && warp < nw) {
+    if (lane == 0) {
         red[NP + 0] = acc_tot;
         red[NP + 1] = acc_mf;
         red[NP + 2] = acc_net;
@@ -2016,8 +2007,7 @@ template <typename S, typename R, int M, int G, typename RC = R>
 __global__ void __launch_bounds__(FREQ_THREADS, M <= 4 ? 2 : 1) k_freq(FreqArgs<S> a) {
     extern __shared__ __align__(16) double fsm[];
     pdl_trigger();
-    freq_item<S, R, M, G, RC>(a, a.item0 + (int)blockIdx.x, a.nitems_all ? a.nitems_all : (int)gridDim.x, fsm,
-                           blockDim.x >> 5);
+    freq_item<S, R, M, G, RC>(a, a.item0 + (int)blockIdx.x, a.nitems_all ? a.nitems_all : (int)gridDim.x, fsm);
 }
 
 // FindActiveBins partials of the current J (src/UpdateLyaJandH.jl:47-97): one warp per cell, over
@@ -2215,10 +2205,9 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned nblocks, lo
     return ok != 0;
 }
 
-// One fused static step of every cloud of a batch in one launch: the advection tiles, a grid
-// barrier, the frequency-kernel items (8 of the CTA's 9 warps take the cells, as in k_freq), a
-// grid barrier, the reduction blocks; each CTA walks the work lists with a grid stride. The rows
-// are staged by per-lane loads. Within a launch every buffer one phase reads was written by an
+// One fused static step of every cloud of a batch in one launch: the packed advection tiles, a grid
+// barrier, the frequency-kernel items, a grid barrier, the reduction blocks, each as its own kernel's
+// CTAs of 8 warps run them; each CTA walks the work lists with a grid stride. Within a launch every buffer one phase reads was written by an
 // earlier launch or after a barrier, so no read meets a stale copy: the advection reads the set
 // the previous launch's frequency phase wrote.
 template <typename S>
@@ -2242,7 +2231,7 @@ __global__ void __launch_bounds__(PT, 2) k_step_persistent(PersistArgs<S> p) {
     }
     if (!grid_barrier(p.bar, gridDim.x, p.polls, p.err)) return;
     for (int it = blockIdx.x; it < p.nitems; it += gridDim.x) {
-        freq_item<S, RF, M, G, RC>(p.freq, it, p.nitems, reinterpret_cast<double *>(psm), FREQ_THREADS / 32);
+        freq_item<S, RF, M, G, RC>(p.freq, it, p.nitems, reinterpret_cast<double *>(psm));
         __syncthreads();
     }
     if (!grid_barrier(p.bar, gridDim.x, p.polls, p.err)) return;
