@@ -698,11 +698,11 @@ __global__ void __launch_bounds__(MTHREADS, MINB) k_advect_tma(AdvArgs<S> a) {
 // three there would be: not tried). Its own columns' rows loaded so too: 256^2 x 64 171 us, with
 // those a row ahead 167.
 // Bound by dependent FP64 latency and instruction issue (24 warps per SM, 80 registers: FP64 pipe 36 %,
-// issue 60 %). Per launch, against tiles of 8 columns x 32 fixed bins with one warp per column and
+// issue 59 %). Per launch, against tiles of 8 columns x 32 fixed bins with one warp per column and
 // branches in the faces: 256^2 x 64 with 53 active bins 262 -> 195 us (FP64), 187 -> 158 us (mixed),
 // 171 -> 132 us (FP32 storage); 512^2 x 128 with 85 active 1877 -> 1088 us; 24 clouds of 17..96
 // cells a side x 48 bins 254 -> 125 us; 131 x 203 x 50 with the HLL flux 155 -> 95 us. Executed warp
-// instructions at 256^2 x 64: 153 -> 125 million from the branch-free faces. A ninth warp for the
+// instructions at 256^2 x 64 early in a run, 16 rows: 153 -> 92 million. A ninth warp for the
 // halo columns and the right face (288 threads, 72 registers) was slower (210 us): it stages four
 // cells to the others' one and holds up the row's barrier.
 constexpr int PT = 256;                // threads
@@ -1463,7 +1463,7 @@ __device__ __forceinline__ void warp_cell_run(int4 it, int warp, int nw, int cpw
 // share (opacities times c~ dt, the prefactor of K, h/kT, the gradients' combinations, column and row) is
 // formed once per 32 cells, one cell per lane; the Peclet numbers come from per-bin constants by
 // three multiply-adds; and the factors of a lane's bins are straight-line code (no branch per bin,
-// padding bins computed and dropped). Warp instructions per launch at 256^2 x 64: 122 -> 96 million;
+// padding bins computed and dropped). Warp instructions per launch at 256^2 x 64: 114 -> 91 million;
 // per launch 178 -> 141 us (FP64), 174 -> 138 (mixed), 163 -> 129 (FP32 storage); 512^2 x 128 1474 ->
 // 1026 us, 24 clouds x 48 bins 158 -> 123 us, 64^2 x 64 27 -> 24 us.
 //
