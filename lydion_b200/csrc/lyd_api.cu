@@ -376,8 +376,8 @@ static int encode_tmaps(lyd_ctx *c) {
 // The staging the advection uses: bulk copies when asked for and the maps exist, else the packed
 // tiles' own copies.
 // The packed tiles are the default in every form: a bulk copy's box is fixed when its map is encoded,
-// so its tiles cannot follow the active window (256^2 x 64, 53 active bins, FP32 storage: 140 us packed,
-// 167 us with bulk copies).
+// so its tiles cannot follow the active window (256^2 x 64, 53 active bins, FP32 storage: 132 us packed,
+// 167 us with bulk copies); the bulk-copy form is there for callers that ask for it.
 static int staging_used(const lyd_ctx *c) {
     return (c->tune.adv_staging == LYD_STAGING_TMA && c->tma_ok) ? LYD_STAGING_TMA : LYD_STAGING_LANES;
 }

@@ -1,6 +1,7 @@
 """AdvectJandH! with J_old apart from J writes a third set of J, H_r, H_Z buffers, which the context keeps between
 such calls and gives back when an adjoint run wants the memory."""
-import numpy as np
+import gc
+
 import pytest
 
 from helpers import matched_pair, norm_err
@@ -23,6 +24,7 @@ def test_an_adjoint_run_gets_the_spare_set_s_memory(oracle_mod):
             assert norm_err(ctx.download(f), getattr(st, f)) < 4e-12, f
 
     free = lambda: torch.cuda.mem_get_info(0)[0]
+    gc.collect()                                  # (no other test's context goes while this one counts)
     for f in ("J", "H_r", "H_Z", "J_old"):
         ctx.download(f)                           # (the staging buffers are there before the count)
     none = free()
